@@ -397,8 +397,10 @@ typedef struct rt_batch rt_batch;
  * speed, never a result.  Fields outside the supported set are clamped: block_threads 64 / 128 /
  * 256, blocks_per_sm up to 2048 / block_threads, chunk (queue items a warp takes per atomic, its
  * segment of the shared queue) 32 .. 1024 in steps of 32, steps (traversal records between lane
- * refills) 1 .. 64, stack_entries 32 / 48 / 64 per lane, raised to what the jobs' trees need.
- * Default: 128 threads, 8 blocks per SM, chunk 32, 3 steps, 32 entries, no treelet, shade_blocks 6,
+ * refills) 1 .. 64, stack_entries 32 / 48 / 64, raised to what the jobs' trees need (kept for callers
+ * that set it: the newest entries of a lane's stack are in shared memory and the rest in local
+ * memory, whatever its value).
+ * Default: 128 threads, 7 blocks per SM, chunk 32, 3 steps, 32 entries, no treelet, shade_blocks 6,
  * refill_idle 0. */
 typedef struct rt_wavefront_tuning {
     uint32_t block_threads, blocks_per_sm, chunk, steps, stack_entries;

@@ -255,7 +255,9 @@ __global__ void __launch_bounds__(128) ph_shade_kernel(const __grid_constant__ P
                 Rng rng;
                 rng.state = __float_as_uint(o.w);
                 f3 origin = xyz(o), dir = xyz(d), power = xyz(pw);
-                live = photon_bounce(p, photon_index, iter, h.x, __float_as_uint(h.y), rng, origin, dir, power) && !last;
+                // h.y holds the hit's prim slot; its record names the triangle
+                const uint32_t tri = __float_as_uint(__ldg(p.scene.tri_ord + 3ull * __float_as_uint(h.y)).w);
+                live = photon_bounce(p, photon_index, iter, h.x, tri, rng, origin, dir, power) && !last;
                 if (live) {
                     w.ro[slot] = make_float4(origin.x, origin.y, origin.z, __uint_as_float(rng.state));
                     w.rd[slot] = make_float4(dir.x, dir.y, dir.z, d.w);

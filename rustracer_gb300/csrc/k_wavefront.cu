@@ -13,7 +13,7 @@
 //
 // extend and shadow run as one persistent traversal launch (`wf_trace_kernel`): the occlusion rays of
 // iteration i-1 ride with the closest-hit rays of iteration i, which need only shade(i-1) too.  The
-// photon pass uses the closest-hit-only form (`wf_extend_kernel`).
+// photon pass uses the same kernel for its closest-hit rays.
 //
 // One path slot per pixel: a pixel's samples run one after the other in its slot, with one RNG
 // stream, exactly as the reference's per-pixel loop.  Every pixel receives its contributions in the
@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "rt_kernels.h"
+#include "rt_traverse.cuh"
 
 namespace rtd {
 
@@ -264,89 +265,6 @@ __global__ void __launch_bounds__(128) wf_generate_kernel(const __grid_constant_
         p.nrm[slot] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
     }
     warp_append(active, slot, p.queue[0], p.counts + 0);
-}
-
-// ------------------------------------------------------------------------------------------------
-// Persistent traversal warps.  A warp takes chunks of `chunk` work items with one atomic and hands
-// them to its idle lanes; every lane then advances its traversal by up to `steps` records before the
-// warp refills again, so lanes whose ray finished early pick up new rays instead of idling.  The
-// traversal stack lives in dynamic shared memory, kStack entries per lane, lane-interleaved.
-// ------------------------------------------------------------------------------------------------
-
-struct WarpFeed {
-    uint32_t next = 0, end = 0;
-    bool more = true;
-};
-
-// Gives each lane with need == true the next item index (or none when the items ran out).  Every lane
-// of the warp calls it; returns the lane's index or 0xFFFFFFFF.
-__device__ __forceinline__ uint32_t warp_take(WarpFeed &f, bool need, uint32_t n, uint32_t *fetch, uint32_t chunk) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t mine = 0xFFFFFFFFu;
-    uint32_t mask = __ballot_sync(0xFFFFFFFFu, need);
-    while (mask != 0u && f.more) {
-        if (f.next >= f.end) {
-            uint32_t base = 0;
-            if (lane == 0u) base = atomicAdd(fetch, chunk);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base >= n) {
-                f.more = false;
-                break;
-            }
-            f.next = base;
-            f.end = min(base + chunk, n);
-        }
-        const uint32_t avail = f.end - f.next;
-        const uint32_t rank = __popc(mask & lanemask_lt());
-        if (need && rank < avail) {
-            mine = f.next + rank;
-            need = false;
-        }
-        f.next += min((uint32_t)__popc(mask), avail);
-        mask = __ballot_sync(0xFFFFFFFFu, need);
-    }
-    return mine;
-}
-
-// extend: closest hit of each queued path (any job: each lane traces its own job's scene).
-template <int kStack, int kBlock, bool kWide>
-__global__ void __launch_bounds__(kBlock) wf_extend_kernel(const __grid_constant__ WaveParams p, uint32_t iter,
-                                                           uint32_t chunk, uint32_t steps) {
-    extern __shared__ uint32_t stack_smem[];
-    uint32_t *stk = stack_smem + threadIdx.x;
-    WarpLeaves &wl = reinterpret_cast<WarpLeaves *>(stack_smem + kStack * kBlock)[threadIdx.x >> 5];
-    const uint32_t n = p.counts[4 * iter];
-    const uint32_t *q = p.queue[iter & 1u];
-    uint32_t *fetch = p.counts + 4 * iter + 2;
-    WarpFeed feed;
-    TravState st;
-    bool has = false;
-    uint32_t slot = 0;
-    for (;;) {
-        const uint32_t item = warp_take(feed, !has, n, fetch, chunk);
-        if (item != 0xFFFFFFFFu) {
-            slot = q[item];
-            const float4 o = p.ro[slot], d = p.rd[slot];
-            const DevScene &sc = p.jobs[__float_as_uint(p.thr[slot].w)].scene;
-            st = trav_begin<kWide>(sc, xyz(o), xyz(d), kInf, (uint32_t)kStack);
-            has = true;
-            if (sc.cnode_count == 0u) {
-                p.hit[slot] = make_float2(kInf, 0.0f);
-                has = false;
-            } else {
-                warp_leaves_set_ray(wl, st);
-            }
-        }
-        if (!__any_sync(0xFFFFFFFFu, has)) break;
-        for (uint32_t k = 0; k < steps; ++k) {
-            if (kWide ? trav_step_warp4(st, has, false, stk, (uint32_t)kBlock, wl)
-                      : trav_step_warp(st, has, false, stk, (uint32_t)kBlock, wl)) {
-                p.hit[slot] = make_float2(st.t, __uint_as_float(trav_hit_prim(st)));
-                has = false;
-            }
-            if (!__any_sync(0xFFFFFFFFu, has)) break;
-        }
-    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -805,20 +723,27 @@ __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ 
 // ------------------------------------------------------------------------------------------------
 // shadow: the deferred NEE occlusion test (gather.wgsl:91-103) and the contribution of visible lights.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void shadow_resolve(const WaveParams &p, uint32_t rec_i, const TravState &st, float limit) {
+__device__ __forceinline__ float shadow_limit(float max_dist) { return max_dist - 0.001f; }
+// The triangle of a closest hit (prim: its slot); a miss gives 0.
+__device__ __forceinline__ uint32_t slot_triangle(const DevScene &s, float t, uint32_t prim) {
+    return t < kInf ? __float_as_uint(__ldg(s.tri_ord + 3ull * prim).w) : 0u;
+}
+// The reference's alpha rule of scenes with cut-out materials: whether the ray's closest hit (t, its prim
+// slot) lets the light through.  Out of line: few scenes need it, and its registers would weigh on the
+// traversal.
+__device__ __noinline__ bool cut_out_hit(const DevScene &s, f3 o, f3 d, float t, uint32_t prim) {
+    const TriFull bt = load_tri(s, slot_triangle(s, t, prim));
+    const Mat bm = load_mat(s, bt.material_id);
+    if ((bm.flags & RT_MAT_FLAG_ALPHA_CUTOUT) == 0u || bm.tex_albedo == RT_TEX_NONE) return false;
+    const Bary b = barycentric(bt, o, d, t);
+    return tex_sample(s.tex[RT_TEX_ALBEDO], b.uvx, b.uvy, (int32_t)bm.tex_albedo).w < 0.5f;
+}
+// t: the ray's closest hit (occlusion rays that may stop early: any hit below the limit), prim its slot.
+__device__ __forceinline__ void shadow_resolve(const WaveParams &p, uint32_t rec_i, float t, uint32_t prim) {
     const float4 o = p.shadow[3ull * rec_i], d = p.shadow[3ull * rec_i + 1], c = p.shadow[3ull * rec_i + 2];
     const uint32_t tag = __float_as_uint(c.w);
     const DevScene &s = p.jobs[tag >> 17].scene;
-    bool shadowed = !(st.t >= limit);
-    if (shadowed && !s.any_hit_shadows) {
-        TriFull bt = load_tri(s, trav_hit_prim(st));
-        Mat bm = load_mat(s, bt.material_id);
-        if ((bm.flags & RT_MAT_FLAG_ALPHA_CUTOUT) != 0u && bm.tex_albedo != RT_TEX_NONE) {
-            Bary b = barycentric(bt, xyz(o), xyz(d), st.t);
-            if (tex_sample(s.tex[RT_TEX_ALBEDO], b.uvx, b.uvy, (int32_t)bm.tex_albedo).w < 0.5f) shadowed = false;
-        }
-    }
-    if (shadowed) return;
+    if (!(t >= shadow_limit(o.w)) && (s.any_hit_shadows || !cut_out_hit(s, xyz(o), xyz(d), t, prim))) return;
     acc_add_term(p, __float_as_uint(d.w), tag & 0xFFFFu, xyz(c), (tag & 0x10000u) != 0u);
 }
 
@@ -828,90 +753,222 @@ __device__ __forceinline__ void shadow_resolve(const WaveParams &p, uint32_t rec
 // them with one tail instead of two.  Closest-hit rays come first in the work list: the longer rays
 // start early and the shorter occlusion rays fill the end.
 constexpr uint32_t kNoIter = 0xFFFFFFFFu;
+constexpr uint32_t kOcclusion = 0x80000000u;  // ray id: shadow record (else path slot)
 
+// Each lane of a warp walks its own ray, `steps` records at a time; then finished lanes write their
+// result and take new rays.  The warp is bound by instruction issue and by the latency of its record
+// fetches together, so the step is kept short and the registers few: 7 blocks of 128 threads per SM
+// (72 registers; 64 registers for 8 blocks spill in the step and measure 4% slower, 80 for 6 blocks 4%),
+// the ray feed in shared memory, no branch in the triangle test.  Config-2 frame (28.5 M closest-hit and
+// 24.9 M occlusion rays): 13.5 ms against 16.3 ms for the kernel this one replaced, which tested every
+// step's leaves at once in a list laid out over the warp and read rays when a lane ran out; 22% fewer
+// instructions, 11% fewer records visited (pending records entered beyond the hit are dropped unread).
+//
 // kCount: the profiling variant, which also counts the records each kind of ray visits and its leaf
 // triangle tests into p.work (one atomic per warp at exit); the same rays and results otherwise.
 // kTree (four-wide only): the block first stages the top kTree records of job 0's tree in shared
-// memory (after the stacks and the WarpLeaves), and lanes on that scene read them from there.
-template <int kStack, int kBlock, bool kWide, bool kCount, int kTree>
-__global__ void __launch_bounds__(kBlock, 1024 / kBlock) wf_trace_kernel(const __grid_constant__ WaveParams p, uint32_t ext_iter,
+// memory (after the stacks and the WarpTravs), and lanes on that scene read them from there.
+// kMulti: the launch's jobs may be on different scenes (each ray carries its own); otherwise the scene
+// comes with the launch, which saves four registers and the job table's loads for every ray.
+template <int kBlock, bool kWide, bool kCount, int kTree, bool kMulti>
+__global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __grid_constant__ WaveParams p, uint32_t ext_iter,
                                                           uint32_t shd_iter, uint32_t chunk, uint32_t steps) {
-    extern __shared__ uint32_t stack_smem[];
-    uint32_t *stk = stack_smem + threadIdx.x;
-    WarpLeaves &wl = reinterpret_cast<WarpLeaves *>(stack_smem + kStack * kBlock)[threadIdx.x >> 5];
-    float4 *tree = nullptr;
-    const float4 *tree_src = nullptr;
-    uint32_t tree_n = 0u;
+    extern __shared__ __align__(16) unsigned char trav_smem[];
+    const uint32_t lane = threadIdx.x & 31u;
+    uint2 *top = reinterpret_cast<uint2 *>(trav_smem) + threadIdx.x;
+    uint2 deep[kMaxStack - kTopStack];
+    WarpTrav *warps = reinterpret_cast<WarpTrav *>(trav_smem + sizeof(uint2) * kTopStack * kBlock);
+    WarpTrav &w = warps[threadIdx.x >> 5];
+    Treelet tree{nullptr, nullptr, 0u};
     if (kTree > 0) {
-        tree = reinterpret_cast<float4 *>(reinterpret_cast<WarpLeaves *>(stack_smem + kStack * kBlock) + kBlock / 32);
+        float4 *t = reinterpret_cast<float4 *>(warps + kBlock / 32);
         const DevScene &s0 = p.jobs[0].scene;
-        tree_src = s0.wnodes;
-        tree_n = s0.wnode_count < (uint32_t)kTree ? s0.wnode_count : (uint32_t)kTree;
-        for (uint32_t i = threadIdx.x; i < 8u * tree_n; i += kBlock) tree[i] = __ldg(tree_src + i);
+        tree.smem = t;
+        tree.src = s0.wnodes;
+        tree.count = s0.wnode_count < (uint32_t)kTree ? s0.wnode_count : (uint32_t)kTree;
+        for (uint32_t i = threadIdx.x; i < 8u * tree.count; i += kBlock) t[i] = __ldg(tree.src + i);
         __syncthreads();
     }
-    const uint32_t n_ext = ext_iter != kNoIter ? p.counts[4 * ext_iter] : 0u;
-    const uint32_t n_shd = shd_iter != kNoIter ? p.counts[4 * shd_iter + 1] : 0u;
+    {
+        const uint32_t n_ext = ext_iter != kNoIter ? p.counts[4 * ext_iter] : 0u;
+        const uint32_t n_shd = shd_iter != kNoIter ? p.counts[4 * shd_iter + 1] : 0u;
+        if (lane == 0u) {
+            w.n_ext = n_ext;
+            w.n = n_ext + n_shd;
+        }
+    }
     const uint32_t *q = p.queue[ext_iter & 1u];
     // Row ext_iter's cursor; the closing launch (no closest-hit rays) takes row shd_iter + 1's, which
     // no other launch uses.  Entry [3] of a row counts shade's photon-lookup requests.
     uint32_t *fetch = p.counts + 4 * (ext_iter != kNoIter ? ext_iter : shd_iter + 1u) + 2;
-    WarpFeed feed;
-    TravState st;
-    bool has = false, occlusion = false, any_hit = false;
-    uint32_t id = 0;  // path slot (closest hit) or shadow record (occlusion)
-    float limit = 0.0f;
+
+    // The work list is dealt out in segments of `chunk` items: the first by warp number, the later ones
+    // by one atomic each, issued a segment ahead.  The entries of the next 32 rays are copied to shared
+    // memory ahead of need, and so are the rays themselves, while the warp walks.
+    uint32_t after = (blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * chunk;  // lane 0: the next segment
+    auto read_ahead = [&]() {
+        const uint32_t n = w.n, n_ext = w.n_ext;
+        uint32_t item = w.item, end = w.seg_end, items = 0u;
+        if (item >= end) {
+            item = __shfl_sync(0xFFFFFFFFu, after, 0);
+            end = min(item + chunk, n);
+            if (item < n && lane == 0u) after = gridDim.x * (kBlock / 32) * chunk + atomicAdd(fetch, chunk);
+        }
+        if (item < end) {
+            items = min(32u, end - item);
+            if (lane < items) {
+                if (item + lane < n_ext) cp_async4(&w.next_queue[lane], q + item + lane);
+                else w.next_queue[lane] = (item + lane - n_ext) | kOcclusion;
+            }
+        }
+        __syncwarp();
+        if (lane == 0u) {
+            w.item = item + items;
+            w.seg_end = end;
+            w.items = items;
+        }
+    };
+    // Starts the copy of the next rays (all the copied ones are claimed) and reads on.
+    auto request = [&]() {
+        const uint32_t items = w.items;
+        if (lane < items) {
+            const uint32_t r = w.next_queue[lane], i = r & ~kOcclusion;
+            const bool occ = (r & kOcclusion) != 0u;
+            const float4 *rec = p.shadow + 3ull * i;
+            cp_async16(&w.next_ro[lane], occ ? rec : p.ro + i);
+            cp_async16(&w.next_rd[lane], occ ? rec + 1 : p.rd + i);
+            w.next_inv[lane].w = __uint_as_float(r);
+            if (kMulti) cp_async4(&w.next_inv[lane].x, occ ? &rec[2].w : &p.thr[i].w);
+        }
+        __syncwarp();
+        if (lane == 0u) w.coming = items;
+        if (items != 0u) read_ahead();
+        __syncwarp();
+    };
+    if (lane == 0u) w.item = w.seg_end = w.at = w.ready = 0u;
+    __syncwarp();
+    read_ahead();
+    cp_async_wait();
+    __syncwarp();
+    request();
+
+    TravLane st;
+    uint32_t id = 0u;
+    bool busy = false, visiting = false, any_hit = false;
+    uint32_t queued = 0u;                 // leaves in the warp's queue
     uint32_t work[4] = {0u, 0u, 0u, 0u};  // kCount: records closest / occlusion, tests closest / occlusion
-    // steps: records between refills (low 16 bits) and the idle-lane count that refills earlier (high)
-    const uint32_t max_steps = steps & 0xFFFFu, refill_idle = steps >> 16;
+    st.node = 0u;
+    st.sp = 0u;
+    // Records between refills (low 16 bits), fewer once `few` or less lanes still walk.
+    const uint32_t max_steps = steps & 0xFFFFu;
+    const int few = (int)(steps >> 16);
     for (;;) {
-        const uint32_t item = warp_take(feed, !has, n_ext + n_shd, fetch, chunk);
-        if (item != 0xFFFFFFFFu) {
-            occlusion = item >= n_ext;
-            if (!occlusion) {
-                id = q[item];
-                const float4 o = p.ro[id], d = p.rd[id];
-                const DevScene &sc = p.jobs[__float_as_uint(p.thr[id].w)].scene;
-                any_hit = false;
-                st = trav_begin<kWide>(sc, xyz(o), xyz(d), kInf, (uint32_t)kStack);
-                has = sc.cnode_count != 0u;
-                if (!has) p.hit[id] = make_float2(kInf, 0.0f);
-            } else {
-                id = item - n_ext;
-                const float4 o = p.shadow[3ull * id], d = p.shadow[3ull * id + 1];
-                const DevScene &sc = p.jobs[__float_as_uint(p.shadow[3ull * id + 2].w) >> 17].scene;
-                limit = o.w - 0.001f;
-                // Without cut-out materials the occlusion test may stop at the first triangle below
-                // the limit; with them the reference's closest-hit-then-alpha rule is kept.
-                any_hit = sc.any_hit_shadows != 0u;
-                st = trav_begin<kWide>(sc, xyz(o), xyz(d), any_hit ? limit : kInf, (uint32_t)kStack);
-                has = sc.cnode_count != 0u;
-                if (!has) {
-                    st.t = kInf;
-                    shadow_resolve(p, id, st, limit);
+        // Idle lanes take the next rays.
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
+        if (idle != 0u) {
+            uint32_t at = w.at, ready = w.ready;
+            const uint32_t coming = w.coming;
+            if (at == ready && coming != 0u) {
+                cp_async_wait();
+                if (lane < coming) {
+                    const f3 inv = mk3(1.0f, 1.0f, 1.0f) / xyz(w.next_rd[lane]);
+                    const float4 x = w.next_inv[lane];
+                    w.next_inv[lane] = make_float4(inv.x, inv.y, inv.z, x.w);
+                    if (kMulti) {
+                        const uint32_t word = __float_as_uint(x.x);  // path: its job; shadow record: its tag
+                        w.next_rd[lane].w = __uint_as_float((__float_as_uint(x.w) & kOcclusion) ? word >> 17 : word);
+                    }
+                }
+                at = 0u;
+                ready = coming;
+                __syncwarp();
+                if (lane == 0u) {
+                    w.ready = coming;
+                    w.coming = 0u;
                 }
             }
-            if (has) warp_leaves_set_ray(wl, st);
+            const uint32_t avail = ready - at;
+            if (avail == 0u) {
+                if (idle == 0xFFFFFFFFu) break;
+            } else {
+                const uint32_t rank = __popc(idle & lanemask_lt());
+                if (!busy && rank < avail) {
+                    const float4 o = w.next_ro[at + rank], d = w.next_rd[at + rank], v = w.next_inv[at + rank];
+                    id = __float_as_uint(v.w);
+                    const bool occ = (id & kOcclusion) != 0u;
+                    const float4 *tris = p.tris0;
+                    uint32_t any = p.any_hit0, empty = p.empty0;
+                    st.records = p.records0;
+                    st.cap = kMaxStack;
+                    if (kMulti) {
+                        const DevScene &sc = p.jobs[__float_as_uint(d.w)].scene;
+                        st.records = kWide ? sc.wnodes : sc.cnodes;
+                        st.cap = kWide ? kMaxStack : sc.stack_cap;
+                        tris = sc.tri_ord;
+                        any = sc.any_hit_shadows;
+                        empty = sc.cnode_count == 0u;
+                    }
+                    // Without cut-out materials the occlusion test may stop at the first triangle below
+                    // the limit; with them the reference's closest-hit-then-alpha rule is kept.
+                    any_hit = occ && any != 0u;
+                    st.t = any_hit ? shadow_limit(o.w) : kInf;
+                    const unsigned long long tp = (unsigned long long)tris;
+                    w.ro[lane] = make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)tp));
+                    w.rd[lane] = make_float4(d.x, d.y, d.z, __uint_as_float((uint32_t)(tp >> 32)));
+                    w.best[lane] = hit_word(st.t, 0u);
+                    st.minus_ro[0] = pack2(-o.x, -o.x);
+                    st.minus_ro[1] = pack2(-o.y, -o.y);
+                    st.minus_ro[2] = pack2(-o.z, -o.z);
+                    st.inv[0] = pack2(v.x, v.x);
+                    st.inv[1] = pack2(v.y, v.y);
+                    st.inv[2] = pack2(v.z, v.z);
+                    st.node = 0u;
+                    st.te = -kInf;
+                    st.sp = 0u;
+                    busy = true;
+                    // No triangle counts below kEps, so a limit at or below it (or a NaN) is never met: the
+                    // ray ends as it starts, and so does any ray of an empty scene.
+                    visiting = empty == 0u && st.t > kEps;
+                }
+                at += min((uint32_t)__popc(idle), avail);
+                __syncwarp();
+                if (lane == 0u) w.at = at;
+                if (at == ready) request();
+            }
         }
-        if (!__any_sync(0xFFFFFFFFu, has)) break;
-        for (uint32_t k = 0; k < max_steps; ++k) {
+        // Up to `steps` records, the queued leaves tested eight at a time; then the rest of them, so that
+        // a lane that is no longer visiting has its result.
+        for (uint32_t k = 0;;) {
             uint32_t tests = 0u;
-            const bool visiting = has;
-            if (kWide ? trav_step_warp4(st, has, any_hit, stk, (uint32_t)kBlock, wl, kCount ? &tests : nullptr,
-                                        kTree > 0 ? tree : nullptr, tree_src, tree_n)
-                      : trav_step_warp(st, has, any_hit, stk, (uint32_t)kBlock, wl, kCount ? &tests : nullptr)) {
-                if (occlusion) shadow_resolve(p, id, st, limit);
-                else p.hit[id] = make_float2(st.t, __uint_as_float(st.prim));  // the hit's prim slot
-                has = false;
+            if (kCount && visiting) work[(id & kOcclusion) ? 1 : 0] += 1u;
+            trav_step<kWide, kTree, kBlock, kMulti>(st, top, deep, visiting, w, queued, tree, p.records0, tests);
+            if (kCount) work[(id & kOcclusion) ? 3 : 2] += tests;
+            const bool end = ++k >= max_steps || __popc(__ballot_sync(0xFFFFFFFFu, visiting)) <= few;
+            if (queued >= 8u || (end && queued != 0u)) {
+                const uint32_t tested = end ? queued : queued & ~7u, left = queued - tested;
+                __syncwarp();
+                for (uint32_t g = 0u; g < tested; g += 8u) test_leaves<kMulti>(w, g, min(8u, tested - g), p.tris0);
+                if (left != 0u) {  // the leaves left over move to the front
+                    const uint2 leaf = w.leaf[tested + (lane & 7u)];
+                    __syncwarp();
+                    if (lane < left) w.leaf[lane] = leaf;
+                }
+                __syncwarp();
+                queued = left;
+                if (busy) {
+                    const float t = hit_t(w.best[lane]);
+                    if (any_hit && t < st.t) visiting = false;
+                    st.t = t;
+                    if (visiting) visiting = trav_settle<kBlock>(st, top, deep);
+                }
             }
-            if (kCount && visiting) {
-                work[occlusion ? 1 : 0] += 1u;
-                work[occlusion ? 3 : 2] += tests;
-            }
-            const uint32_t busy = __ballot_sync(0xFFFFFFFFu, has);
-            if (busy == 0u) break;
-            // early refill once `refill_idle` lanes wait and the queue still has work
-            if (refill_idle != 0u && 32u - (uint32_t)__popc(busy) >= refill_idle && feed.more) break;
+            if (end) break;
+        }
+        if (busy && !visiting) {
+            const uint32_t prim = (uint32_t)w.best[lane];
+            if (id & kOcclusion) shadow_resolve(p, id & ~kOcclusion, st.t, prim);
+            else p.hit[id] = make_float2(st.t, __uint_as_float(prim));  // the hit's prim slot
+            busy = false;
         }
     }
     if (kCount && p.work) {
@@ -920,7 +977,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) wf_trace_kernel(const _
             uint32_t v = work[i];
 #pragma unroll
             for (uint32_t d = 16u; d > 0u; d >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, d);
-            if ((threadIdx.x & 31u) == 0u) atomicAdd(p.work + i, (unsigned long long)v);
+            if (lane == 0u) atomicAdd(p.work + i, (unsigned long long)v);
         }
     }
 }
@@ -990,7 +1047,7 @@ __global__ void wf_count_kernel(const __grid_constant__ WaveParams p, uint32_t i
 // ------------------------------------------------------------------------------------------------
 // Host launcher: the gather pass of one frame of every job.
 // ------------------------------------------------------------------------------------------------
-WaveTuning default_tuning() { return WaveTuning{128u, 8u, 32u, 3u, 32u, 0u, 6u, 0u}; }
+WaveTuning default_tuning() { return WaveTuning{128u, 7u, 32u, 3u, 32u, 0u, 6u, 0u}; }
 
 bool normalize_tuning(WaveTuning &t, uint32_t stack_need) {
     const WaveTuning in = t;
@@ -1009,104 +1066,79 @@ bool normalize_tuning(WaveTuning &t, uint32_t stack_need) {
 
 namespace {
 
-using ExtendKernel = void (*)(const WaveParams, uint32_t, uint32_t, uint32_t);
 using TraceKernel = void (*)(const WaveParams, uint32_t, uint32_t, uint32_t, uint32_t);
 
-template <int kStack, int kBlock>
-void pick(const WaveTuning &t, bool wide, bool count, ExtendKernel &ext, TraceKernel &trc) {
-    if ((int)t.stack_entries == kStack && (int)t.block_threads == kBlock) {
-        ext = wide ? wf_extend_kernel<kStack, kBlock, true> : wf_extend_kernel<kStack, kBlock, false>;
-        constexpr int kT = (int)kTreeletRecords;
-        const bool tree = wide && t.treelet != 0u;
-        if (!wide)
-            trc = count ? wf_trace_kernel<kStack, kBlock, false, true, 0> : wf_trace_kernel<kStack, kBlock, false, false, 0>;
-        else if (tree)
-            trc = count ? wf_trace_kernel<kStack, kBlock, true, true, kT> : wf_trace_kernel<kStack, kBlock, true, false, kT>;
-        else
-            trc = count ? wf_trace_kernel<kStack, kBlock, true, true, 0> : wf_trace_kernel<kStack, kBlock, true, false, 0>;
-    }
+// Dynamic shared memory of a traversal block: the lane-interleaved stack tops, one WarpTrav per warp, then
+// the treelet (four-wide launches with t.treelet set).
+size_t trav_smem_bytes(uint32_t block_threads, bool tree) {
+    return (size_t)kTopStack * block_threads * sizeof(uint2) + (block_threads / 32u) * sizeof(WarpTrav) +
+           (tree ? (size_t)kTreeletRecords * 8u * sizeof(float4) : 0u);
 }
 
-// Dynamic shared memory of a traversal block: the lane-interleaved stacks, then one WarpLeaves per warp,
-// then the treelet (four-wide launches with t.treelet set).
-size_t trav_smem_bytes(const WaveTuning &t, bool wide = false) {
-    return (size_t)t.stack_entries * t.block_threads * sizeof(uint32_t) + (t.block_threads / 32u) * sizeof(WarpLeaves) +
-           (wide && t.treelet ? (size_t)kTreeletRecords * 8u * sizeof(float4) : 0u);
+// wf_trace_kernel's `steps`.
+uint32_t trace_steps(const WaveTuning &t) { return t.steps | (t.refill_idle ? 32u - t.refill_idle : 0u) << 16; }
+
+// multi: the jobs may be on different scenes.  The counting and treelet variants are compiled for that
+// case only, which covers the other.
+template <int kBlock>
+TraceKernel trace_kernel_of(bool wide, bool count, bool tree, bool multi) {
+    constexpr int kT = (int)kTreeletRecords;
+    if (!wide) return count ? wf_trace_kernel<kBlock, false, true, 0, true> : wf_trace_kernel<kBlock, false, false, 0, true>;
+    if (tree) return count ? wf_trace_kernel<kBlock, true, true, kT, true> : wf_trace_kernel<kBlock, true, false, kT, true>;
+    if (count) return wf_trace_kernel<kBlock, true, true, 0, true>;
+    return multi ? wf_trace_kernel<kBlock, true, false, 0, true> : wf_trace_kernel<kBlock, true, false, 0, false>;
 }
 
-void trav_kernels(const WaveTuning &t, bool wide, ExtendKernel &ext, TraceKernel &shd, bool count = false) {
-    ext = nullptr;
-    shd = nullptr;
-    pick<32, 64>(t, wide, count, ext, shd);
-    pick<32, 128>(t, wide, count, ext, shd);
-    pick<32, 256>(t, wide, count, ext, shd);
-    pick<48, 64>(t, wide, count, ext, shd);
-    pick<48, 128>(t, wide, count, ext, shd);
-    pick<48, 256>(t, wide, count, ext, shd);
-    pick<64, 64>(t, wide, count, ext, shd);
-    pick<64, 128>(t, wide, count, ext, shd);
-    pick<64, 256>(t, wide, count, ext, shd);
+TraceKernel trace_kernel(const WaveTuning &t, bool wide, bool count, bool multi) {
+    const bool tree = wide && t.treelet != 0u;
+    if (t.block_threads == 64u) return trace_kernel_of<64>(wide, count, tree, multi);
+    if (t.block_threads == 256u) return trace_kernel_of<256>(wide, count, tree, multi);
+    return trace_kernel_of<128>(wide, count, tree, multi);
 }
 
 }  // namespace
 
-template <int kStack, int kBlock, bool kWide>
-void opt_in_smem() {
-    // Blocks above 48 KB of dynamic shared memory need the opt-in; set it for every shape.
-    const int bytes = (int)trav_smem_bytes(WaveTuning{(uint32_t)kBlock, 1u, 64u, 8u, (uint32_t)kStack, 0u, 4u, 0u});
-    const int tree_bytes =
-        (int)trav_smem_bytes(WaveTuning{(uint32_t)kBlock, 1u, 64u, 8u, (uint32_t)kStack, 1u, 4u, 0u}, true);
-    constexpr int kT = (int)kTreeletRecords;
-    cudaFuncSetAttribute(wf_extend_kernel<kStack, kBlock, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(wf_trace_kernel<kStack, kBlock, kWide, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         bytes);
-    cudaFuncSetAttribute(wf_trace_kernel<kStack, kBlock, kWide, true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         bytes);
-    if (kWide) {
-        cudaFuncSetAttribute(wf_trace_kernel<kStack, kBlock, true, false, kT>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, tree_bytes);
-        cudaFuncSetAttribute(wf_trace_kernel<kStack, kBlock, true, true, kT>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, tree_bytes);
-    }
-}
-
-template <bool kWide>
-void opt_in_all() {
-    opt_in_smem<32, 64, kWide>();
-    opt_in_smem<32, 128, kWide>();
-    opt_in_smem<32, 256, kWide>();
-    opt_in_smem<48, 64, kWide>();
-    opt_in_smem<48, 128, kWide>();
-    opt_in_smem<48, 256, kWide>();
-    opt_in_smem<64, 64, kWide>();
-    opt_in_smem<64, 128, kWide>();
-    opt_in_smem<64, 256, kWide>();
-}
-
 void prepare_wavefront_kernels() {
-    opt_in_all<false>();
-    opt_in_all<true>();
+    // Blocks above 48 KB of dynamic shared memory need the opt-in; set it for every variant.
+    for (uint32_t block : {64u, 128u, 256u})
+        for (int v = 0; v < 16; ++v) {
+            const bool wide = (v & 1) != 0, count = (v & 2) != 0, multi = (v & 4) != 0, tree = wide && (v & 8) != 0;
+            WaveTuning t = default_tuning();
+            t.block_threads = block;
+            t.treelet = tree ? kTreeletRecords : 0u;
+            cudaFuncSetAttribute(reinterpret_cast<const void *>(trace_kernel(t, wide, count, multi)),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trav_smem_bytes(block, tree));
+        }
 }
 
-cudaError_t launch_extend(const WaveParams &p, uint32_t iter, uint64_t max_items, const DevScene &scene, int num_sms,
+namespace {
+void set_scene0(WaveParams &p, const DevScene &scene, bool wide) {
+    p.records0 = wide ? scene.wnodes : scene.cnodes;
+    p.tris0 = scene.tri_ord;
+    p.any_hit0 = scene.any_hit_shadows;
+    p.empty0 = scene.cnode_count == 0u ? 1u : 0u;
+}
+}  // namespace
+
+cudaError_t launch_extend(const WaveParams &params, uint32_t iter, uint64_t max_items, const DevScene &scene, int num_sms,
                           const WaveTuning &tune, cudaStream_t st) {
     const bool wide = scene.wnodes != nullptr;
+    WaveParams p = params;
+    set_scene0(p, scene, wide);
     WaveTuning t = tune;
     normalize_tuning(t, wide ? scene.wide_stack : scene.stack_cap);
-    ExtendKernel ext;
-    TraceKernel trc;
-    trav_kernels(t, wide, ext, trc);
-    const size_t smem = trav_smem_bytes(t);
     const uint64_t blocks_needed = (max_items + t.block_threads - 1u) / t.block_threads;
     const uint64_t persistent = (uint64_t)num_sms * t.blocks_per_sm;
     const uint32_t grid = (uint32_t)(blocks_needed < persistent ? (blocks_needed ? blocks_needed : 1u) : persistent);
-    ext<<<grid, t.block_threads, smem, st>>>(p, iter, t.chunk, t.steps);
+    trace_kernel(t, wide, false, false)<<<grid, t.block_threads, trav_smem_bytes(t.block_threads, wide && t.treelet), st>>>(
+        p, iter, kNoIter, t.chunk, trace_steps(t));
     return cudaGetLastError();
 }
 
-cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t n_jobs, uint32_t iters, int num_sms,
+cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uint32_t n_jobs, uint32_t iters, int num_sms,
                              const WaveTuning &tune, cudaStream_t st, WaveProfile *prof) {
     cudaError_t e;
+    WaveParams p = params;
     if ((e = cudaMemsetAsync(p.counts, 0, sizeof(uint32_t) * 4 * (size_t)(iters + 1), st)) != cudaSuccess) return e;
     uint64_t slots = 0;
     uint32_t stack_need = 0, wide_need = 0;
@@ -1119,13 +1151,12 @@ cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t
         wide_need = jobs[j].wide_stack > wide_need ? jobs[j].wide_stack : wide_need;
         wide = wide && jobs[j].wide != 0u;
     }
+    if (n_jobs == 1u) set_scene0(p, *jobs[0].scene, wide);
     if (tiles) wf_generate_kernel<<<(unsigned)((tiles + 3u) / 4u), 128, 0, st>>>(p, (uint32_t)tiles);
     WaveTuning t = tune;
     normalize_tuning(t, wide ? wide_need : stack_need);
-    ExtendKernel ext;
-    TraceKernel trc;
-    trav_kernels(t, wide, ext, trc, p.work != nullptr);
-    const size_t smem = trav_smem_bytes(t, wide);
+    const TraceKernel trc = trace_kernel(t, wide, p.work != nullptr, n_jobs > 1u);
+    const size_t smem = trav_smem_bytes(t.block_threads, wide && t.treelet);
     // A launch carries up to one path per slot plus one occlusion ray per slot.
     const uint64_t blocks_needed = (2u * slots + t.block_threads - 1u) / t.block_threads;
     const uint64_t persistent = (uint64_t)num_sms * t.blocks_per_sm;
@@ -1159,7 +1190,7 @@ cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t
     };
     for (uint32_t it = 0; it < iters; ++it) {
         mark(prof ? prof->trace_ev : nullptr, n_trc, 0);
-        trc<<<grid, t.block_threads, smem, st>>>(p, it, it ? it - 1u : kNoIter, t.chunk, t.steps | (t.refill_idle << 16));
+        trc<<<grid, t.block_threads, smem, st>>>(p, it, it ? it - 1u : kNoIter, t.chunk, trace_steps(t));
         mark(prof ? prof->trace_ev : nullptr, n_trc++, 1);
         mark(prof ? prof->shade_ev : nullptr, n_shd, 0);
         shade<<<shade_grid, 128, 0, st>>>(p, it);
@@ -1172,7 +1203,7 @@ cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t
     }
     if (iters) {
         mark(prof ? prof->trace_ev : nullptr, n_trc, 0);
-        trc<<<grid, t.block_threads, smem, st>>>(p, kNoIter, iters - 1u, t.chunk, t.steps | (t.refill_idle << 16));
+        trc<<<grid, t.block_threads, smem, st>>>(p, kNoIter, iters - 1u, t.chunk, trace_steps(t));
         mark(prof ? prof->trace_ev : nullptr, n_trc++, 1);
     }
     if (prof) {

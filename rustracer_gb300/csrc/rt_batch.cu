@@ -101,7 +101,11 @@ std::vector<unsigned char> BatchEngine::signature(rt_renderer *const *rs, uint32
         put(s, r->cfg.exposure);
         put(s, r->cfg.gamma);
         put(s, r->scene.stack_cap);
-        put(s, r->scene.wnodes);  // picks the traversal kernels
+        put(s, r->scene.wnodes);  // picks the traversal kernels; a one-job frame's launches carry the scene
+        put(s, r->scene.cnodes);
+        put(s, r->scene.tri_ord);
+        put(s, r->scene.cnode_count);
+        put(s, r->scene.any_hit_shadows);
         put(s, r->scene.wide_stack);
         put(s, r->glow);
         put(s, r->marker);
@@ -118,7 +122,8 @@ int BatchEngine::enqueue(rt_renderer *const *rs, uint32_t n, uint32_t iters, con
         shapes[j] = rtd::JobShape{r->cfg.width, r->cfg.height, r->cfg.width * r->cfg.height, base[j],
                                   r->scene.stack_cap, r->cfg.enable_photon_map ? 1u : 0u,
                                   r->cfg.debug_view != 0u ? 1u : 0u, r->scene.wnodes ? 1u : 0u,
-                                  r->scene.wide_stack};
+                                  r->scene.wide_stack,
+                                  &r->scene};
     }
     const rtd::WaveParams wp = path.params(jobs.device(), n, counters.as<unsigned long long>());
     RT_CK(rtd::launch_wavefront(wp, shapes.data(), n, iters, num_sms, tuning, stream));
@@ -314,8 +319,7 @@ int BatchEngine::autotune(rt_renderer *const *rs, uint32_t n, uint32_t trial_fra
     // Coordinate descent, one pass over the launch-shape dimensions; a change is kept when it is
     // faster by more than 2% (frame-to-frame noise).
     const uint32_t blocks[] = {64u, 128u, 256u};
-    const uint32_t per_sm[] = {2u, 4u, 6u, 8u, 12u, 16u, 24u, 32u};
-    const uint32_t stacks[] = {32u, 48u, 64u};
+    const uint32_t per_sm[] = {2u, 3u, 4u, 6u, 7u, 8u, 12u, 14u};
     const uint32_t chunks[] = {32u, 64u, 128u, 256u};
     const uint32_t steps[] = {3u, 4u, 8u, 16u};
     const uint32_t refills[] = {0u, 8u, 12u};
@@ -336,7 +340,6 @@ int BatchEngine::autotune(rt_renderer *const *rs, uint32_t n, uint32_t trial_fra
     };
     sweep(&rtd::WaveTuning::block_threads, blocks, 3);
     sweep(&rtd::WaveTuning::blocks_per_sm, per_sm, 8);
-    sweep(&rtd::WaveTuning::stack_entries, stacks, 3);
     sweep(&rtd::WaveTuning::chunk, chunks, 4);
     sweep(&rtd::WaveTuning::steps, steps, 4);
     sweep(&rtd::WaveTuning::refill_idle, refills, 3);

@@ -310,320 +310,6 @@ __device__ __forceinline__ float intersect_triangle(f3 ro, f3 rd, f3 v0, f3 v1, 
     return kInf;
 }
 
-// BVH traversal over the child-pair records.  Each record fetch tests both children's boxes with the
-// reference's slab test (gather.wgsl:71-75: (bmin - ro) / d, te <= ta && ta > 0 && te < t); leaf
-// children are intersected on the spot, internal children are visited nearest entry first with the
-// farther one pushed (a push is dropped once `stack_cap` entries are in use, as the reference drops
-// pushes at 63).  The tree is the reference's, so the closest hit is the reference's.  Triangles hit at
-// exactly equal t resolve to the lowest prim slot: leaves hold consecutive slot ranges with the left
-// child's below the right's (bvh.rs:159-219), so the reference's left-first walk, where the first
-// strictly smaller t wins, meets the lowest slot first.  During the walk st.prim holds the best prim
-// slot; trav_hit_prim gives the triangle index.  The stack lives in shared memory, one
-// 4-byte column per thread.  TravState makes the traversal resumable one record at a time, so
-// persistent warps can refill lanes whose ray finished.
-struct TravState {
-    f3 ro, rd, inv;
-    float t;
-    uint32_t prim, node, sp;  // prim: the prim slot of the best hit so far
-    const float4 *cnodes, *tri_ord;  // the traversal layout of the ray's scene
-    uint32_t cap;                    // stack entries this scene may use
-};
-
-// kWide: walk the four-wide records with the lane's whole stack (stack_entries, at least
-// s.wide_stack, so no push is dropped); otherwise the two-wide records with the reference's push
-// limit (s.stack_cap, at most stack_entries).
-template <bool kWide>
-__device__ __forceinline__ TravState trav_begin(const DevScene &s, f3 ro, f3 rd, float t_limit,
-                                                uint32_t stack_entries) {
-    TravState st;
-    st.cnodes = kWide ? s.wnodes : s.cnodes;
-    st.tri_ord = s.tri_ord;
-    st.cap = kWide ? stack_entries : s.stack_cap;
-    st.ro = ro;
-    st.rd = rd;
-    st.inv = mk3(1.0f, 1.0f, 1.0f) / rd;
-    st.t = t_limit;
-    st.prim = 0u;
-    st.node = 0u;
-    st.sp = 0u;
-    return st;
-}
-
-// One traversal step for every lane of a warp; all 32 lanes call it together.  `active` lanes visit
-// their current record.  The triangles of the record's hit leaves are tested by the whole warp: the
-// leaf work of all lanes is laid out as one list (lane order, left leaf before right leaf, triangles
-// in leaf order), cut into rounds of 32 tests, one per lane, and each lane then folds the results of
-// its own tests in list order (a test wins when its t is strictly below the best so far, or equal to it
-// with a lower prim slot), so a lane's result is what testing its leaves one by one gives.  Testing them one by
-// one in each lane instead leaves the warp waiting on the lanes with four-triangle leaves.
-//
-// Returns true for an active lane whose traversal has finished (st.t and the prim slot st.prim hold
-// the closest hit below the starting st.t).  `any` lanes (occlusion queries) also finish at the first record whose
-// leaves hold a triangle below st.t; st.t is then the smallest such t of that record.  WarpLeaves is
-// per warp, and warp_leaves_set_ray must have stored a lane's ray before its first step.
-struct WarpLeaves {
-    float4 ray[2][32];  // per lane: (ro, low half of tri_ord), (rd, high half of tri_ord)
-    uint4 leaf_ref[32];    // four-wide step: per lane the first prim slot of each hit leaf
-    uint4 leaf_start[32];  // and where its tests start in the lane's run (0xFFFFFFFF: none)
-    uint32_t owner[32];
-    float t[32];
-    uint32_t prim[32];
-};
-
-__device__ __forceinline__ void warp_leaves_set_ray(WarpLeaves &w, const TravState &st) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long tp = (unsigned long long)st.tri_ord;
-    w.ray[0][lane] = make_float4(st.ro.x, st.ro.y, st.ro.z, __uint_as_float((uint32_t)tp));
-    w.ray[1][lane] = make_float4(st.rd.x, st.rd.y, st.rd.z, __uint_as_float((uint32_t)(tp >> 32)));
-}
-
-// The leaf tests of one traversal step for the whole warp: lane l has n_l tests (its run), laid out
-// in lane order and cut into rounds of 32; tri_of(owner, j) gives the prim slot of the owner's j-th
-// test (every lane calls it, with its own arguments).  Each lane folds its own results in run order
-// into st.t / st.prim (a test wins when its t is strictly below the best so far, or equal to it with a
-// lower prim slot) and returns whether any of them won.
-template <typename TriOf>
-__device__ __forceinline__ bool warp_leaf_rounds(TravState &st, uint32_t n, WarpLeaves &w, TriOf tri_of) {
-    const uint32_t lane = threadIdx.x & 31u;
-    if (!__any_sync(0xFFFFFFFFu, n != 0u)) return false;  // no lane reached a leaf this step
-    uint32_t incl = n;
-#pragma unroll
-    for (uint32_t d = 1u; d < 32u; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-        if (lane >= d) incl += v;
-    }
-    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    const uint32_t excl = incl - n;
-    bool found = false;
-    for (uint32_t base = 0u; base < total; base += 32u) {
-        // This round tests list entries [base, base + 32); a lane owning some of them marks where its
-        // run starts, so every position finds its owner as the last start at or below it.
-        const uint32_t lo = excl > base ? excl : base;
-        const uint32_t hi = excl + n < base + 32u ? excl + n : base + 32u;
-        const bool mine = lo < hi;
-        if (mine) w.owner[lo - base] = lane;
-        const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, mine ? 1u << (lo - base) : 0u);
-        __syncwarp();
-        const uint32_t start = 31u - __clz((starts | 1u) & (0xFFFFFFFFu >> (31u - lane)));
-        const uint32_t o = w.owner[start];
-        const uint32_t o_excl = __shfl_sync(0xFFFFFFFFu, excl, o);
-        const uint32_t o_tri = tri_of(o, base + lane - o_excl);  // every lane calls: shuffles inside
-        float t = kInf;
-        uint32_t prim = 0u;
-        if (base + lane < total) {
-            const float4 r0 = w.ray[0][o], r1 = w.ray[1][o];
-            const float4 *tris = reinterpret_cast<const float4 *>(
-                ((unsigned long long)__float_as_uint(r1.w) << 32) | (unsigned long long)__float_as_uint(r0.w));
-            const uint32_t tri = o_tri;
-            const float4 *tp = tris + 3ull * tri;
-            const float4 v0 = __ldg(tp), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
-            const f3 ro = xyz(r0), rd = xyz(r1);
-            // Moller-Trumbore (common.wgsl:78-100) with the edges precomputed.
-            const f3 h3 = cross(rd, xyz(e2));
-            const float a = dot(xyz(e1), h3);
-            if (!(fabsf(a) < 1e-7f)) {
-                const float f = 1.0f / a;
-                const f3 sv = ro - xyz(v0);
-                const float u = f * dot(sv, h3);
-                if (!(u < 0.0f || u > 1.0f)) {
-                    const f3 q = cross(sv, xyz(e1));
-                    const float v = f * dot(rd, q);
-                    if (!(v < 0.0f || u + v > 1.0f)) {
-                        const float tt = f * dot(xyz(e2), q);
-                        if (tt > kEps) t = tt;
-                    }
-                }
-            }
-            prim = tri;
-        }
-        w.t[lane] = t;
-        w.prim[lane] = prim;
-        __syncwarp();
-        if (mine) {
-            for (uint32_t k = lo - base; k < hi - base; ++k) {
-                const float tk = w.t[k];
-                const uint32_t sk = w.prim[k];
-                if (tk < st.t || (tk == st.t && sk < st.prim)) {
-                    st.t = tk;
-                    st.prim = sk;
-                    found = true;
-                }
-            }
-        }
-        __syncwarp();
-    }
-    return found;
-}
-
-// tests_out (optional): the lane's leaf triangle tests of this step (the work counters of the
-// profiling kernels).
-__device__ __forceinline__ bool trav_step_warp(TravState &st, bool active, bool any, uint32_t *stk, uint32_t stride,
-                                               WarpLeaves &w, uint32_t *tests_out = nullptr) {
-    bool hl = false, hr = false;
-    float le = 0.0f, re = 0.0f;
-    uint32_t lref = 0u, lcnt = 0u, rref = 0u, rcnt = 0u;
-    if (active) {
-        const float4 *np = st.cnodes + 4ull * st.node;
-        const float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
-        const f3 ro = st.ro, inv = st.inv;
-        const f3 a0 = (xyz(q0) - ro) * inv, a1 = (xyz(q1) - ro) * inv;
-        const f3 b0 = (xyz(q2) - ro) * inv, b1 = (xyz(q3) - ro) * inv;
-        le = fmax3f(fminf(a0.x, a1.x), fminf(a0.y, a1.y), fminf(a0.z, a1.z));
-        const float lx = fmin3f(fmaxf(a0.x, a1.x), fmaxf(a0.y, a1.y), fmaxf(a0.z, a1.z));
-        re = fmax3f(fminf(b0.x, b1.x), fminf(b0.y, b1.y), fminf(b0.z, b1.z));
-        const float rx = fmin3f(fmaxf(b0.x, b1.x), fmaxf(b0.y, b1.y), fmaxf(b0.z, b1.z));
-        hl = le <= lx && lx > 0.0f && le < st.t;
-        hr = re <= rx && rx > 0.0f && re < st.t;
-        lref = __float_as_uint(q0.w);
-        lcnt = __float_as_uint(q1.w);
-        rref = __float_as_uint(q2.w);
-        rcnt = __float_as_uint(q3.w);
-    }
-    const uint32_t nl = (hl && lcnt != 0u) ? lcnt : 0u;
-    const uint32_t n = nl + ((hr && rcnt != 0u) ? rcnt : 0u);
-    if (tests_out) *tests_out = n;
-    // The next record does not depend on this record's leaf results (they only lower st.t for later
-    // box tests), so the lane moves on first and its next record is on the way to L1 while the warp
-    // tests leaves.
-    bool exhausted = false;
-    if (active) {
-        const bool il = hl && lcnt == 0u, ir = hr && rcnt == 0u;
-        if (il && ir) {
-            const bool left_first = le <= re;
-            const uint32_t far = left_first ? rref : lref;
-            st.node = left_first ? lref : rref;
-            if (st.sp < st.cap) {
-                stk[st.sp * stride] = far;
-                st.sp += 1u;
-            }
-        } else if (il) {
-            st.node = lref;
-        } else if (ir) {
-            st.node = rref;
-        } else if (st.sp == 0u) {
-            exhausted = true;
-        } else {
-            st.sp -= 1u;
-            st.node = stk[st.sp * stride];
-        }
-        if (!exhausted) asm volatile("prefetch.global.L1 [%0];" ::"l"(st.cnodes + 4ull * st.node));
-    }
-    const bool found = warp_leaf_rounds(st, n, w, [&](uint32_t o, uint32_t j) {
-        const uint32_t o_nl = __shfl_sync(0xFFFFFFFFu, nl, o);
-        const uint32_t o_lref = __shfl_sync(0xFFFFFFFFu, lref, o);
-        const uint32_t o_rref = __shfl_sync(0xFFFFFFFFu, rref, o);
-        return j < o_nl ? o_lref + j : o_rref + (j - o_nl);
-    });
-    return active && (exhausted || (any && found));
-}
-
-// trav_step_warp over the four-wide records: each active lane tests the four child boxes of its
-// record with the same slab test, queues the hit leaves' triangles (child order) for the warp's leaf
-// rounds, and visits the hit internal children nearest entry first (the others pushed, farthest
-// first; the stack holds every pending entry).  Same results as the two-wide walk: the closest hit
-// below the starting st.t, ties resolved to the lowest prim slot as in the two-wide walk.
-//
-// tree (optional): the block's treelet, the first tree_n records of the four-wide layout of the scene
-// whose records start at tree_src, staged in shared memory; a lane on that scene reads those records
-// from there (the breadth-first layout puts the top levels first).
-__device__ __forceinline__ bool trav_step_warp4(TravState &st, bool active, bool any, uint32_t *stk, uint32_t stride,
-                                                WarpLeaves &w, uint32_t *tests_out = nullptr,
-                                                const float4 *tree = nullptr, const float4 *tree_src = nullptr,
-                                                uint32_t tree_n = 0u) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n = 0u;
-    bool exhausted = false;
-    if (active) {
-        float4 q[8];
-        if (tree != nullptr && st.cnodes == tree_src && st.node < tree_n) {
-            const float4 *tp = tree + 8u * st.node;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) q[i] = tp[i];
-        } else {
-            // the 128-byte record as four 32-byte loads (records are 128-byte aligned)
-            const float4 *np = st.cnodes + 8ull * st.node;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ldg32(np + 2 * i, q[2 * i], q[2 * i + 1]);
-        }
-        const f3 ro = st.ro, inv = st.inv;
-        float key[4];
-        uint32_t ref[4];
-        // The hit leaves go straight to the lane's leaf slots (first prim slot, start of its tests in
-        // the lane's run); unused slots keep start 0xFFFFFFFF.  The previous step's readers are done
-        // (each leaf round ends at a warp barrier).
-        uint32_t *lr = &w.leaf_ref[lane].x, *ls = &w.leaf_start[lane].x;
-        w.leaf_start[lane] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-        uint32_t n_leaf = 0u;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const f3 a0 = (xyz(q[2 * c]) - ro) * inv, a1 = (xyz(q[2 * c + 1]) - ro) * inv;
-            const float te = fmax3f(fminf(a0.x, a1.x), fminf(a0.y, a1.y), fminf(a0.z, a1.z));
-            const float tx = fmin3f(fmaxf(a0.x, a1.x), fmaxf(a0.y, a1.y), fmaxf(a0.z, a1.z));
-            const uint32_t cref = __float_as_uint(q[2 * c].w), cnt = __float_as_uint(q[2 * c + 1].w);
-            const bool hit = cnt != 0xFFFFFFFFu && te <= tx && tx > 0.0f && te < st.t;
-            ref[c] = cref;
-            key[c] = (hit && cnt == 0u) ? te : __int_as_float(0x7F800000);  // +inf: not a pending child
-            if (hit && cnt != 0u) {
-                lr[n_leaf] = cref;
-                ls[n_leaf] = n;
-                n_leaf += 1u;
-                n += cnt;
-            }
-        }
-        // Near-first order of the hit internal children (a fixed five-exchange network).
-        auto cswap = [&](int i, int j) {
-            if (key[j] < key[i]) {
-                const float tk = key[i];
-                key[i] = key[j];
-                key[j] = tk;
-                const uint32_t tr = ref[i];
-                ref[i] = ref[j];
-                ref[j] = tr;
-            }
-        };
-        cswap(0, 1);
-        cswap(2, 3);
-        cswap(0, 2);
-        cswap(1, 3);
-        cswap(1, 2);
-        const float kNone = __int_as_float(0x7F800000);
-        const uint32_t m = (key[0] < kNone ? 1u : 0u) + (key[1] < kNone ? 1u : 0u) + (key[2] < kNone ? 1u : 0u) +
-                           (key[3] < kNone ? 1u : 0u);
-        if (m != 0u) {
-            st.node = ref[0];
-#pragma unroll
-            for (int i = 3; i >= 1; --i)
-                if ((uint32_t)i < m && st.sp < st.cap) {
-                    stk[st.sp * stride] = ref[i];
-                    st.sp += 1u;
-                }
-        } else if (st.sp == 0u) {
-            exhausted = true;
-        } else {
-            st.sp -= 1u;
-            st.node = stk[st.sp * stride];
-        }
-        if (!exhausted && !(tree != nullptr && st.cnodes == tree_src && st.node < tree_n))
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(st.cnodes + 8ull * st.node));
-    }
-    if (tests_out) *tests_out = n;
-    const bool found = warp_leaf_rounds(st, n, w, [&](uint32_t o, uint32_t j) {
-        const uint4 r = w.leaf_ref[o], b = w.leaf_start[o];
-        const uint32_t i = (j >= b.y ? 1u : 0u) + (j >= b.z ? 1u : 0u) + (j >= b.w ? 1u : 0u);
-        const uint32_t first = i == 0u ? r.x : (i == 1u ? r.y : (i == 2u ? r.z : r.w));
-        const uint32_t at = i == 0u ? b.x : (i == 1u ? b.y : (i == 2u ? b.z : b.w));
-        return first + (j - at);
-    });
-    return active && (exhausted || (any && found));
-}
-
-// The triangle index of a finished closest-hit traversal (st.prim holds the hit's prim slot; a miss
-// gives 0).
-__device__ __forceinline__ uint32_t trav_hit_prim(const TravState &st) {
-    return st.t < kInf ? __float_as_uint(__ldg(st.tri_ord + 3ull * st.prim).w) : 0u;
-}
-
-
 struct Bary {
     float uvx, uvy, u, v;
 };

@@ -47,6 +47,10 @@ struct WaveParams {
     // Work counters of the profiling traversal kernels (null otherwise): traversal records visited
     // by closest-hit / occlusion rays, then their leaf triangle tests.
     unsigned long long *work;
+    // The traversal layout of a one-job launch's scene (its records, leaf-ordered triangles), whether its
+    // occlusion rays may stop at any hit, and whether it has no triangles; filled by the launchers.
+    const float4 *records0, *tris0;
+    uint32_t any_hit0, empty0;
 };
 // Host-side shape of a job for the per-job launches.
 struct JobShape {
@@ -55,6 +59,7 @@ struct JobShape {
     uint32_t debug;    // the job renders a debug view (rt_image_params._pad[0] != 0)
     uint32_t wide;     // the job's scene has four-wide records (DevScene.wnodes)
     uint32_t wide_stack;  // stack entries a walk of them can need
+    const DevScene *scene;  // the job's scene (a host copy; its arrays are on the device)
 };
 // Launch shape of the persistent traversal kernels (extend, shadow); no effect on any result.
 struct WaveTuning {
@@ -62,7 +67,7 @@ struct WaveTuning {
     uint32_t blocks_per_sm;  // persistent blocks per SM (the grid is capped by the work)
     uint32_t chunk;          // queue items a warp takes per atomic: its segment of the queue
     uint32_t steps;          // traversal records between lane refills
-    uint32_t stack_entries;  // shared-memory stack per lane: 32, 48 or 64 (raised to the jobs' need)
+    uint32_t stack_entries;  // 32, 48 or 64 (raised to the jobs' need); no kernel depends on it
     uint32_t treelet;        // four-wide records at the top of the tree staged in shared memory per
                              // block: 0 or kTreeletRecords
     uint32_t shade_blocks;   // shade kernel compiled for 4, 5 or 6 resident blocks of 128 per SM
@@ -70,7 +75,7 @@ struct WaveTuning {
                              // idle (0: only after `steps`)
 };
 // Records of the treelet: the first records of the breadth-first four-wide layout (the root, its
-// children and most of their children), 2 KB, which fits beside 8 blocks of 128 traversal threads.
+// children and most of their children), 2 KB.
 constexpr uint32_t kTreeletRecords = 16;
 WaveTuning default_tuning();
 // Clamps a tuning to supported values (stack raised to `stack_need`); false if it had to change.
@@ -103,7 +108,7 @@ struct PhotonWave {
     float4 *ro;        // origin, .w = RNG state
     float4 *rd;        // direction, .w = photon index
     float4 *pw;        // power, .w = job index 0 (read by the shared closest-hit kernel)
-    float2 *hit;       // closest t, primitive
+    float2 *hit;       // closest t, the hit's prim slot
     uint32_t *queue[2];
     uint32_t *counts;  // 4 per bounce (+1): [0] photons queued, [2] fetch cursor of the hit kernel
 };
@@ -115,7 +120,7 @@ PhotonWave photon_wave_at(void *base, uint32_t n);
 // The photon pass (photon_trace.wgsl:91-260) as a wavefront: jobs_dev[0].scene must be p.scene.
 cudaError_t launch_photon_wave(const PhotonTraceParams &p, const PhotonWave &w, const DevJob *jobs_dev, int num_sms,
                                const WaveTuning &tune, cudaStream_t st);
-// One closest-hit pass of the persistent traversal kernel over queue[iter & 1] (count at
+// One pass of the persistent traversal kernel over the closest-hit rays of queue[iter & 1] (count at
 // counts[4 iter]); `max_items` bounds the grid.
 cudaError_t launch_extend(const WaveParams &p, uint32_t iter, uint64_t max_items, const DevScene &scene, int num_sms,
                           const WaveTuning &tune, cudaStream_t st);

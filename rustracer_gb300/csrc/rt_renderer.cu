@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -381,6 +382,20 @@ int resident_scene_create(const rt_scene_desc *sd, rt_resident_scene **out) {
     if (rt::traversal_width() == 4u && sd->bvh_node_count > 0) {
         rt::build_wide_layout(sd->bvh_nodes, sd->bvh_node_count, wide);
         if (wide.stack_need > 64u) wide.nodes.clear();
+        // The device order of a child's 32 bytes, (min.x, max.x, min.y, max.y, min.z, max.z, ref, count);
+        // empty places get a NaN box, on which no slab test passes, so the kernels need no check for them.
+        for (size_t c = 0; c < wide.nodes.size(); c += 8) {
+            float *n = &wide.nodes[c], o[8];
+            uint32_t count;
+            std::memcpy(&count, n + 7, 4);
+            for (int a = 0; a < 3; ++a) {
+                o[2 * a] = count == 0xFFFFFFFFu ? std::numeric_limits<float>::quiet_NaN() : n[a];
+                o[2 * a + 1] = count == 0xFFFFFFFFu ? std::numeric_limits<float>::quiet_NaN() : n[4 + a];
+            }
+            std::memcpy(o + 6, n + 3, 4);
+            std::memcpy(o + 7, n + 7, 4);
+            std::memcpy(n, o, sizeof(o));
+        }
         if (!wide.nodes.empty() && (st = upload(res->d_wnodes, wide.nodes.data(), wide.nodes.size(), s)) != RT_OK)
             return fail(st);
     }
@@ -647,7 +662,8 @@ extern "C" int rt_render_frame(rt_renderer *r) {
                                   c.enable_photon_map ? 1u : 0u,
                                   c.debug_view != 0u ? 1u : 0u,
                                   r->scene.wnodes ? 1u : 0u,
-                                  r->scene.wide_stack};
+                                  r->scene.wide_stack,
+                                  &r->scene};
         if (r->prof_flags) {
             if (int st = rt::profiled_gather(r, wp, shape, iters)) return st;
         } else {
