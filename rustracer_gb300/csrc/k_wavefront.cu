@@ -43,6 +43,12 @@ struct PathAcc {
     f3 col;
     float lum_sum, lum2_sum, sl;
 };
+// The NEE term of a path's last bounce waits in its slot (p.nee: the contribution and a word) until its
+// occlusion ray has been traced: kNeeLit is set if the light is visible, and the slot's next shade (or
+// finalize) adds the term first of all.  The word's low bits: the sample it belongs to, and whether only
+// its luminance counts (photon debug).
+constexpr uint32_t kNeePending = 0x20000u, kNeeLumaOnly = 0x10000u, kNeeLit = 0x80000000u;
+
 __device__ __forceinline__ void add_radiance(uint32_t s, PathAcc &a, f3 c) {
     a.col = a.col + c;
     float l = luma(c);
@@ -66,6 +72,19 @@ __device__ __forceinline__ void acc_add_term(const WaveParams &p, uint32_t slot,
     a[0] = a0;
     *lum2 += l * l;
     if (s < 8u) reinterpret_cast<float *>(a + 2)[s] += l;
+}
+// A lit NEE term added to a slot's accumulator, whose words for sample s0 are in A.
+__device__ __forceinline__ void add_nee(const float4 &nee, float4 *acc, uint32_t s0, PathAcc &A) {
+    const uint32_t word = __float_as_uint(nee.w), s = word & 0xFFFFu;
+    const f3 c = xyz(nee);
+    const float l = luma(c);
+    if (!(word & kNeeLumaOnly)) A.col = A.col + c;
+    A.lum_sum += l;
+    A.lum2_sum += l * l;
+    if (s < 8u) {
+        if (s == s0) A.sl += l;
+        else reinterpret_cast<float *>(acc + 2)[s] += l;  // the sample that ended with this term
+    }
 }
 __device__ __forceinline__ Accum load_acc(const WaveParams &p, uint32_t pix) {
     const float4 a = p.acc[4 * (size_t)pix], b = p.acc[4 * (size_t)pix + 1], c = p.acc[4 * (size_t)pix + 2],
@@ -263,6 +282,7 @@ __global__ void __launch_bounds__(128) wf_generate_kernel(const __grid_constant_
         p.acc[4 * (size_t)slot + 2] = z;
         p.acc[4 * (size_t)slot + 3] = z;
         p.nrm[slot] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+        p.nee[slot] = z;
     }
     warp_append(active, slot, p.queue[0], p.counts + 0);
 }
@@ -353,9 +373,8 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         f3 ph_hp = mk3(0.0f, 0.0f, 0.0f), ph_n = ph_hp, ph_td = ph_hp;
         uint32_t ph_sidx = 0;
         uint32_t slot = 0;
-        f3 sh_o = mk3(0.0f, 0.0f, 0.0f), sh_d = sh_o, sh_c = sh_o;
+        f3 sh_o = mk3(0.0f, 0.0f, 0.0f), sh_d = sh_o;
         float sh_max = 0.0f;
-        uint32_t sh_tag = 0;
         if (valid) {
             slot = q[i];
             const float4 o4 = p.ro[slot], d4 = p.rd[slot], t4 = p.thr[slot];
@@ -381,9 +400,11 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
             const uint32_t prim = s_orig[threadIdx.x];  // the hit triangle (h2.y holds its prim slot)
             float4 *acc = p.acc + 4 * (size_t)slot;
             const uint32_t sidx0 = sidx;
-            const float4 acc0 = acc[0];
+            const float4 acc0 = acc[0], nee = p.nee[slot];
             float4 acc1 = acc[1];  // .x = lum2_sum, .y = first_depth
             PathAcc A{xyz(acc0), acc0.w, acc1.x, sidx0 < 8u ? reinterpret_cast<const float *>(acc + 2)[sidx0] : 0.0f};
+            const uint32_t nee_word = __float_as_uint(nee.w);
+            if (nee_word & kNeeLit) add_nee(nee, acc, sidx0, A);
             bool first_hit = false;  // this step found a nearer first hit (normal and depth change)
             float4 nrm = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             bool alive = true;  // the sample continues with another segment
@@ -541,9 +562,10 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
                             emit_shadow = true;
                             sh_o = ls.o;
                             sh_d = ls.wi;
-                            sh_c = c_nee;
                             sh_max = ls.max_dist;
-                            sh_tag = (sidx & 0xFFFFu) | (nee_luma_only ? 0x10000u : 0u) | (jid << 17);
+                            p.nee[slot] = make_float4(c_nee.x, c_nee.y, c_nee.z,
+                                                      __uint_as_float((sidx & 0xFFFFu) | kNeePending |
+                                                                      (nee_luma_only ? kNeeLumaOnly : 0u)));
                         }
                         if (do_spec) {
                             rd = sample_spec_dir(rd, shn, a, rng);
@@ -580,6 +602,7 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
             } else {
                 keep = true;
             }
+            if (!emit_shadow && nee_word != 0u) p.nee[slot].w = 0.0f;
             p.ro[slot] = make_float4(ro.x, ro.y, ro.z, __uint_as_float(rng.state));
             p.rd[slot] = make_float4(rd.x, rd.y, rd.z, __uint_as_float(pack_sb(sidx, b)));
             p.thr[slot] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(jid));
@@ -618,10 +641,9 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         __syncthreads();
         // NEE shadow ray (deferred) and the photon-map lookup request.
         if (emit_shadow) {
-            float4 *rec = p.shadow + 3ull * s_spos[li];
+            float4 *rec = p.shadow + 2ull * s_spos[li];
             rec[0] = make_float4(sh_o.x, sh_o.y, sh_o.z, sh_max);
             rec[1] = make_float4(sh_d.x, sh_d.y, sh_d.z, __uint_as_float(slot));
-            rec[2] = make_float4(sh_c.x, sh_c.y, sh_c.z, __uint_as_float(sh_tag));
         }
         if (kPhotons && emit_photon) {
             float4 *rec = p.preq + 3ull * s_ppos[li];
@@ -721,31 +743,29 @@ __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------------------------------------
-// shadow: the deferred NEE occlusion test (gather.wgsl:91-103) and the contribution of visible lights.
+// shadow: the deferred NEE occlusion test (gather.wgsl:91-103); a visible light marks its slot's NEE term.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float shadow_limit(float max_dist) { return max_dist - 0.001f; }
 // The triangle of a closest hit (prim: its slot); a miss gives 0.
 __device__ __forceinline__ uint32_t slot_triangle(const DevScene &s, float t, uint32_t prim) {
     return t < kInf ? __float_as_uint(__ldg(s.tri_ord + 3ull * prim).w) : 0u;
 }
-// The reference's alpha rule of scenes with cut-out materials: whether the ray's closest hit (t, its prim
-// slot) lets the light through.  Out of line: few scenes need it, and its registers would weigh on the
-// traversal.
-__device__ __noinline__ bool cut_out_hit(const DevScene &s, f3 o, f3 d, float t, uint32_t prim) {
-    const TriFull bt = load_tri(s, slot_triangle(s, t, prim));
+// Whether the light of an occlusion ray in a scene with cut-out materials is visible (gather.wgsl:91-103):
+// its closest hit (hit_word) lies at or beyond the limit, or is cut away there by its texture's alpha.  Out of
+// line: few scenes need it, and its registers would weigh on the traversal.
+__device__ __noinline__ bool cut_out_lit(const DevScene &s, float4 ro, float4 rd, float limit,
+                                         unsigned long long hit) {
+    const float t = hit_t(hit);
+    if (t >= limit) return true;  // (not for a NaN limit, which counts as occluded)
+    const TriFull bt = load_tri(s, t < kInf ? __float_as_uint(__ldg(s.tri_ord + 3ull * (uint32_t)hit).w) : 0u);
     const Mat bm = load_mat(s, bt.material_id);
     if ((bm.flags & RT_MAT_FLAG_ALPHA_CUTOUT) == 0u || bm.tex_albedo == RT_TEX_NONE) return false;
-    const Bary b = barycentric(bt, o, d, t);
+    const Bary b = barycentric(bt, xyz(ro), xyz(rd), t);
     return tex_sample(s.tex[RT_TEX_ALBEDO], b.uvx, b.uvy, (int32_t)bm.tex_albedo).w < 0.5f;
 }
-// t: the ray's closest hit (occlusion rays that may stop early: any hit below the limit), prim its slot.
-__device__ __forceinline__ void shadow_resolve(const WaveParams &p, uint32_t rec_i, float t, uint32_t prim) {
-    const float4 o = p.shadow[3ull * rec_i], d = p.shadow[3ull * rec_i + 1], c = p.shadow[3ull * rec_i + 2];
-    const uint32_t tag = __float_as_uint(c.w);
-    const DevScene &s = p.jobs[tag >> 17].scene;
-    if (!(t >= shadow_limit(o.w)) && (s.any_hit_shadows || !cut_out_hit(s, xyz(o), xyz(d), t, prim))) return;
-    acc_add_term(p, __float_as_uint(d.w), tag & 0xFFFFu, xyz(c), (tag & 0x10000u) != 0u);
-}
+
+// How far a ray that looks for its closest hit below a limit searches: a little beyond it, so that
+// rounding in a box's entry cannot lose a hit before it.
+__device__ __forceinline__ float search_limit(float limit) { return limit > kEps ? limit * 1.001f : kInf; }
 
 // trace: the occlusion rays of iteration `shd_iter` and the closest-hit rays of iteration `ext_iter` in
 // one persistent launch (either may be kNoIter).  Both depend only on the shade pass before them and
@@ -753,7 +773,7 @@ __device__ __forceinline__ void shadow_resolve(const WaveParams &p, uint32_t rec
 // them with one tail instead of two.  Closest-hit rays come first in the work list: the longer rays
 // start early and the shorter occlusion rays fill the end.
 constexpr uint32_t kNoIter = 0xFFFFFFFFu;
-constexpr uint32_t kOcclusion = 0x80000000u;  // ray id: shadow record (else path slot)
+constexpr uint32_t kOcclusion = 0x80000000u;  // ray id: path slot, and whether it is the slot's occlusion ray
 
 // Each lane of a warp walks its own ray, `steps` records at a time; then finished lanes write their
 // result and take new rays.  The warp is bound by instruction issue and by the latency of its record
@@ -770,7 +790,9 @@ constexpr uint32_t kOcclusion = 0x80000000u;  // ray id: shadow record (else pat
 // memory (after the stacks and the WarpTravs), and lanes on that scene read them from there.
 // kMulti: the launch's jobs may be on different scenes (each ray carries its own); otherwise the scene
 // comes with the launch, which saves four registers and the job table's loads for every ray.
-template <int kBlock, bool kWide, bool kCount, int kTree, bool kMulti>
+// kCut: scenes of the launch may have cut-out materials.  Without them every occlusion ray may stop at its
+// first hit, and the call of the alpha rule with its spills goes.
+template <int kBlock, bool kWide, bool kCount, int kTree, bool kMulti, bool kCut>
 __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __grid_constant__ WaveParams p, uint32_t ext_iter,
                                                           uint32_t shd_iter, uint32_t chunk, uint32_t steps) {
     extern __shared__ __align__(16) unsigned char trav_smem[];
@@ -818,7 +840,7 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
             items = min(32u, end - item);
             if (lane < items) {
                 if (item + lane < n_ext) cp_async4(&w.next_queue[lane], q + item + lane);
-                else w.next_queue[lane] = (item + lane - n_ext) | kOcclusion;
+                else cp_async4(&w.next_queue[lane], &p.shadow[2ull * (item + lane - n_ext) + 1].w);  // its slot
             }
         }
         __syncwarp();
@@ -826,19 +848,20 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
             w.item = item + items;
             w.seg_end = end;
             w.items = items;
+            w.first = item;
         }
     };
     // Starts the copy of the next rays (all the copied ones are claimed) and reads on.
     auto request = [&]() {
         const uint32_t items = w.items;
         if (lane < items) {
-            const uint32_t r = w.next_queue[lane], i = r & ~kOcclusion;
-            const bool occ = (r & kOcclusion) != 0u;
-            const float4 *rec = p.shadow + 3ull * i;
-            cp_async16(&w.next_ro[lane], occ ? rec : p.ro + i);
-            cp_async16(&w.next_rd[lane], occ ? rec + 1 : p.rd + i);
-            w.next_inv[lane].w = __uint_as_float(r);
-            if (kMulti) cp_async4(&w.next_inv[lane].x, occ ? &rec[2].w : &p.thr[i].w);
+            const uint32_t slot = w.next_queue[lane], item = w.first + lane, n_ext = w.n_ext;
+            const bool occ = item >= n_ext;
+            const float4 *rec = p.shadow + 2ull * (item - n_ext);
+            cp_async16(&w.next_ro[lane], occ ? rec : p.ro + slot);
+            cp_async16(&w.next_rd[lane], occ ? rec + 1 : p.rd + slot);
+            w.next_inv[lane].w = __uint_as_float(occ ? slot | kOcclusion : slot);
+            if (kMulti) cp_async4(&w.next_inv[lane].x, &p.thr[slot].w);
         }
         __syncwarp();
         if (lane == 0u) w.coming = items;
@@ -854,11 +877,19 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
 
     TravLane st;
     uint32_t id = 0u;
-    bool busy = false, visiting = false, any_hit = false;
+    bool busy = false, visiting = false, any_hit = false, found = false;
+    bool careful = false, held = false;   // walked again; waits for its leaves' tests
     uint32_t queued = 0u;                 // leaves in the warp's queue
     uint32_t work[4] = {0u, 0u, 0u, 0u};  // kCount: records closest / occlusion, tests closest / occlusion
-    st.node = 0u;
-    st.sp = 0u;
+    // The lane's ray starts at the root with st.t, and no hit yet.
+    auto begin = [&]() {
+        w.best[lane] = hit_word(st.t, 0u);
+        // (an occlusion ray that may stop early takes no interest in hits beyond its limit)
+        w.second[lane] = any_hit ? __float_as_uint(st.t) : 0x7F800000u;
+        st.node = 0u;
+        st.te = -kInf;
+        st.sp = 0u;
+    };
     // Records between refills (low 16 bits), fewer once `few` or less lanes still walk.
     const uint32_t max_steps = steps & 0xFFFFu;
     const int few = (int)(steps >> 16);
@@ -874,10 +905,7 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
                     const f3 inv = mk3(1.0f, 1.0f, 1.0f) / xyz(w.next_rd[lane]);
                     const float4 x = w.next_inv[lane];
                     w.next_inv[lane] = make_float4(inv.x, inv.y, inv.z, x.w);
-                    if (kMulti) {
-                        const uint32_t word = __float_as_uint(x.x);  // path: its job; shadow record: its tag
-                        w.next_rd[lane].w = __uint_as_float((__float_as_uint(x.w) & kOcclusion) ? word >> 17 : word);
-                    }
+                    if (kMulti) w.next_rd[lane].w = x.x;
                 }
                 at = 0u;
                 ready = coming;
@@ -908,23 +936,27 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
                         any = sc.any_hit_shadows;
                         empty = sc.cnode_count == 0u;
                     }
-                    // Without cut-out materials the occlusion test may stop at the first triangle below
-                    // the limit; with them the reference's closest-hit-then-alpha rule is kept.
-                    any_hit = occ && any != 0u;
-                    st.t = any_hit ? shadow_limit(o.w) : kInf;
+                    // An occlusion ray asks for hits below the limit: any one without cut-out materials, the
+                    // closest with them (the reference's closest-hit-then-alpha rule; looked for a little
+                    // beyond the limit, so that rounding in a box's entry cannot lose a hit before it).
+                    any_hit = occ && (!kCut || any != 0u);
+                    found = false;
+                    st.t = occ ? o.w - 0.001f : kInf;
+                    if (kCut && occ && !any_hit) {
+                        w.limit[lane] = st.t;
+                        st.t = search_limit(st.t);
+                    }
                     const unsigned long long tp = (unsigned long long)tris;
                     w.ro[lane] = make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)tp));
                     w.rd[lane] = make_float4(d.x, d.y, d.z, __uint_as_float((uint32_t)(tp >> 32)));
-                    w.best[lane] = hit_word(st.t, 0u);
                     st.minus_ro[0] = pack2(-o.x, -o.x);
                     st.minus_ro[1] = pack2(-o.y, -o.y);
                     st.minus_ro[2] = pack2(-o.z, -o.z);
                     st.inv[0] = pack2(v.x, v.x);
                     st.inv[1] = pack2(v.y, v.y);
                     st.inv[2] = pack2(v.z, v.z);
-                    st.node = 0u;
-                    st.te = -kInf;
-                    st.sp = 0u;
+                    begin();
+                    careful = false;
                     busy = true;
                     // No triangle counts below kEps, so a limit at or below it (or a NaN) is never met: the
                     // ray ends as it starts, and so does any ray of an empty scene.
@@ -941,8 +973,12 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
         for (uint32_t k = 0;;) {
             uint32_t tests = 0u;
             if (kCount && visiting) work[(id & kOcclusion) ? 1 : 0] += 1u;
-            trav_step<kWide, kTree, kBlock, kMulti>(st, top, deep, visiting, w, queued, tree, p.records0, tests);
+            trav_step<kWide, kTree, kBlock, kMulti>(st, top, deep, visiting, careful, w, queued, tree, p.records0, tests);
             if (kCount) work[(id & kOcclusion) ? 3 : 2] += tests;
+            if (careful && tests != 0u) {
+                held = visiting;
+                visiting = false;
+            }
             const bool end = ++k >= max_steps || __popc(__ballot_sync(0xFFFFFFFFu, visiting)) <= few;
             if (queued >= 8u || (end && queued != 0u)) {
                 const uint32_t tested = end ? queued : queued & ~7u, left = queued - tested;
@@ -957,19 +993,48 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
                 queued = left;
                 if (busy) {
                     const float t = hit_t(w.best[lane]);
-                    if (any_hit && t < st.t) visiting = false;
+                    if (t < st.t) {
+                        found = true;
+                        if (any_hit) visiting = false;
+                    }
                     st.t = t;
-                    if (visiting) visiting = trav_settle<kBlock>(st, top, deep);
+                    if (visiting || held) visiting = trav_settle<kBlock>(st, top, deep);
+                    held = false;
                 }
             }
             if (end) break;
         }
-        if (busy && !visiting) {
-            const uint32_t prim = (uint32_t)w.best[lane];
-            if (id & kOcclusion) shadow_resolve(p, id & ~kOcclusion, st.t, prim);
-            else p.hit[id] = make_float2(st.t, __uint_as_float(prim));  // the hit's prim slot
+        if (busy && !visiting) do {
+            const uint32_t slot = id & ~kOcclusion;
+            bool lit = !found && st.t == st.t;  // (a NaN limit counts as occluded)
+            if (!any_hit) {
+                const unsigned long long hit = w.best[lane];
+                float margin = p.tie_margin0;
+                if (kMulti) margin = p.jobs[__float_as_uint(p.thr[slot].w)].scene.tie_margin;
+                const float t = hit_t(hit);
+                bool again = !careful && __uint_as_float(w.second[lane]) <= t + (t * kTieRelative + margin);
+                if (again) {
+                    const float4 ro = w.ro[lane], rd = w.rd[lane];
+                    const float4 *tris = p.tris0;
+                    if (kMulti) tris = ray_triangles(ro, rd);
+                    again = !(hit_entry_bound(tris, (uint32_t)hit, xyz(ro), xyz(rd), margin * 0x1p-5f) <
+                              __uint_as_float(w.second[lane]));
+                }
+                if (again) {  // from the root
+                    st.t = kCut && (id & kOcclusion) ? search_limit(w.limit[lane]) : kInf;
+                    begin();
+                    careful = visiting = true;
+                    continue;
+                }
+                if (kCut && (id & kOcclusion))
+                    lit = cut_out_lit(p.jobs[__float_as_uint(p.thr[slot].w)].scene, w.ro[lane], w.rd[lane], w.limit[lane],
+                                      hit);
+                else  // the hit's prim slot
+                    p.hit[slot] = make_float2(t, __uint_as_float((uint32_t)hit));
+            }
+            if ((id & kOcclusion) && lit) atomicOr(reinterpret_cast<uint32_t *>(&p.nee[slot].w), kNeeLit);
             busy = false;
-        }
+        } while (false);
     }
     if (kCount && p.work) {
 #pragma unroll
@@ -994,6 +1059,17 @@ __global__ void __launch_bounds__(256) wf_finalize_kernel(const __grid_constant_
     if (pix >= job.npix) return;
     const uint32_t spp = job.spp;
     Accum A = load_acc(p, slot);
+    const float4 nee = p.nee[slot];
+    if (__float_as_uint(nee.w) & kNeeLit) {  // the last bounce's term
+        const uint32_t word = __float_as_uint(nee.w), s = word & 0xFFFFu;
+        const float l = luma(xyz(nee));
+        if (!(word & kNeeLumaOnly)) A.col = A.col + xyz(nee);
+        A.lum_sum += l;
+        A.lum2_sum += l * l;
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; ++i)
+            if (i == s) A.sl[i] += l;
+    }
     const float first_depth = p.acc[4 * (size_t)slot + 1].y;
     const float4 nrm = p.nrm[slot];
     if (spp <= 8u) {
@@ -1078,22 +1154,28 @@ size_t trav_smem_bytes(uint32_t block_threads, bool tree) {
 // wf_trace_kernel's `steps`.
 uint32_t trace_steps(const WaveTuning &t) { return t.steps | (t.refill_idle ? 32u - t.refill_idle : 0u) << 16; }
 
-// multi: the jobs may be on different scenes.  The counting and treelet variants are compiled for that
-// case only, which covers the other.
+// multi: the jobs may be on different scenes; cut: some may have cut-out materials.  The two-wide, counting
+// and treelet variants are compiled for both only, which covers the rest.
 template <int kBlock>
-TraceKernel trace_kernel_of(bool wide, bool count, bool tree, bool multi) {
+TraceKernel trace_kernel_of(bool wide, bool count, bool tree, bool multi, bool cut) {
     constexpr int kT = (int)kTreeletRecords;
-    if (!wide) return count ? wf_trace_kernel<kBlock, false, true, 0, true> : wf_trace_kernel<kBlock, false, false, 0, true>;
-    if (tree) return count ? wf_trace_kernel<kBlock, true, true, kT, true> : wf_trace_kernel<kBlock, true, false, kT, true>;
-    if (count) return wf_trace_kernel<kBlock, true, true, 0, true>;
-    return multi ? wf_trace_kernel<kBlock, true, false, 0, true> : wf_trace_kernel<kBlock, true, false, 0, false>;
+    if (!wide)
+        return count ? wf_trace_kernel<kBlock, false, true, 0, true, true>
+                     : wf_trace_kernel<kBlock, false, false, 0, true, true>;
+    if (tree)
+        return count ? wf_trace_kernel<kBlock, true, true, kT, true, true>
+                     : wf_trace_kernel<kBlock, true, false, kT, true, true>;
+    if (count) return wf_trace_kernel<kBlock, true, true, 0, true, true>;
+    if (multi)
+        return cut ? wf_trace_kernel<kBlock, true, false, 0, true, true> : wf_trace_kernel<kBlock, true, false, 0, true, false>;
+    return cut ? wf_trace_kernel<kBlock, true, false, 0, false, true> : wf_trace_kernel<kBlock, true, false, 0, false, false>;
 }
 
-TraceKernel trace_kernel(const WaveTuning &t, bool wide, bool count, bool multi) {
+TraceKernel trace_kernel(const WaveTuning &t, bool wide, bool count, bool multi, bool cut) {
     const bool tree = wide && t.treelet != 0u;
-    if (t.block_threads == 64u) return trace_kernel_of<64>(wide, count, tree, multi);
-    if (t.block_threads == 256u) return trace_kernel_of<256>(wide, count, tree, multi);
-    return trace_kernel_of<128>(wide, count, tree, multi);
+    if (t.block_threads == 64u) return trace_kernel_of<64>(wide, count, tree, multi, cut);
+    if (t.block_threads == 256u) return trace_kernel_of<256>(wide, count, tree, multi, cut);
+    return trace_kernel_of<128>(wide, count, tree, multi, cut);
 }
 
 }  // namespace
@@ -1101,12 +1183,13 @@ TraceKernel trace_kernel(const WaveTuning &t, bool wide, bool count, bool multi)
 void prepare_wavefront_kernels() {
     // Blocks above 48 KB of dynamic shared memory need the opt-in; set it for every variant.
     for (uint32_t block : {64u, 128u, 256u})
-        for (int v = 0; v < 16; ++v) {
+        for (int v = 0; v < 32; ++v) {
             const bool wide = (v & 1) != 0, count = (v & 2) != 0, multi = (v & 4) != 0, tree = wide && (v & 8) != 0;
+            const bool cut = (v & 16) != 0;
             WaveTuning t = default_tuning();
             t.block_threads = block;
             t.treelet = tree ? kTreeletRecords : 0u;
-            cudaFuncSetAttribute(reinterpret_cast<const void *>(trace_kernel(t, wide, count, multi)),
+            cudaFuncSetAttribute(reinterpret_cast<const void *>(trace_kernel(t, wide, count, multi, cut)),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trav_smem_bytes(block, tree));
         }
 }
@@ -1117,6 +1200,7 @@ void set_scene0(WaveParams &p, const DevScene &scene, bool wide) {
     p.tris0 = scene.tri_ord;
     p.any_hit0 = scene.any_hit_shadows;
     p.empty0 = scene.cnode_count == 0u ? 1u : 0u;
+    p.tie_margin0 = scene.tie_margin;
 }
 }  // namespace
 
@@ -1130,7 +1214,7 @@ cudaError_t launch_extend(const WaveParams &params, uint32_t iter, uint64_t max_
     const uint64_t blocks_needed = (max_items + t.block_threads - 1u) / t.block_threads;
     const uint64_t persistent = (uint64_t)num_sms * t.blocks_per_sm;
     const uint32_t grid = (uint32_t)(blocks_needed < persistent ? (blocks_needed ? blocks_needed : 1u) : persistent);
-    trace_kernel(t, wide, false, false)<<<grid, t.block_threads, trav_smem_bytes(t.block_threads, wide && t.treelet), st>>>(
+    trace_kernel(t, wide, false, false, false)<<<grid, t.block_threads, trav_smem_bytes(t.block_threads, wide && t.treelet), st>>>(
         p, iter, kNoIter, t.chunk, trace_steps(t));
     return cudaGetLastError();
 }
@@ -1143,6 +1227,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     uint64_t slots = 0;
     uint32_t stack_need = 0, wide_need = 0;
     bool wide = n_jobs > 0;  // four-wide records when every job's scene has them
+    bool cut = false;
     uint64_t tiles = 0;
     for (uint32_t j = 0; j < n_jobs; ++j) {
         tiles += ((jobs[j].width + 7u) / 8u) * ((jobs[j].height + 3u) / 4u);
@@ -1150,12 +1235,13 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         stack_need = jobs[j].stack_cap > stack_need ? jobs[j].stack_cap : stack_need;
         wide_need = jobs[j].wide_stack > wide_need ? jobs[j].wide_stack : wide_need;
         wide = wide && jobs[j].wide != 0u;
+        cut = cut || jobs[j].scene->any_hit_shadows == 0u;
     }
     if (n_jobs == 1u) set_scene0(p, *jobs[0].scene, wide);
     if (tiles) wf_generate_kernel<<<(unsigned)((tiles + 3u) / 4u), 128, 0, st>>>(p, (uint32_t)tiles);
     WaveTuning t = tune;
     normalize_tuning(t, wide ? wide_need : stack_need);
-    const TraceKernel trc = trace_kernel(t, wide, p.work != nullptr, n_jobs > 1u);
+    const TraceKernel trc = trace_kernel(t, wide, p.work != nullptr, n_jobs > 1u, cut);
     const size_t smem = trav_smem_bytes(t.block_threads, wide && t.treelet);
     // A launch carries up to one path per slot plus one occlusion ray per slot.
     const uint64_t blocks_needed = (2u * slots + t.block_threads - 1u) / t.block_threads;

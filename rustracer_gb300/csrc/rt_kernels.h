@@ -41,16 +41,18 @@ struct WaveParams {
     float4 *nrm;       // first-hit shading normal
     uint32_t *queue[2];
     uint32_t *counts;  // per iteration: [0] paths queued, [1] shadow rays, [2] trace cursor, [3] photon lookups
-    float4 *shadow;    // 3 per deferred NEE ray: (origin, max_dist), (dir, slot), (contribution, tag)
+    float4 *shadow;    // 2 per deferred NEE ray: (origin, max_dist), (dir, slot)
+    float4 *nee;       // the slot's pending NEE term: contribution, word (kNeePending / kNeeLit / ...)
     float4 *preq;      // 3 per photon-map lookup: (hit point, slot), (normal, sample), (throughput, job)
     unsigned long long *counters;  // [0] segments, [1] shadow rays (cumulative)
     // Work counters of the profiling traversal kernels (null otherwise): traversal records visited
     // by closest-hit / occlusion rays, then their leaf triangle tests.
     unsigned long long *work;
-    // The traversal layout of a one-job launch's scene (its records, leaf-ordered triangles), whether its
-    // occlusion rays may stop at any hit, and whether it has no triangles; filled by the launchers.
+    // A one-job launch's scene: its records, leaf-ordered triangles, whether its occlusion rays may stop at
+    // any hit, whether it has no triangles, and its tie margin; filled by the launchers.
     const float4 *records0, *tris0;
     uint32_t any_hit0, empty0;
+    float tie_margin0;
 };
 // Host-side shape of a job for the per-job launches.
 struct JobShape {

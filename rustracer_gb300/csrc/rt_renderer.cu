@@ -8,7 +8,7 @@
 //           as rgba8 arrays (layer-major); the traversal layout derived from the reference's BVH:
 //           one 64 B record per internal node, one 48 B leaf-ordered triangle record per prim slot.
 //   path:   per pixel, origin / direction / throughput (16 B each), hit 8 B, accumulators 64 B,
-//           first normal 16 B, two queue entries 4 B, one deferred shadow ray 48 B, one photon-lookup
+//           first normal 16 B, two queue entries 4 B, one deferred shadow ray 32 B, its NEE term 16 B, one photon-lookup
 //           request 48 B (240 B / pixel).
 //   frame:  frame, denoise ping-pong, moments, gbuffer, accumulation (float4 per pixel each) and the
 //           rgba8 output image.
@@ -255,12 +255,12 @@ rt_renderer::~rt_renderer() {
     if (pooled) rt::renderer_pool_release(device);
 }
 
-std::array<rt::DevBuf *, 32> rt_renderer::buffers() {
+std::array<rt::DevBuf *, 33> rt_renderer::buffers() {
     return {&d_lights,   &d_frame,   &d_pingpong, &d_moments,     &d_gbuffer,     &d_accum,       &d_output,
             &d_photons,  &d_keys,    &d_rank,     &d_order,       &d_sorted,      &d_sorted_pos,  &d_counts,
             &d_meta,     &d_cursor,  &d_partials, &d_total,       &d_counters,    &d_work,        &jobs.dev,
             &path.ro,    &path.rd,   &path.thr,   &path.hit,      &path.acc,      &path.nrm,      &path.queue[0],
-            &path.queue[1], &path.shadow, &path.preq, &path.counts};
+            &path.queue[1], &path.shadow, &path.nee,  &path.preq, &path.counts};
 }
 
 void rt_renderer::bind_buffers(cudaMemPool_t pool) {
@@ -411,6 +411,9 @@ int resident_scene_create(const rt_scene_desc *sd, rt_resident_scene **out) {
     ds.wide_stack = wide.nodes.empty() ? 0u : wide.stack_need;
     // A near-first traversal holds at most one pending entry per tree level.
     ds.stack_cap = lay.max_depth < 32u ? 32u : 63u;
+    for (int a = 0; a < 3 && sd->bvh_node_count; ++a)
+        ds.tie_margin = std::max({ds.tie_margin, 0x1p-17f * std::fabs(sd->bvh_nodes[0].bbox_min[a]),
+                                  0x1p-17f * std::fabs(sd->bvh_nodes[0].bbox_max[a])});
     ds.any_hit_shadows = 1u;
     for (uint64_t i = 0; i < sd->material_count; ++i)
         if ((sd->materials[i].flags & RT_MAT_FLAG_ALPHA_CUTOUT) && sd->materials[i].tex_albedo != RT_TEX_NONE)

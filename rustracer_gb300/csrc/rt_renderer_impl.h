@@ -102,15 +102,15 @@ struct FrameEventRing {
 
 // Wavefront path state for `slots` pixel slots (240 B per slot) and the per-iteration counters.
 struct PathState {
-    DevBuf ro, rd, thr, hit, acc, nrm, queue[2], shadow, preq, counts;
+    DevBuf ro, rd, thr, hit, acc, nrm, queue[2], shadow, nee, preq, counts;
     size_t slots = 0, counts_bytes = 0;
     // (Re)allocates when too small.  The caller's stream must be idle.
     cudaError_t ensure(size_t n_slots, uint32_t iters) {
         cudaError_t e;
         if (n_slots > slots) {
-            DevBuf *b[10] = {&ro, &rd, &thr, &nrm, &hit, &acc, &queue[0], &queue[1], &shadow, &preq};
-            const size_t sz[10] = {16, 16, 16, 16, 8, 64, 4, 4, 48, 48};
-            for (int i = 0; i < 10; ++i)
+            DevBuf *b[11] = {&ro, &rd, &thr, &nrm, &hit, &acc, &queue[0], &queue[1], &shadow, &nee, &preq};
+            const size_t sz[11] = {16, 16, 16, 16, 8, 64, 4, 4, 32, 16, 48};
+            for (int i = 0; i < 11; ++i)
                 if ((e = b[i]->alloc(n_slots * sz[i])) != cudaSuccess) {
                     slots = 0;
                     return e;
@@ -142,6 +142,7 @@ struct PathState {
         w.queue[1] = queue[1].as<uint32_t>();
         w.counts = counts.as<uint32_t>();
         w.shadow = shadow.as<float4>();
+        w.nee = nee.as<float4>();
         w.preq = preq.as<float4>();
         w.counters = counters;
         return w;
@@ -247,7 +248,7 @@ struct rt_renderer {
     // Every device buffer above comes from the device's renderer pool in the renderer's stream order
     // (bind_buffers at create; release_buffers before the stream goes).
     bool pooled = false;
-    std::array<rt::DevBuf *, 32> buffers();  // every device buffer the renderer owns
+    std::array<rt::DevBuf *, 33> buffers();  // every device buffer the renderer owns
     void bind_buffers(cudaMemPool_t pool);
     void release_buffers();
     ~rt_renderer();

@@ -12,6 +12,15 @@
 // the first strictly smaller t wins, meets the lowest slot first.  The best hit of a lane's ray is one
 // 64-bit word, t's bits above the prim slot (t is positive, so the words order as (t, slot) pairs), and a
 // test that hits lowers it with an atomic minimum, whatever order the tests come in.
+//
+// The order could matter in one case.  A walk that tests leaves as it meets them never tests a leaf it
+// enters at or beyond the hit it already has; with its leaves still queued, a lane may.  Such a leaf can
+// only change the result if the nearest hit lies nearer than its own leaf's box is entered, and a second
+// hit fits in between.  Both distances are rounded values of nearly the same number, so the walk keeps the
+// second nearest hit's t too, and when the two nearest hits are closer than kTieRelative of t plus
+// DevScene.tie_margin, a bound on the entry decides (hit_entry_bound); a ray it does not clear (about one
+// in a million) is walked again, waiting for the tests of each record's leaves before it goes on.  Results
+// do not depend on which rays share a warp.
 #pragma once
 #include "rt_device.cuh"
 
@@ -22,6 +31,8 @@ namespace rtd {
 // 2% slower, 14 0.5%, 16 (6 blocks) 9%.
 constexpr uint32_t kTopStack = 11, kMaxStack = 64;
 // Leaves a warp's queue holds: up to 7 wait from earlier steps, and a step adds up to 4 per lane.
+// Two hits farther apart than this part of their distance (and tie_margin) are no tie.
+constexpr float kTieRelative = 0x1p-10f;
 constexpr uint32_t kLeafCap = 7 + 4 * 32 + 1;
 
 // A warp's shared state.
@@ -31,13 +42,15 @@ struct __align__(16) WarpTrav {
     // The next rays of the warp's queue segment, copied in ahead of need: origin, direction (.w: job
     // index), reciprocal direction (.w: ray id).
     float4 next_ro[32], next_rd[32], next_inv[32];
-    uint32_t next_queue[32];  // work-list entries of the rays after those
+    uint32_t next_queue[32];  // path slots of the rays after those
     uint32_t n_ext, n;        // the work list: closest-hit rays, then occlusion rays up to n
     uint32_t item, seg_end;   // the warp's segment of the work list: first item not read ahead, end
-    uint32_t items;           // entries in next_queue
+    uint32_t items, first;    // entries in next_queue, the first one's item
     uint32_t at, ready;       // rays [at, ready) of the copied ones are unclaimed
     uint32_t coming;          // rays being copied
     unsigned long long best[32];  // t bits << 32 | prim slot
+    uint32_t second[32];          // bits of the second nearest hit's t
+    float limit[32];              // occlusion rays: hits below it count
     uint2 leaf[kLeafCap];         // queued leaves: first prim slot, count << 5 | owner lane
 };
 
@@ -58,6 +71,26 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// The scene's tri_ord carried by a ray of WarpTrav.
+__device__ __forceinline__ const float4 *ray_triangles(float4 ro, float4 rd) {
+    return reinterpret_cast<const float4 *>(((unsigned long long)__float_as_uint(rd.w) << 32) |
+                                            (unsigned long long)__float_as_uint(ro.w));
+}
+
+// Moller-Trumbore (common.wgsl:78-100) with the edges precomputed, without a branch; 0 for a miss (hits
+// count above kEps).
+__device__ __forceinline__ float hit_distance(f3 ro, f3 rd, float4 v0, float4 e1, float4 e2) {
+    const f3 h3 = cross(rd, xyz(e2));
+    const float a = dot(xyz(e1), h3);
+    const float f = 1.0f / a;
+    const f3 sv = ro - xyz(v0);
+    const float u = f * dot(sv, h3);
+    const f3 q = cross(sv, xyz(e1));
+    const float v = f * dot(rd, q);
+    const float t = f * dot(xyz(e2), q);
+    return fabsf(a) < 1e-7f || u < 0.0f || u > 1.0f || v < 0.0f || u + v > 1.0f ? 0.0f : t;
+}
+
 // Tests the triangles of queued leaves [first, first + n), n <= 8: lane l takes triangles l % 4,
 // l % 4 + 4, ... of leaf l / 4, against the ray of the lane that queued it.
 // tris: the scene's leaf-ordered triangles (kMulti: each ray's own, from its record).
@@ -68,32 +101,18 @@ __device__ __forceinline__ void test_leaves(WarpTrav &w, uint32_t first, uint32_
     const uint2 leaf = w.leaf[first + e];
     const uint32_t ref = leaf.x, o = leaf.y & 31u, cnt = leaf.y >> 5;
     const float4 r0 = w.ro[o], r1 = w.rd[o];
-    if (kMulti)
-        tris = reinterpret_cast<const float4 *>(((unsigned long long)__float_as_uint(r1.w) << 32) |
-                                                (unsigned long long)__float_as_uint(r0.w));
+    if (kMulti) tris = ray_triangles(r0, r1);
     const f3 ro = xyz(r0), rd = xyz(r1);
-    unsigned long long best = w.best[o];
-    bool found = false;
     for (uint32_t k = lane & 3u; k < cnt; k += 4u) {
         const float4 *tp = tris + 3ull * (ref + k);
         const float4 v0 = __ldg(tp), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
-        // Moller-Trumbore (common.wgsl:78-100) with the edges precomputed.
-        const f3 h3 = cross(rd, xyz(e2));
-        const float a = dot(xyz(e1), h3);
-        const float f = 1.0f / a;
-        const f3 sv = ro - xyz(v0);
-        const float u = f * dot(sv, h3);
-        const f3 q = cross(sv, xyz(e1));
-        const float v = f * dot(rd, q);
-        const float t = f * dot(xyz(e2), q);
-        const bool miss = fabsf(a) < 1e-7f || u < 0.0f || u > 1.0f || v < 0.0f || u + v > 1.0f;
-        const unsigned long long word = hit_word(t, ref + k);
-        if (!miss && t > kEps && word < best) {
-            best = word;
-            found = true;
+        const float t = hit_distance(ro, rd, v0, e1, e2);
+        // (a hit beyond the second nearest one changes nothing)
+        if (t > kEps && __float_as_uint(t) <= w.second[o]) {
+            const unsigned long long word = hit_word(t, ref + k), old = atomicMin(&w.best[o], word);
+            atomicMin(&w.second[o], (uint32_t)((word < old ? old : word) >> 32));
         }
     }
-    if (found) atomicMin(&w.best[o], best);
 }
 
 // Two floats of a packed pair, and the pairs' IEEE sum and product (each half rounded as the scalar
@@ -114,6 +133,19 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
+}
+
+// An upper bound on where a ray enters the leaf box of the triangle in `prim`: the entry into the
+// triangle's own box, which lies inside, with its corners rebuilt from the edges and moved by delta (more
+// than their rounding).
+__device__ __forceinline__ float hit_entry_bound(const float4 *tris, uint32_t prim, f3 ro, f3 rd, float delta) {
+    const float4 *tp = tris + 3ull * prim;
+    const f3 v0 = xyz(__ldg(tp)), v1 = v0 + xyz(__ldg(tp + 1)), v2 = v0 + xyz(__ldg(tp + 2));
+    const f3 lo = vmin(v0, vmin(v1, v2)) - ro, hi = vmax(v0, vmax(v1, v2)) - ro;
+    const float x = (rd.x > 0.0f ? lo.x + delta : hi.x - delta) / rd.x, y = (rd.y > 0.0f ? lo.y + delta : hi.y - delta) / rd.y,
+                z = (rd.z > 0.0f ? lo.z + delta : hi.z - delta) / rd.z;
+    const float te = fmax3f(x, y, z);
+    return te + fabsf(te) * 0x1p-20f;
 }
 
 // One ray's walk, kept by its lane.
@@ -162,15 +194,16 @@ struct Treelet {
 
 // One step of every lane of a warp: `visiting` lanes test the child boxes of their record, queue the
 // hit leaves behind the `queued` ones in w, and move on to the next record (visiting ends when none is
-// left).  records: the scene's (kMulti: each ray's own, st.records).  tests counts the lane's queued
-// triangles.  Every lane calls it.
+// left).  records: the scene's (kMulti: each ray's own, st.records).  tests: the lane's queued triangles
+// are added.  Every lane calls it.
 //
 // A child is 32 bytes, one load: four-wide (min.x, max.x, min.y, max.y), (min.z, max.z, ref, count), so
 // that both planes of an axis go through one packed subtraction and one packed product; two-wide
 // (min, ref), (max, count).
 template <bool kWide, int kTree, int kBlock, bool kMulti>
-__device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep, bool &visiting, WarpTrav &w,
-                                          uint32_t &queued, const Treelet &tree, const float4 *records, uint32_t &tests) {
+__device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep, bool &visiting, bool careful, WarpTrav &w,
+                                          uint32_t &queued, const Treelet &tree, const float4 *records,
+                                          uint32_t &tests) {
     constexpr int K = kWide ? 4 : 2;
     if (kMulti) records = st.records;
     const float kNone = __int_as_float(0x7F800000);
@@ -186,9 +219,9 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
         } else {
             // Neighbouring lanes take a record's children in different orders: records are aligned to their
             // size, so one child of 32 records lies in a fourth of L1's banks and its load takes a data
-            // cycle per lane, not per four lanes (trace 3% slower).  The order children are tested in
-            // changes nothing.
-            const uintptr_t np = reinterpret_cast<uintptr_t>(records + (size_t)(2 * K) * st.node) + (threadIdx.x % K) * 32u;
+            // cycle per lane, not per four lanes (trace 3% slower).  Their order
+            // can only matter to a careful ray.
+            const uintptr_t np = reinterpret_cast<uintptr_t>(records + (size_t)(2 * K) * st.node) + (careful ? 0u : (threadIdx.x % K) * 32u);
 #pragma unroll
             for (int i = 0; i < K; ++i) ldg32(reinterpret_cast<const float4 *>(np ^ (i * 32u)), q[2 * i], q[2 * i + 1]);
         }
@@ -217,7 +250,8 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
     for (int c = 0; c < K; ++c) {
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, cnt[c] != 0u);
         if (cnt[c] != 0u) {
-            w.leaf[queued + __popc(m & lanemask_lt())] = make_uint2(ref[c], cnt[c] << 5 | (threadIdx.x & 31u));
+            w.leaf[queued + __popc(m & lanemask_lt())] =
+                make_uint2(ref[c], cnt[c] << 5 | (threadIdx.x & 31u));
             tests += cnt[c];
         }
         queued += __popc(m);

@@ -78,3 +78,48 @@ def test_ray_counts(gpu, orc, w, h):
     cfg = rt.RenderConfig(width=w, height=h, spp=1, accumulate_frames=1, enable_denoise=False)
     r, o = render_both(orc, scene, cfg, 1)
     assert match_frac(r.read_accumulation(), o.accum) >= FRAC
+
+
+def layered_scene():
+    """Axis-aligned quads in pairs a rounding error apart, tiled edge to edge: a ray's two nearest hits are
+    ties or nearly so, and lie no farther than the (flat) boxes they are in."""
+    s = rt.Scene()
+    mats = [s.add_material(rt.lambertian(c)) for c in ((0.9, 0.2, 0.2), (0.2, 0.9, 0.2), (0.3, 0.3, 0.9))]
+    mats.append(s.add_material(rt.metal((0.9, 0.8, 0.5), 0.2)))
+    rng = np.random.default_rng(5)
+    for layer in range(3):
+        for i in range(6):
+            for j in range(6):
+                x, y = 0.7 * (i - 3), 0.7 * (j - 3)
+                z = np.float32(-0.37 - 1.1 * layer) + np.float32(rng.integers(0, 3)) * np.float32(2.0 ** -24)
+                quad = [[x, y, z], [x + 0.7, y, z], [x + 0.7, y + 0.7, z], [x, y + 0.7, z]]
+                for m in rng.choice(4, 2, replace=False):
+                    s.add_mesh(quad, [0, 1, 2, 0, 2, 3], mats[m])
+                    quad = [[a, b, c - np.float32(2.0 ** -24)] for a, b, c in quad]
+    return lit(s)
+
+
+def test_near_ties_do_not_depend_on_the_launch(gpu, width):
+    """Which rays share a warp, how often it tests leaves and how its jobs are batched change no hit."""
+    s = layered_scene()
+    cfg = rt.RenderConfig(width=301, height=203, spp=2, accumulate_frames=1, enable_denoise=False, max_bounces=6)
+
+    def image(**tuning):
+        r = rt.Renderer(s, cfg)
+        r.update_camera(CAM)
+        r.tuning = dict(r.tuning, **tuning)
+        r.record_frame()
+        return r.read_accumulation()
+
+    ref = image()
+    for tuning in (dict(), dict(steps=1), dict(steps=7, chunk=64), dict(block_threads=64, blocks_per_sm=2),
+                   dict(block_threads=256, blocks_per_sm=1, chunk=256)):
+        assert np.array_equal(image(**tuning), ref), tuning
+    rs = [rt.Renderer(s, cfg) for _ in range(3)]
+    for r in rs:
+        r.update_camera(CAM)
+    b = rt.Batch(rs, use_graphs=False)
+    b.render_frame()
+    for r in rs:
+        assert np.array_equal(r.read_accumulation(), ref)
+    b.close()
