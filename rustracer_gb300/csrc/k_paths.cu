@@ -1,0 +1,231 @@
+// The gather pass of few paths in one launch (gather.wgsl:91-593).  A warp takes up to 32 paths and runs
+// extend, shade, photon lookup and shadow for all of them until the last sample of the last pixel has ended,
+// with the wavefront's traversal (the occlusion rays of a step ride with the closest-hit rays of the next one,
+// taken by whichever lanes are idle) and its per-path steps in the same order, so the images are the same
+// bit for bit.  Two uses:
+//
+//   a frame of few pixels as a whole, generate and finalize included;
+//   the end of a larger frame: a launch in front of a shade pass that returns at once while more than `most`
+//   paths are queued and otherwise runs all that is left of them.
+//
+// What bounds few paths in the wavefront is its chain of launches, each of them one dependent load after the
+// other for a fraction of a warp per scheduler: the Cornell box at 256 x 256, 5 segments deep, took 15
+// launches and 188 us.  Here a warp waits for its own loads only.  It is bound by the latency of one path's
+// instructions (a walk of three records about 4,400 cycles, a shade step 5,000 and more).  With more paths
+// than the SMs hold at once the compacted queues win: lanes whose path has ended idle here until the warp's
+// last one ends.
+#include "rt_paths.cuh"
+
+namespace rtd {
+
+namespace {
+constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 4;  // 128 registers
+// Paths per warp when they are too few for 32 each: below this a warp's idle lanes gain nothing (measured at
+// 64 x 64: 2, 4 and 8 alike, 16 10% slower, 32 28%).
+constexpr uint32_t kPathsShare = 4;
+}  // namespace
+
+template <bool kMulti, bool kPhotons, bool kWhole>
+__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kernel(const __grid_constant__ WaveParams p,
+                                                                                  uint32_t iter, uint32_t most) {
+    extern __shared__ __align__(16) unsigned char trav_smem[];
+    // kWhole: `most` pixel positions, 8 x 4 tiles as in generate; otherwise the paths queued for `iter`.
+    const uint32_t n = kWhole ? most : p.counts[4 * iter];
+    if (!kWhole && n > most) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint2 *top = reinterpret_cast<uint2 *>(trav_smem) + threadIdx.x;
+    uint2 deep[kMaxStack - kTopStack];
+    WarpTrav &w = reinterpret_cast<WarpTrav *>(trav_smem + sizeof(uint2) * kTopStack * kPathsBlock)[threadIdx.x >> 5];
+    const Treelet tree{nullptr, nullptr, 0u};
+    LaneWalk r;
+    r.busy = r.visiting = r.any_hit = r.careful = r.held = false;
+    r.st.sp = 0u;
+    uint32_t segments = 0u, shadow_rays = 0u;
+    // Few paths are spread over all warps.
+    const uint32_t warps = gridDim.x * (kPathsBlock / 32);
+    const uint32_t share = min(32u, max(kPathsShare, (n + warps - 1u) / warps));
+    for (uint32_t base = share * (blockIdx.x * (kPathsBlock / 32) + (threadIdx.x >> 5)); base < n; base += share * warps) {
+        bool alive = lane < share && base + lane < n;
+        uint32_t slot = 0u, jid = 0u;
+        if (kWhole) {
+            const uint32_t at = min(base + lane, n - 1u), gtile = at >> 5;
+            if (kMulti) jid = job_of(p, gtile, [](const DevJob &j) { return j.tile0; });
+            const DevJob &job = p.jobs[jid];
+            const uint32_t W = job.ip.width, tiles_x = (W + 7u) / 8u, tile = gtile - job.tile0;
+            const uint32_t px = tile % tiles_x * 8u + (at & 7u), py = tile / tiles_x * 4u + (at >> 3 & 3u);
+            alive = alive && px < W && py < job.ip.height;
+            slot = job.base + py * W + px;
+            if (alive) start_slot(p, job, jid, px, py, slot);
+        } else if (alive) {
+            slot = p.queue[iter & 1u][base + lane];
+            if (kMulti) jid = __float_as_uint(p.thr[slot].w);
+        }
+        const bool mine = alive;
+        const DevJob &job = p.jobs[jid];
+        const DevScene &sc = job.scene;
+        const float4 *records = kMulti ? sc.wnodes : p.records0, *tris = kMulti ? sc.tri_ord : p.tris0;
+        const bool empty = kMulti ? sc.cnode_count == 0u : p.empty0 != 0u;
+        const bool any = kMulti ? sc.any_hit_shadows != 0u : p.any_hit0 != 0u;
+        ShadeOut out;
+        out.sh_o = out.sh_d = mk3(0.0f, 0.0f, 0.0f);
+        out.sh_max = 0.0f;
+        for (bool traced = !kWhole;; traced = false) {
+            float hit_dist = kInf;
+            uint32_t hit_slot = 0u;
+            bool lit = false;
+            if (traced) {  // the wavefront has traced the queued paths and the shadow rays before them
+                if (alive) {
+                    const float2 h = p.hit[slot];
+                    hit_dist = h.x;
+                    hit_slot = __float_as_uint(h.y);
+                }
+            } else {
+                // The occlusion rays of the last shade step, packed for whichever lane takes them; the
+                // direction's .w: the lane that waits for the answer.
+                const uint32_t occ_mask = __ballot_sync(0xFFFFFFFFu, out.shadow), n_occ = __popc(occ_mask);
+                if (out.shadow) {
+                    const uint32_t k = __popc(occ_mask & lanemask_lt());
+                    w.next_ro[k] = make_float4(out.sh_o.x, out.sh_o.y, out.sh_o.z, out.sh_max);
+                    w.next_rd[k] = make_float4(out.sh_d.x, out.sh_d.y, out.sh_d.z, __uint_as_float(lane));
+                    if (kMulti) w.next_queue[k] = jid;
+                    shadow_rays += 1u;
+                }
+                if (lane == 0u) w.coming = 0u;  // the answers: lanes whose light is visible
+                __syncwarp();
+                uint32_t at = 0u, owner = lane, occ_job = 0u;
+                bool occ = false;
+                if (alive) {
+                    const float4 o = p.ro[slot], d = p.rd[slot];
+                    r.st.records = records;
+                    r.st.cap = kMaxStack;
+                    r.any_hit = false;
+                    r.st.t = kInf;
+                    if (kMulti) w.margin[lane] = sc.tie_margin;
+                    walk_begin(r, w, xyz(o), xyz(d), mk3(1.0f, 1.0f, 1.0f) / xyz(d), tris);
+                    r.visiting = !empty;
+                    segments += 1u;
+                }
+                for (;;) {
+                    const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !r.busy);
+                    if (idle == 0xFFFFFFFFu && at == n_occ) break;
+                    if (idle != 0u && at != n_occ) {
+                        const uint32_t k = at + __popc(idle & lanemask_lt());
+                        if (!r.busy && k < n_occ) {
+                            const float4 o = w.next_ro[k], d = w.next_rd[k];
+                            owner = __float_as_uint(d.w);
+                            occ = true;
+                            const float4 *otris = tris;
+                            bool oany = any;
+                            r.st.records = records;
+                            r.st.cap = kMaxStack;
+                            if (kMulti) {
+                                occ_job = w.next_queue[k];
+                                const DevScene &os = p.jobs[occ_job].scene;
+                                r.st.records = os.wnodes;
+                                otris = os.tri_ord;
+                                oany = os.any_hit_shadows != 0u;
+                                w.margin[lane] = os.tie_margin;
+                            }
+                            // (see wf_trace_kernel)
+                            r.any_hit = oany;
+                            r.st.t = o.w - 0.001f;
+                            if (!oany) {
+                                w.limit[lane] = r.st.t;
+                                r.st.t = search_limit(r.st.t);
+                            }
+                            walk_begin(r, w, xyz(o), xyz(d), mk3(1.0f, 1.0f, 1.0f) / xyz(d), otris);
+                            r.visiting = r.st.t > kEps;
+                        }
+                        at = min(at + (uint32_t)__popc(idle), n_occ);
+                    }
+                    uint32_t visits = 0u, tests = 0u;
+                    walk_records<true, 0, kPathsBlock, kMulti, false>(r, w, top, deep, tree, p.records0, p.tris0, 3u, 0,
+                                                                      visits, tests);
+                    if (r.busy && !r.visiting) do {
+                        bool clear = !r.found && r.st.t == r.st.t;  // (a NaN limit counts as occluded)
+                        if (!r.any_hit) {
+                            if (walk_again<kMulti>(r, w, p.tris0, kMulti ? w.margin[lane] : p.tie_margin0,
+                                                   occ ? search_limit(w.limit[lane]) : kInf))
+                                continue;
+                            const unsigned long long hit = w.best[lane];
+                            if (occ) {
+                                clear = cut_out_lit(p.jobs[occ_job].scene, w.ro[lane], w.rd[lane], w.limit[lane], hit);
+                            } else {
+                                hit_dist = hit_t(hit);
+                                hit_slot = (uint32_t)hit;
+                            }
+                        }
+                        if (occ && clear) atomicOr(&w.coming, 1u << owner);
+                        r.busy = false;
+                    } while (false);
+                }
+                __syncwarp();
+                lit = (w.coming >> lane & 1u) != 0u;
+                __syncwarp();
+            }
+            if (!alive) {
+                // an ended path's last term is finalize's to add
+                if (lit) p.nee[slot].w = __uint_as_float(__float_as_uint(p.nee[slot].w) | kNeeLit);
+                out.shadow = false;
+            }
+            if (!__any_sync(0xFFFFFFFFu, alive)) break;
+            if (alive) {
+                uint32_t prim = 0u, word = 0u;
+                if (hit_dist < kInf) {
+                    prim = __float_as_uint(__ldg(tris + 3ull * hit_slot).w);
+                    word = __float_as_uint(__ldg(tris + 3ull * hit_slot + 1).w);
+                }
+                out = shade_path<kPhotons, false>(p, slot, hit_dist, prim, word >> 2, lit);
+                if (kPhotons && out.photon)
+                    photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td);
+                alive = out.keep;
+            }
+        }
+        if (kWhole && mine) finalize_slot(p, job, slot);
+    }
+    segments = __reduce_add_sync(0xFFFFFFFFu, segments);
+    shadow_rays = __reduce_add_sync(0xFFFFFFFFu, shadow_rays);
+    if (lane == 0u && p.counters && (segments | shadow_rays) != 0u) {
+        atomicAdd(p.counters, (unsigned long long)segments);
+        atomicAdd(p.counters + 1, (unsigned long long)shadow_rays);
+    }
+}
+
+namespace {
+using PathsKernel = void (*)(const WaveParams, uint32_t, uint32_t);
+template <bool kWhole>
+PathsKernel paths_kernel(bool multi, bool photons) {
+    if (multi) return photons ? wf_paths_kernel<true, true, kWhole> : wf_paths_kernel<true, false, kWhole>;
+    return photons ? wf_paths_kernel<false, true, kWhole> : wf_paths_kernel<false, false, kWhole>;
+}
+}  // namespace
+
+void prepare_paths_kernels() {
+    for (int v = 0; v < 4; ++v) {
+        const int bytes = (int)trav_smem_bytes(kPathsBlock, false);
+        cudaFuncSetAttribute(reinterpret_cast<const void *>(paths_kernel<true>((v & 1) != 0, (v & 2) != 0)),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaFuncSetAttribute(reinterpret_cast<const void *>(paths_kernel<false>((v & 1) != 0, (v & 2) != 0)),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    }
+}
+
+// As many paths as the SMs hold threads of the kernel.  Measured against the wavefront (gather, ms): 320 x 240
+// 1 spp in a 20k-triangle room 0.39 against 0.43, 2 spp in a 328k-triangle room 0.90 against 1.25, cut-out
+// foliage 0.71 against 0.91; at 400 x 300 0.43 against 0.45; at 480 x 270 1.32 against 1.14.
+uint32_t paths_limit(int num_sms) { return (uint32_t)num_sms * kPathsBlocksPerSm * kPathsBlock; }
+
+cudaError_t launch_paths_frame(const WaveParams &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st) {
+    const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
+    paths_kernel<true>(multi, photons)<<<blocks, kPathsBlock, trav_smem_bytes(kPathsBlock, false), st>>>(p, 0u, 32u * tiles);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, int num_sms,
+                              cudaStream_t st) {
+    const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
+    paths_kernel<false>(multi, photons)<<<blocks, kPathsBlock, trav_smem_bytes(kPathsBlock, false), st>>>(p, iter, most);
+    return cudaGetLastError();
+}
+
+}  // namespace rtd

@@ -92,6 +92,14 @@ struct WaveProfile {
 // generate (per job), iters x (extend, shade, shadow) over all jobs, finalize (per job), counters.
 cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t n_jobs, uint32_t iters, int num_sms,
                              const WaveTuning &tune, cudaStream_t st, WaveProfile *prof = nullptr);
+// The gather pass of few paths in one launch (k_paths.cu): a whole frame of at most paths_limit pixels in
+// `tiles` 8 x 4 tiles, or, if at most `most` paths are queued for iteration `iter` (traced, not yet shaded),
+// the rest of theirs.
+uint32_t paths_limit(int num_sms);
+cudaError_t launch_paths_frame(const WaveParams &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st);
+cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, int num_sms,
+                              cudaStream_t st);
+void prepare_paths_kernels();
 int device_sm_count();
 // One-time kernel attributes (shared-memory opt-ins); call before capturing launches into a graph.
 void prepare_kernels();

@@ -1,0 +1,648 @@
+// One path of the gather pass (gather.wgsl:91-593), step by step: what the wavefront's kernels
+// (k_wavefront.cu) each run for one queued path and the one-launch form (k_paths.cu) runs in a loop.
+#pragma once
+#include "rt_kernels.h"
+#include "rt_traverse.cuh"
+
+namespace rtd {
+
+__device__ __forceinline__ float luma(f3 c) { return dot(c, mk3(0.2126f, 0.7152f, 0.0722f)); }
+
+struct Accum {
+    f3 col;
+    float lum_sum, lum2_sum;
+    float sl[8];
+};
+// The words of a slot's accumulator one shade step can change: every term it adds belongs to the
+// sample it started with, so only that sample's luminance sum is loaded and stored with the colour
+// and the two luminance moments.
+struct PathAcc {
+    f3 col;
+    float lum_sum, lum2_sum, sl;
+};
+// The NEE term of a path's last bounce waits in its slot (p.nee: the contribution and a word) until its
+// occlusion ray has been traced: kNeeLit is set if the light is visible, and the slot's next shade (or
+// finalize) adds the term first of all.  The word's low bits: the sample it belongs to, and whether only
+// its luminance counts (photon debug).
+constexpr uint32_t kNeePending = 0x20000u, kNeeLumaOnly = 0x10000u, kNeeLit = 0x80000000u;
+
+__device__ __forceinline__ void add_radiance(uint32_t s, PathAcc &a, f3 c) {
+    a.col = a.col + c;
+    float l = luma(c);
+    a.lum_sum += l;
+    a.lum2_sum += l * l;
+    if (s < 8u) a.sl += l;
+}
+// One radiance term (or only its luminance) added straight into a slot's accumulator in memory:
+// colour, the two luminance moments and the sample's luminance sum, as every path step adds them.
+__device__ __forceinline__ void acc_add_term(const WaveParams &p, uint32_t slot, uint32_t s, f3 c, bool luma_only) {
+    float4 *a = p.acc + 4 * (size_t)slot;
+    float4 a0 = a[0];
+    float *lum2 = reinterpret_cast<float *>(a + 1);
+    const float l = luma(c);
+    if (!luma_only) {
+        a0.x = a0.x + c.x;
+        a0.y = a0.y + c.y;
+        a0.z = a0.z + c.z;
+    }
+    a0.w += l;
+    a[0] = a0;
+    *lum2 += l * l;
+    if (s < 8u) reinterpret_cast<float *>(a + 2)[s] += l;
+}
+// A lit NEE term added to a slot's accumulator, whose words for sample s0 are in A.
+__device__ __forceinline__ void add_nee(const float4 &nee, float4 *acc, uint32_t s0, PathAcc &A) {
+    const uint32_t word = __float_as_uint(nee.w), s = word & 0xFFFFu;
+    const f3 c = xyz(nee);
+    const float l = luma(c);
+    if (!(word & kNeeLumaOnly)) A.col = A.col + c;
+    A.lum_sum += l;
+    A.lum2_sum += l * l;
+    if (s < 8u) {
+        if (s == s0) A.sl += l;
+        else reinterpret_cast<float *>(acc + 2)[s] += l;  // the sample that ended with this term
+    }
+}
+__device__ __forceinline__ Accum load_acc(const WaveParams &p, uint32_t pix) {
+    const float4 a = p.acc[4 * (size_t)pix], b = p.acc[4 * (size_t)pix + 1], c = p.acc[4 * (size_t)pix + 2],
+                 d = p.acc[4 * (size_t)pix + 3];
+    Accum A;
+    A.col = mk3(a.x, a.y, a.z);
+    A.lum_sum = a.w;
+    A.lum2_sum = b.x;
+    A.sl[0] = c.x; A.sl[1] = c.y; A.sl[2] = c.z; A.sl[3] = c.w;
+    A.sl[4] = d.x; A.sl[5] = d.y; A.sl[6] = d.z; A.sl[7] = d.w;
+    return A;
+}
+
+__device__ __forceinline__ f3 sky_color(f3 dir, f3 zenith, f3 horizon, float intensity) {
+    float t = clampf(dir.y * 0.5f + 0.5f, 0.0f, 1.0f);
+    return mix3(horizon, zenith, sqrtf(t)) * intensity;  // pow(t, 0.5) for t in [0, 1]
+}
+__device__ __forceinline__ float smith_g1(float nd, float a) {
+    float k = a * 0.5f;
+    return nd / (nd * (1.0f - k) + k);
+}
+__device__ __forceinline__ f3 spec_ggx(f3 wo, f3 n, f3 wi, float a, f3 f0) {
+    float ndl = dot(n, wi);
+    float ndv = dot(n, wo);
+    if (ndl <= 0.0f || ndv <= 0.0f) return mk3(0.0f, 0.0f, 0.0f);
+    f3 h = normalize(wo + wi);
+    float ndh = fmaxf(dot(n, h), 0.0f);
+    float a2 = a * a;
+    float dd = ndh * ndh * (a2 - 1.0f) + 1.0f;
+    float D = a2 / (kPi * dd * dd);
+    f3 F = fresnel_schlick(fmaxf(dot(wo, h), 0.0f), f0);
+    return F * (D * smith_g1(ndl, a) * smith_g1(ndv, a) / (4.0f * ndl * ndv));
+}
+__device__ __forceinline__ f3 sample_spec_dir(f3 rd, f3 n, float a, Rng &rng) {
+    f3 up = fabsf(n.y) < 0.999f ? mk3(0.0f, 1.0f, 0.0f) : mk3(1.0f, 0.0f, 0.0f);
+    f3 bt = normalize(cross(up, n));
+    f3 bb = cross(n, bt);
+    f3 mrd = -rd;
+    f3 v = mk3(dot(bt, mrd), dot(bb, mrd), dot(n, mrd));
+    f3 vh = normalize(mk3(a * v.x, a * v.y, fmaxf(v.z, 1e-4f)));
+    float l2 = vh.x * vh.x + vh.y * vh.y;
+    f3 t1 = l2 > 0.0f ? mk3(-vh.y, vh.x, 0.0f) * (1.0f / sqrtf(l2)) : mk3(1.0f, 0.0f, 0.0f);
+    f3 t2 = cross(vh, t1);
+    float r = sqrtf(rng_f32(rng));
+    float phi = 2.0f * kPi * rng_f32(rng);
+    float sp, cp;
+    sincos_fixed(phi, sp, cp);
+    float x = r * cp;
+    float y = r * sp;
+    float s = 0.5f * (1.0f + vh.z);
+    float yy = (1.0f - s) * sqrtf(fmaxf(0.0f, 1.0f - x * x)) + s * y;
+    f3 hh = x * t1 + yy * t2 + sqrtf(fmaxf(0.0f, 1.0f - x * x - yy * yy)) * vh;
+    f3 hn = normalize(hh);
+    f3 m = bt * hn.x + bb * hn.y + n * hn.z;
+    f3 out = reflect(rd, m);
+    return dot(out, n) > 0.0f ? out : reflect(rd, n);
+}
+
+// The light sample of direct_light (gather.wgsl:152-206) up to its shadow query.  `occlude` is set
+// when the sample needs the shadow ray (origin o, direction ld, max_dist); e is the unoccluded value.
+struct LightSample {
+    f3 e, wi, o;
+    float max_dist;
+    bool occlude;
+};
+__device__ __forceinline__ LightSample light_sample(const DevJob &job, f3 hp, f3 sn, Rng &rng) {
+    const DevScene &s = job.scene;
+    const uint32_t n = s.light_count;
+    const f3 zero = mk3(0.0f, 0.0f, 0.0f);
+    LightSample ls{zero, sn, zero, 0.0f, false};
+    if (n == 0u) return ls;
+    uint32_t li = f2u_sat(rng_f32(rng) * (float)n);
+    li = li < n ? li : n - 1u;
+    const Light l = load_light(s, li);
+    const float fn = (float)n;
+    if (l.kind == 0u) {
+        f3 to = l.data - hp;
+        float r2 = dot(to, to);
+        float r = sqrtf(r2);
+        f3 ld = to / r;
+        ls.wi = ld;
+        if (dot(sn, ld) <= 0.0f) return ls;
+        f3 pl = mk3(job.ip.point_light_emission[0], job.ip.point_light_emission[1], job.ip.point_light_emission[2]);
+        ls.e = l.color * l.intensity * pl * fmaxf(dot(sn, ld), 0.0f) / (r2 + 0.01f) * fn;
+        ls.o = hp + sn * 0.01f;
+        ls.max_dist = r - 0.001f;
+        ls.occlude = true;
+    } else if (l.kind == 1u) {
+        f3 ld = normalize(l.data);
+        float ndl = dot(sn, ld);
+        ls.wi = ld;
+        if (ndl <= 0.0f) return ls;
+        ls.e = l.color * l.intensity * ndl * fn;
+        ls.o = hp + sn * 0.01f;
+        ls.max_dist = 1e30f;
+        ls.occlude = true;
+    } else if (l.kind == 2u) {
+        TriFull tri = load_tri(s, f2u_sat(l.data.x));
+        Mat mat = load_mat(s, tri.material_id);
+        float u1 = rng_f32(rng);
+        float u2 = rng_f32(rng);
+        float su = sqrtf(u1);
+        float u = 1.0f - su;
+        float v = u2 * su;
+        float w = 1.0f - u - v;
+        f3 lp = tri.v0 * w + tri.v1 * u + tri.v2 * v;
+        float uvx = tri.uv0x * w + tri.uv1x * u + tri.uv2x * v;
+        float uvy = tri.uv0y * w + tri.uv1y * u + tri.uv2y * v;
+        f3 le = l.color;
+        if (mat.tex_emissive != RT_TEX_NONE) {
+            float4 t = tex_sample(s.tex[RT_TEX_EMISSIVE], uvx, uvy, (int32_t)mat.tex_emissive);
+            le = le * mk3(t.x, t.y, t.z);
+        }
+        le = le * mk3(job.ip.light_emission[0], job.ip.light_emission[1], job.ip.light_emission[2]);
+        f3 to = lp - hp;
+        float r2 = dot(to, to);
+        float r = sqrtf(r2);
+        f3 ld = to / r;
+        ls.wi = ld;
+        float ndl = dot(sn, ld);
+        if (ndl <= 0.0f) return ls;
+        f3 ln = triangle_normal(tri.v0, tri.v1, tri.v2);
+        float ndl_l = dot(ln, -ld);
+        if (ndl_l <= 0.0f) return ls;
+        float area = 0.5f * len3(cross(tri.v1 - tri.v0, tri.v2 - tri.v0));
+        ls.e = le * l.intensity * ndl * ndl_l * area * fn / (r2 + 0.01f);
+        ls.o = hp + sn * 0.01f;
+        ls.max_dist = r - 0.001f;
+        ls.occlude = true;
+    }
+    return ls;
+}
+
+__device__ __forceinline__ int32_t clampi(int32_t x, int32_t lo, int32_t hi) { return x < lo ? lo : (x > hi ? hi : x); }
+
+// The camera ray of the pixel's next sample (gather.wgsl:292-297).
+__device__ __forceinline__ void camera_ray(const DevJob &job, uint32_t px, uint32_t py, Rng &rng, f3 &ro, f3 &rd) {
+    const rt_camera_uniform &cam = job.cam;
+    float jx = rng_f32(rng) - 0.5f;
+    float jy = rng_f32(rng) - 0.5f;
+    float ux = ((float)px + jx) * cam.inv_half_res[0] - 1.0f;
+    float uy = 1.0f - ((float)py + jy) * cam.inv_half_res[1];
+    ro = mk3(cam.position[0], cam.position[1], cam.position[2]);
+    rd = normalize(mk3(cam.forward[0], cam.forward[1], cam.forward[2]) +
+                   mk3(cam.right[0], cam.right[1], cam.right[2]) * ux + mk3(cam.up[0], cam.up[1], cam.up[2]) * uy);
+}
+
+__device__ __forceinline__ uint32_t pack_sb(uint32_t s, uint32_t b) { return (s & 0xFFFFu) | (b << 16); }
+
+// The last job whose first index (`first` of DevJob: base slot or first tile) is at or below i; jobs
+// are laid out in order, so their first indices ascend.
+template <typename First>
+__device__ __forceinline__ uint32_t job_of(const WaveParams &p, uint32_t i, First first) {
+    uint32_t lo = 0u, hi = p.n_jobs;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (first(p.jobs[mid]) <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// The pixel's slot with the camera ray of its first sample (gather.wgsl:262-297) and nothing accumulated.
+__device__ __forceinline__ void start_slot(const WaveParams &p, const DevJob &job, uint32_t jid, uint32_t px, uint32_t py,
+                                           uint32_t slot) {
+    uint32_t base_seed = slot - job.base + job.ip.frame * 2654435761u;
+    Rng rng = rng_init(base_seed * 1664525u + 1013904223u);
+    f3 ro, rd;
+    camera_ray(job, px, py, rng, ro, rd);
+    p.ro[slot] = make_float4(ro.x, ro.y, ro.z, __uint_as_float(rng.state));
+    p.rd[slot] = make_float4(rd.x, rd.y, rd.z, __uint_as_float(pack_sb(0u, 0u)));
+    p.thr[slot] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(jid));
+    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    p.acc[4 * (size_t)slot] = z;
+    p.acc[4 * (size_t)slot + 1] = make_float4(0.0f, 1e30f, 0.0f, 0.0f);
+    p.acc[4 * (size_t)slot + 2] = z;
+    p.acc[4 * (size_t)slot + 3] = z;
+    p.nrm[slot] = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
+    p.nee[slot] = z;
+}
+
+// What one shade step of a path leaves to do: its occlusion ray and photon-map lookup, and whether the slot
+// goes on (the path's next segment or the pixel's next sample; ray and state are in the slot).
+struct ShadeOut {
+    bool keep = false, shadow = false, photon = false;
+    f3 sh_o, sh_d;  // occlusion ray, up to sh_max
+    float sh_max;
+    f3 ph_hp, ph_n, ph_td;  // lookup: hit point, shading normal, throughput x diffuse weight
+    uint32_t ph_sidx;
+};
+
+// One loop body of gather.wgsl:299-537 for the path in `slot`, whose ray hit triangle `prim` at hit_t (a miss:
+// kInf); hmat: the hit's material, known before its triangle, or kNoMat.  lit: the light of the slot's
+// pending NEE term is visible (also if its word says so).
+template <bool kPhotons, bool kDebug>
+__device__ __forceinline__ ShadeOut shade_path(const WaveParams &p, uint32_t slot, float hit_t, uint32_t prim,
+                                               uint32_t hmat, bool lit) {
+    ShadeOut out;
+    out.sh_o = out.sh_d = out.ph_hp = out.ph_n = out.ph_td = mk3(0.0f, 0.0f, 0.0f);
+    out.sh_max = 0.0f;
+    out.ph_sidx = 0u;
+    const float4 o4 = p.ro[slot], d4 = p.rd[slot], t4 = p.thr[slot];
+    const uint32_t jid = __float_as_uint(t4.w);
+    const DevJob &job = p.jobs[jid];
+    const DevScene &s = job.scene;
+    const rt_image_params &ip = job.ip;
+    const uint32_t W = ip.width;
+    const uint32_t spp = job.spp;
+    const uint32_t debug_view = ip._pad[0];
+    const float env_intensity = s.env_intensity;
+    const f3 env_color = mk3(s.env_color[0], s.env_color[1], s.env_color[2]);
+    const f3 env_horizon = mk3(s.env_horizon[0], s.env_horizon[1], s.env_horizon[2]);
+    const uint32_t pix = slot - job.base;
+    const uint32_t px = pix % W, py = pix / W;
+    f3 ro = xyz(o4), rd = xyz(d4), thr = xyz(t4);
+    Rng rng{__float_as_uint(o4.w)};
+    const uint32_t sb = __float_as_uint(d4.w);
+    uint32_t sidx = sb & 0xFFFFu, b = sb >> 16;
+    float4 *acc = p.acc + 4 * (size_t)slot;
+    const uint32_t sidx0 = sidx;
+    const float4 acc0 = acc[0], nee = p.nee[slot];
+    float4 acc1 = acc[1];  // .x = lum2_sum, .y = first_depth
+    PathAcc A{xyz(acc0), acc0.w, acc1.x, sidx0 < 8u ? reinterpret_cast<const float *>(acc + 2)[sidx0] : 0.0f};
+    const uint32_t nee_word = __float_as_uint(nee.w);
+    if (lit || (nee_word & kNeeLit)) add_nee(nee, acc, sidx0, A);
+    bool first_hit = false;  // this step found a nearer first hit (normal and depth change)
+    float4 nrm = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    bool alive = true;  // the sample continues with another segment
+
+    if (hit_t >= kInf) {
+        if (b > 0u) add_radiance(sidx, A, thr * sky_color(rd, env_color, env_horizon, env_intensity));
+        alive = false;
+    } else {
+        const TriFull tr = load_tri(s, prim);
+        Mat mat;
+        if (hmat != kNoMat) mat = load_mat(s, hmat);
+        else mat = load_mat(s, tr.material_id);
+        const f3 hp = ro + rd * hit_t;
+        const Bary bb = barycentric(tr, ro, rd, hit_t);
+        const float uvx = bb.uvx, uvy = bb.uvy;
+        bool done_step = false;  // a `continue` of the reference loop
+
+        if ((mat.flags & RT_MAT_FLAG_ALPHA_CUTOUT) != 0u && mat.tex_albedo != RT_TEX_NONE &&
+            tex_sample(s.tex[RT_TEX_ALBEDO], uvx, uvy, (int32_t)mat.tex_albedo).w < 0.5f) {
+            ro = hp + rd * 0.002f;
+            done_step = true;
+        }
+        if (!done_step) {
+            const f3 gn = triangle_normal(tr.v0, tr.v1, tr.v2);
+            const bool ff = dot(rd, gn) < 0.0f;
+            const f3 sn_geom = smooth_normal(tr, bb, gn);
+            const f3 sn = ff ? sn_geom : -sn_geom;
+            f3 shn = sn;
+            if (mat.tex_normal != RT_TEX_NONE) {
+                float4 t = tex_sample(s.tex[RT_TEX_NORMAL], uvx, uvy, (int32_t)mat.tex_normal);
+                f3 nm = mk3(t.x, t.y, t.z) * 2.0f - mk3(1.0f, 1.0f, 1.0f);
+                f3 ft, fb;
+                tangent_frame(tr, sn, ft, fb);
+                shn = normalize(ft * nm.x + fb * nm.y + sn * nm.z);
+            }
+            if (b == 0u && hit_t < acc1.y) {
+                nrm = make_float4(sn.x, sn.y, sn.z, 0.0f);
+                first_hit = true;
+                acc1.y = hit_t;
+            }
+            f3 albedo = mat.albedo;
+            float rough = mat.roughness, metal = mat.metallic;
+            if (mat.tex_albedo != RT_TEX_NONE) {
+                float4 t = tex_sample(s.tex[RT_TEX_ALBEDO], uvx, uvy, (int32_t)mat.tex_albedo);
+                albedo = mat.albedo * mk3(t.x, t.y, t.z);
+            }
+            if (mat.tex_mr != RT_TEX_NONE) {
+                float4 mr = tex_sample(s.tex[RT_TEX_MR], uvx, uvy, (int32_t)mat.tex_mr);
+                rough = clampf(mat.roughness * mr.y, 0.0f, 1.0f);
+                metal = clampf(mat.metallic * mr.z, 0.0f, 1.0f);
+            }
+            f3 emis = mat.emissive;
+            if (mat.tex_emissive != RT_TEX_NONE) {
+                float4 t = tex_sample(s.tex[RT_TEX_EMISSIVE], uvx, uvy, (int32_t)mat.tex_emissive);
+                emis = mat.emissive * mk3(t.x, t.y, t.z);
+            }
+            add_radiance(sidx, A, thr * emis);
+
+            bool stop = false;
+            if (kDebug && debug_view != 0u) {  // gather.wgsl:359-419
+                const f3 half = mk3(0.5f, 0.5f, 0.5f);
+                stop = true;
+                switch (debug_view) {
+                    case 1: A.col = mk3(uvx, uvy, 0.0f); break;
+                    case 2: A.col = sn * 0.5f + half; break;
+                    case 3: A.col = shn * 0.5f + half; break;
+                    case 4: A.col = gn * 0.5f + half; break;
+                    case 5: A.col = emis; break;
+                    case 8:
+                    case 9: {
+                        float pu = (float)px / (float)ip.width, pv = (float)py / (float)ip.height;
+                        float4 t =
+                            tex_sample(s.tex[debug_view == 8 ? RT_TEX_EMISSIVE : RT_TEX_ALBEDO], pu, pv, 0);
+                        A.col = mk3(t.x, t.y, t.z);
+                        break;
+                    }
+                    case 11: {
+                        float4 t = tex_sample(s.tex[RT_TEX_EMISSIVE], uvx, uvy, 0);
+                        A.col = mk3(t.x, t.y, t.z);
+                        break;
+                    }
+                    case 12: A.col = mat.emissive; break;
+                    case 13: A.col = mk3((float)mat.tex_emissive / 65535.0f, 0.0f, 0.0f); break;
+                    case 17: A.col = mk3(uvx - floorf(uvx), uvy - floorf(uvy), 0.0f); break;
+                    case 18: {
+                        float4 t = tex_sample(s.tex[RT_TEX_ALBEDO], uvx, uvy, (int32_t)mat.tex_albedo);
+                        A.col = mk3(t.x, t.y, t.z);
+                        break;
+                    }
+                    case 19:
+                    case 20: {
+                        f3 ft, fb;
+                        tangent_frame(tr, sn, ft, fb);
+                        A.col = (debug_view == 19 ? ft : fb) * 0.5f + half;
+                        break;
+                    }
+                    case 21: A.col = hp; break;
+                    default: stop = false; break;
+                }
+            }
+            if (stop) {
+                alive = false;
+            } else if (mat.kind == 2u) {  // dielectric (gather.wgsl:421-436)
+                float qd = (mat.ior - 1.0f) / (mat.ior + 1.0f);
+                float f0s = qd * qd;
+                float ct = fabsf(dot(rd, shn));
+                float fr = fresnel_schlick(ct, mk3(f0s, f0s, f0s)).x;
+                if (rng_f32(rng) < fr) {
+                    rd = reflect(rd, shn);
+                    ro = hp + shn * 0.001f;
+                } else {
+                    float eta = ff ? 1.0f / mat.ior : mat.ior;
+                    rd = refract(rd, shn, eta);
+                    ro = hp - shn * 0.001f;
+                    thr = thr * mat.albedo;
+                }
+            } else {  // metallic-roughness (gather.wgsl:439-537)
+                f3 f0 = mk3(0.04f * (1.0f - metal) + albedo.x * metal, 0.04f * (1.0f - metal) + albedo.y * metal,
+                            0.04f * (1.0f - metal) + albedo.z * metal);
+                f3 wo = -rd;
+                float a = fmaxf(rough * rough, 1e-3f);
+                f3 fr = fresnel_schlick(fabsf(dot(rd, shn)), f0);
+                f3 diffuse_weight = (1.0f - metal) * albedo;
+                float sp = max3(fr);
+                float dp = max3(diffuse_weight);
+                float ratio = sp / (sp + dp);
+                float spec_prob = clampf(sp + dp <= 0.0f ? 0.5f : ratio, 0.001f, 0.999f);
+                bool do_spec = rng_f32(rng) < spec_prob;
+                f3 dscale = diffuse_weight / (1.0f - spec_prob);
+
+                LightSample ls = light_sample(job, hp, shn, rng);
+                f3 c_nee;
+                if (!do_spec) {
+                    if (env_intensity > 0.0f)
+                        add_radiance(sidx, A, thr * dscale * sky_color(shn, env_color, env_horizon, env_intensity));
+                    c_nee = thr * dscale * ls.e / kPi;
+                    add_radiance(sidx, A, thr * albedo * ip.ambient);
+                } else {
+                    c_nee = thr * spec_ggx(wo, shn, ls.wi, a, f0) * ls.e / spec_prob;
+                }
+                bool nee_luma_only = false;
+                if (kPhotons && ip.use_photons == 1u && !do_spec) {  // gather.wgsl:473-514
+                    // The lookup runs in wf_photon_kernel right after this pass; its term
+                    // lands before this bounce's NEE term, as here.  Photon debug mode
+                    // overwrites the colour after the lookup and keeps only the luminance of
+                    // the NEE term, whatever the lookup finds.
+                    out.photon = true;
+                    out.ph_hp = hp;
+                    out.ph_n = shn;
+                    out.ph_td = thr * dscale;
+                    out.ph_sidx = sidx;
+                    if (ip.photon_debug == 1u) nee_luma_only = true;
+                }
+                if (ls.occlude && (c_nee.x != 0.0f || c_nee.y != 0.0f || c_nee.z != 0.0f)) {
+                    out.shadow = true;
+                    out.sh_o = ls.o;
+                    out.sh_d = ls.wi;
+                    out.sh_max = ls.max_dist;
+                    p.nee[slot] = make_float4(c_nee.x, c_nee.y, c_nee.z,
+                                              __uint_as_float((sidx & 0xFFFFu) | kNeePending |
+                                                              (nee_luma_only ? kNeeLumaOnly : 0u)));
+                }
+                if (do_spec) {
+                    rd = sample_spec_dir(rd, shn, a, rng);
+                    ro = hp + shn * 0.001f;
+                    f3 h = normalize(wo + rd);
+                    float ndl = fmaxf(dot(shn, rd), 0.0f);
+                    thr = thr * fresnel_schlick(fmaxf(dot(wo, h), 0.0f), f0) * smith_g1(ndl, a) / spec_prob;
+                } else {
+                    f3 local = sample_cosine_hemisphere(rng);
+                    rd = to_world(local, shn);
+                    ro = hp + shn * 0.001f;
+                    thr = thr * dscale;
+                    if (kPhotons && ip.use_photons == 1u) alive = false;
+                }
+                if (alive) {
+                    float pr = max3(thr);
+                    if (pr <= 0.0f || rng_f32(rng) > pr) alive = false;
+                    else thr = thr / pr;
+                }
+            }
+        }
+    }
+    // for-loop step: the segment index advances; the sample ends after max_bounces segments.
+    b += 1u;
+    if (alive && b >= job.max_bounces) alive = false;
+    if (!alive) {
+        sidx += 1u;
+        if (sidx < spp) {
+            camera_ray(job, px, py, rng, ro, rd);
+            thr = mk3(1.0f, 1.0f, 1.0f);
+            b = 0u;
+            out.keep = true;
+        }
+    } else {
+        out.keep = true;
+    }
+    if (!out.shadow && nee_word != 0u) p.nee[slot].w = 0.0f;
+    p.ro[slot] = make_float4(ro.x, ro.y, ro.z, __uint_as_float(rng.state));
+    p.rd[slot] = make_float4(rd.x, rd.y, rd.z, __uint_as_float(pack_sb(sidx, b)));
+    p.thr[slot] = make_float4(thr.x, thr.y, thr.z, __uint_as_float(jid));
+    acc[0] = make_float4(A.col.x, A.col.y, A.col.z, A.lum_sum);
+    acc[1] = make_float4(A.lum2_sum, acc1.y, acc1.z, acc1.w);
+    if (sidx0 < 8u) reinterpret_cast<float *>(acc + 2)[sidx0] = A.sl;
+    if (first_hit) p.nrm[slot] = nrm;
+    return out;
+}
+
+// The photon-map lookup of sample sidx of the path in `slot`: hit point hp, shading normal shn, throughput x
+// diffuse weight td.
+__device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob &job, uint32_t slot, uint32_t sidx, f3 hp,
+                                              f3 shn, f3 td) {
+    const rt_image_params &ip = job.ip;
+    const rt_grid_params &gp = job.gp;
+    const float r2max = ip.photon_radius * ip.photon_radius;
+    f3 ph_sum = mk3(0.0f, 0.0f, 0.0f);
+    uint32_t ph_hits = 0u, budget = 384u;
+    bool done = false;
+    const int32_t bx = f2i_sat((hp.x - gp.room_min_x) / gp.cell_size);
+    const int32_t by = f2i_sat((hp.y - gp.room_min_y) / gp.cell_size);
+    const int32_t bz = f2i_sat((hp.z - gp.room_min_z) / gp.cell_size);
+    const int32_t gxmax = (int32_t)gp.grid_x - 1, gymax = (int32_t)gp.grid_y - 1, gzmax = (int32_t)gp.grid_z - 1;
+    // The 27 cells in the reference's order (dz, then dy, then dx), walked as one flat loop over
+    // (cell, photon group) so each thread moves to its next cell on its own instead of the warp
+    // waiting at every cell for its fullest one.
+    auto cell_at = [&](uint32_t i) {
+        const int32_t dz = (int32_t)(i / 9u) - 1, dy = (int32_t)((i / 3u) % 3u) - 1, dx = (int32_t)(i % 3u) - 1;
+        const int32_t cx = clampi((int32_t)((uint32_t)bx + (uint32_t)dx), 0, gxmax);
+        const int32_t cy = clampi((int32_t)((uint32_t)by + (uint32_t)dy), 0, gymax);
+        const int32_t cz = clampi((int32_t)((uint32_t)bz + (uint32_t)dz), 0, gzmax);
+        return (uint32_t)cx + (uint32_t)cy * gp.grid_x + (uint32_t)cz * gp.grid_x * gp.grid_y;
+    };
+    // Photon indices are u32 and clamped to the last sorted photon (the backend's rule for an
+    // out-of-range index; the grid's ranges never leave the array).
+    const uint32_t last = (uint32_t)job.sorted_count - 1u;
+    const float4 *posv = job.sorted_pos ? job.sorted_pos : job.sorted_photons;
+    const uint32_t pstride = job.sorted_pos ? 1u : 4u;
+    uint32_t ci = 0u, k = 0u;
+    uint2 m = __ldg(job.grid_meta + cell_at(0u));
+    if (job.sorted_count == 0u) m.y = 0u, ci = 27u;
+    while (!done) {
+        if (k >= m.y) {
+            if (++ci >= 27u) break;  // also ends at once for an empty photon map
+            m = __ldg(job.grid_meta + cell_at(ci));
+            k = 0u;
+            continue;
+        }
+        // A group of four photons: positions loaded together (from the compact position array
+        // when there is one), then tested in order with the budget and the hit cap.
+        float4 pos[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j) pos[j] = __ldg(posv + (size_t)min(m.x + k + j, last) * pstride);
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j) {
+            if (done || k + j >= m.y) break;
+            if (budget == 0u) {
+                done = true;
+                break;
+            }
+            budget -= 1u;
+            const f3 dd = xyz(pos[j]) - hp;
+            const float d2 = dot(dd, dd);
+            if (d2 < r2max) {
+                const float4 *ph = job.sorted_photons + 4ull * min(m.x + k + j, last);
+                const f3 pw = xyz(__ldg(ph + 1));
+                const f3 inc = xyz(__ldg(ph + 2));
+                ph_sum = ph_sum + pw * fmaxf(dot(shn, -inc), 0.0f);
+                ph_hits += 1u;
+                if (ph_hits >= 64u) done = true;
+            }
+        }
+        k += 4u;
+    }
+    if (ph_hits > 0u)
+        acc_add_term(p, slot, sidx,
+                     td * ph_sum * ip.photon_scale / (kPi * (float)ph_hits * ip.photon_radius * ip.photon_radius),
+                     false);
+    if (ip.photon_debug == 1u) {
+        const float density = fminf((float)ph_hits / 64.0f, 1.0f);
+        const f3 col = mk3(1.0f - density, density, 0.0f) * 2.0f;
+        float4 *a = p.acc + 4 * (size_t)slot;
+        a[0] = make_float4(col.x, col.y, col.z, a[0].w);
+    }
+}
+
+// Whether the light of an occlusion ray in a scene with cut-out materials is visible (gather.wgsl:91-103):
+// its closest hit (hit_word) lies at or beyond the limit, or is cut away there by its texture's alpha.  Out of
+// line: few scenes need it, and its registers would weigh on the traversal.
+static __device__ __noinline__ bool cut_out_lit(const DevScene &s, float4 ro, float4 rd, float limit,
+                                         unsigned long long hit) {
+    const float t = hit_t(hit);
+    if (t >= limit) return true;  // (not for a NaN limit, which counts as occluded)
+    const TriFull bt = load_tri(s, t < kInf ? __float_as_uint(__ldg(s.tri_ord + 3ull * (uint32_t)hit).w) : 0u);
+    const Mat bm = load_mat(s, bt.material_id);
+    if ((bm.flags & RT_MAT_FLAG_ALPHA_CUTOUT) == 0u || bm.tex_albedo == RT_TEX_NONE) return false;
+    const Bary b = barycentric(bt, xyz(ro), xyz(rd), t);
+    return tex_sample(s.tex[RT_TEX_ALBEDO], b.uvx, b.uvy, (int32_t)bm.tex_albedo).w < 0.5f;
+}
+
+// How far a ray that looks for its closest hit below a limit searches: a little beyond it, so that
+// rounding in a box's entry cannot lose a hit before it.
+__device__ __forceinline__ float search_limit(float limit) { return limit > kEps ? limit * 1.001f : kInf; }
+
+// The pixel in `slot`: the last NEE term, the firefly sigma clamp and the frame outputs (gather.wgsl:548-593).
+__device__ __forceinline__ void finalize_slot(const WaveParams &p, const DevJob &job, uint32_t slot) {
+    const uint32_t pix = slot - job.base;
+    if (pix >= job.npix) return;
+    const uint32_t spp = job.spp;
+    Accum A = load_acc(p, slot);
+    const float4 nee = p.nee[slot];
+    if (__float_as_uint(nee.w) & kNeeLit) {  // the last bounce's term
+        const uint32_t word = __float_as_uint(nee.w), s = word & 0xFFFFu;
+        const float l = luma(xyz(nee));
+        if (!(word & kNeeLumaOnly)) A.col = A.col + xyz(nee);
+        A.lum_sum += l;
+        A.lum2_sum += l * l;
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; ++i)
+            if (i == s) A.sl[i] += l;
+    }
+    const float first_depth = p.acc[4 * (size_t)slot + 1].y;
+    const float4 nrm = p.nrm[slot];
+    if (spp <= 8u) {
+        float *sl = A.sl;
+        for (uint32_t i = 1; i < spp; ++i) {
+            float key = sl[i];
+            uint32_t j = i;
+            while (j > 0u && sl[j - 1u] > key) {
+                sl[j] = sl[j - 1u];
+                j -= 1u;
+            }
+            sl[j] = key;
+        }
+        float median = (sl[(spp - 1u) / 2u] + sl[spp / 2u]) * 0.5f;
+        uint32_t half = spp / 2u > 1u ? spp / 2u : 1u;
+        float spread = 0.0f;
+        for (uint32_t i = 0; i < half; ++i) {
+            float dd = sl[i] - median;
+            spread += dd * dd;
+        }
+        float sigma = fmaxf(sqrtf(spread / (float)half), 0.25f * median + 1e-5f);
+        float thresh = median + 3.0f * sigma;
+        float cl = 0.0f, cl2 = 0.0f;
+        for (uint32_t i = 0; i < spp; ++i) {
+            float lc = fminf(sl[i], thresh);
+            cl += lc;
+            cl2 += lc * lc;
+        }
+        A.col = A.col * (cl / fmaxf(A.lum_sum, 1e-10f));
+        A.lum_sum = cl;
+        A.lum2_sum = cl2;
+    }
+    f3 col = vmin(A.col / (float)spp, mk3(10.0f, 10.0f, 10.0f));
+    job.frame[pix] = make_float4(col.x, col.y, col.z, 1.0f);
+    job.moments[pix] = make_float4(fminf(A.lum_sum / (float)spp, 10.0f), fminf(A.lum2_sum / (float)spp, 100.0f), 0.0f, 0.0f);
+    job.gbuffer[pix] = make_float4(nrm.x, nrm.y, nrm.z, first_depth);
+}
+
+}  // namespace rtd

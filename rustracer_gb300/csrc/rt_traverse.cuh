@@ -22,7 +22,7 @@
 // in a million) is walked again, waiting for the tests of each record's leaves before it goes on.  Results
 // do not depend on which rays share a warp.
 #pragma once
-#include "rt_device.cuh"
+#include "rt_kernels.h"
 
 namespace rtd {
 
@@ -50,7 +50,8 @@ struct __align__(16) WarpTrav {
     uint32_t coming;          // rays being copied
     unsigned long long best[32];  // t bits << 32 | prim slot
     uint32_t second[32];          // bits of the second nearest hit's t
-    float limit[32];              // occlusion rays: hits below it count
+    float limit[32];              // occlusion rays that look for the closest hit: hits below it count
+    float margin[32];             // the scene's tie margin (launches over several scenes)
     uint2 leaf[kLeafCap];         // queued leaves: first prim slot, count << 5 | owner lane
 };
 
@@ -283,6 +284,112 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
             if (key[i] < kNone) trav_push<kBlock>(st, top, deep, ref[i], key[i]);
         visiting = trav_settle<kBlock>(st, top, deep);
     }
+}
+
+// A lane and its ray: idle, or walking until it visits no more records.
+struct LaneWalk {
+    TravLane st;
+    bool busy, visiting;
+    bool any_hit;        // an occlusion ray that may stop at its first hit below st.t
+    bool found;          // a hit below the starting st.t
+    bool careful, held;  // walked again; waits for its leaves' tests
+};
+
+// The ray at the root with st.t, and no hit yet.
+__device__ __forceinline__ void walk_root(LaneWalk &r, WarpTrav &w) {
+    const uint32_t lane = threadIdx.x & 31u;
+    w.best[lane] = hit_word(r.st.t, 0u);
+    // (an occlusion ray that may stop early takes no interest in hits beyond its limit)
+    w.second[lane] = r.any_hit ? __float_as_uint(r.st.t) : 0x7F800000u;
+    r.st.node = 0u;
+    r.st.te = -kInf;
+    r.st.sp = 0u;
+}
+// Gives the lane a ray to walk (r.st.t, records and cap and r.any_hit are set): origin o, direction d, the
+// scene's triangles.
+__device__ __forceinline__ void walk_begin(LaneWalk &r, WarpTrav &w, f3 o, f3 d, f3 inv, const float4 *tris) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long tp = (unsigned long long)tris;
+    w.ro[lane] = make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)tp));
+    w.rd[lane] = make_float4(d.x, d.y, d.z, __uint_as_float((uint32_t)(tp >> 32)));
+    r.st.minus_ro[0] = pack2(-o.x, -o.x);
+    r.st.minus_ro[1] = pack2(-o.y, -o.y);
+    r.st.minus_ro[2] = pack2(-o.z, -o.z);
+    r.st.inv[0] = pack2(inv.x, inv.x);
+    r.st.inv[1] = pack2(inv.y, inv.y);
+    r.st.inv[2] = pack2(inv.z, inv.z);
+    walk_root(r, w);
+    r.found = r.careful = false;
+    r.busy = true;
+}
+
+// Up to max_steps records for every lane of a warp (fewer once `few` or less lanes still walk), the queued
+// leaves tested eight at a time; then the rest of them, so that a lane that is no longer visiting has its
+// result.  visits and tests (kCount) count the lane's records and triangles.
+template <bool kWide, int kTree, int kBlock, bool kMulti, bool kCount>
+__device__ __forceinline__ void walk_records(LaneWalk &r, WarpTrav &w, uint2 *top, uint2 *deep, const Treelet &tree,
+                                             const float4 *records, const float4 *tris, uint32_t max_steps, int few,
+                                             uint32_t &visits, uint32_t &tests) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t queued = 0u;
+    for (uint32_t k = 0;;) {
+        uint32_t n = 0u;
+        if (kCount && r.visiting) visits += 1u;
+        trav_step<kWide, kTree, kBlock, kMulti>(r.st, top, deep, r.visiting, r.careful, w, queued, tree, records, n);
+        if (kCount) tests += n;
+        if (r.careful && n != 0u) {
+            r.held = r.visiting;
+            r.visiting = false;
+        }
+        const bool end = ++k >= max_steps || __popc(__ballot_sync(0xFFFFFFFFu, r.visiting)) <= few;
+        if (queued >= 8u || (end && queued != 0u)) {
+            const uint32_t tested = end ? queued : queued & ~7u, left = queued - tested;
+            __syncwarp();
+            for (uint32_t g = 0u; g < tested; g += 8u) test_leaves<kMulti>(w, g, min(8u, tested - g), tris);
+            if (left != 0u) {  // the leaves left over move to the front
+                const uint2 leaf = w.leaf[tested + (lane & 7u)];
+                __syncwarp();
+                if (lane < left) w.leaf[lane] = leaf;
+            }
+            __syncwarp();
+            queued = left;
+            if (r.busy) {
+                const float t = hit_t(w.best[lane]);
+                if (t < r.st.t) {
+                    r.found = true;
+                    if (r.any_hit) r.visiting = false;
+                }
+                r.st.t = t;
+                if (r.visiting || r.held) r.visiting = trav_settle<kBlock>(r.st, top, deep);
+                r.held = false;
+            }
+        }
+        if (end) break;
+    }
+}
+
+// Whether a ray that looked for its closest hit and is done has to be walked again, carefully (see the top of
+// this file); `start` is the t it started with.
+template <bool kMulti>
+__device__ __forceinline__ bool walk_again(LaneWalk &r, WarpTrav &w, const float4 *tris, float margin, float start) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long hit = w.best[lane];
+    const float t = hit_t(hit), second = __uint_as_float(w.second[lane]);
+    if (r.careful || !(second <= t + (t * kTieRelative + margin))) return false;
+    const float4 ro = w.ro[lane], rd = w.rd[lane];
+    if (kMulti) tris = ray_triangles(ro, rd);
+    if (hit_entry_bound(tris, (uint32_t)hit, xyz(ro), xyz(rd), margin * 0x1p-5f) < second) return false;
+    r.st.t = start;
+    walk_root(r, w);
+    r.careful = r.visiting = true;
+    return true;
+}
+
+// Dynamic shared memory of a traversal block: the lane-interleaved stack tops, one WarpTrav per warp, then
+// the treelet (four-wide launches with a treelet).
+inline size_t trav_smem_bytes(uint32_t block_threads, bool tree) {
+    return (size_t)kTopStack * block_threads * sizeof(uint2) + (block_threads / 32u) * sizeof(WarpTrav) +
+           (tree ? (size_t)kTreeletRecords * 8u * sizeof(float4) : 0u);
 }
 
 }  // namespace rtd
