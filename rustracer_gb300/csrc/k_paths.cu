@@ -36,6 +36,9 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     uint2 *top = reinterpret_cast<uint2 *>(trav_smem) + threadIdx.x;
     uint2 deep[kMaxStack - kTopStack];
     WarpTrav &w = reinterpret_cast<WarpTrav *>(trav_smem + sizeof(uint2) * kTopStack * kPathsBlock)[threadIdx.x >> 5];
+    // Between walks the warp's traversal state and stacks hold the photon lookups' runs.
+    const LookupRuns runs{reinterpret_cast<uint2 *>(&w) + lane, top, kPathsBlock};
+    static_assert(sizeof(WarpTrav) >= 32 * kRunsA * sizeof(uint2) && kTopStack >= kLookupCells - kRunsA, "lookup runs");
     const Treelet tree{nullptr, nullptr, 0u};
     LaneWalk r;
     r.busy = r.visiting = r.any_hit = r.careful = r.held = false;
@@ -177,9 +180,10 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                 }
                 out = shade_path<kPhotons, false>(p, slot, hit_dist, prim, word >> 2, lit);
                 if (kPhotons && out.photon)
-                    photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td);
+                    photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td, runs);
                 alive = out.keep;
             }
+            if (kPhotons) __syncwarp();
         }
         if (kWhole && mine) finalize_slot(p, job, slot);
     }

@@ -188,10 +188,13 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ WaveParams p, uint32_t iter) {
     const uint32_t n = p.counts[4 * iter + 3];
+    __shared__ uint2 s_runs[4][kLookupCells * 32];
+    uint2 *mine = s_runs[threadIdx.x >> 5] + (threadIdx.x & 31u);
+    const LookupRuns runs{mine, mine + 32u * kRunsA, 32u};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 r0 = p.preq[3ull * i], r1 = p.preq[3ull * i + 1], r2 = p.preq[3ull * i + 2];
         photon_lookup(p, p.jobs[__float_as_uint(r2.w)], __float_as_uint(r0.w), __float_as_uint(r1.w), xyz(r0), xyz(r1),
-                      xyz(r2));
+                      xyz(r2), runs);
     }
 }
 

@@ -495,74 +495,137 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveParams &p, uint32_t slo
     return out;
 }
 
-// The photon-map lookup of sample sidx of the path in `slot`: hit point hp, shading normal shn, throughput x
-// diffuse weight td.
+// The photons a lookup may examine, as runs of the sorted array: at most one run per cell of the 27.  Lane l
+// of a warp keeps run i at a[32 i + l] for i < kRunsA, the rest at b[b_stride (i - kRunsA)].
+constexpr uint32_t kLookupCells = 27u, kRunsA = 16u;
+struct LookupRuns {
+    uint2 *a, *b;
+    uint32_t b_stride;
+    __device__ __forceinline__ uint2 &operator[](uint32_t i) const {
+        return i < kRunsA ? a[32u * i] : b[b_stride * (i - kRunsA)];
+    }
+};
+
+// Squared distance along one axis from x to the photons of cell c: none lie nearer than its faces, less
+// `margin` for the rounding in the key; those below the grid are kept in cell 0, and those beyond it in the
+// cells of the next row or plane, a grid's width away.
+__device__ __forceinline__ float cell_distance2(float x, float grid_min, float cell, int32_t c, float margin) {
+    const float lo = grid_min + (float)c * cell;
+    const float d = fmaxf(c == 0 ? 0.0f : lo - x, x - (lo + cell)) - margin;
+    return d > 0.0f ? d * d : 0.0f;
+}
+
+// The photon-map lookup (gather.wgsl:473-514) of sample sidx of the path in `slot`: hit point hp, shading normal
+// shn, throughput x diffuse weight td.
+//
+// The reference examines the 27 cells around the hit point in order (dz, then dy, then dx), at most 384
+// photons, and adds the first 64 within the radius.  First the photons to test are laid out as runs: cells
+// farther than the radius only use up the budget, neighbouring cells of a row merge.  With radius = cell / 2
+// on a surface, four of its nine occupied cells remain.  Then the runs are tested as one flat loop over
+// groups of eight photons, so a thread moves to its next run by itself.  Bound by the latency of the photon
+// loads (issue 35% busy), so a group's tests come before its hits: 1920 x 1080 at 4 spp, 2^20 photons in 128^3
+// cells, 3.19 ms of lookups per frame before (every cell tested, a hit's loads between the tests of a group of
+// four), 2.38 with the runs, 2.07 with the hits after the tests, 1.79 with groups of eight (sixteen: 1.76, and
+// slower for few lookups).
 __device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob &job, uint32_t slot, uint32_t sidx, f3 hp,
-                                              f3 shn, f3 td) {
+                                              f3 shn, f3 td, const LookupRuns &runs) {
     const rt_image_params &ip = job.ip;
     const rt_grid_params &gp = job.gp;
-    const float r2max = ip.photon_radius * ip.photon_radius;
-    f3 ph_sum = mk3(0.0f, 0.0f, 0.0f);
-    uint32_t ph_hits = 0u, budget = 384u;
-    bool done = false;
-    const int32_t bx = f2i_sat((hp.x - gp.room_min_x) / gp.cell_size);
-    const int32_t by = f2i_sat((hp.y - gp.room_min_y) / gp.cell_size);
-    const int32_t bz = f2i_sat((hp.z - gp.room_min_z) / gp.cell_size);
-    const int32_t gxmax = (int32_t)gp.grid_x - 1, gymax = (int32_t)gp.grid_y - 1, gzmax = (int32_t)gp.grid_z - 1;
-    // The 27 cells in the reference's order (dz, then dy, then dx), walked as one flat loop over
-    // (cell, photon group) so each thread moves to its next cell on its own instead of the warp
-    // waiting at every cell for its fullest one.
-    auto cell_at = [&](uint32_t i) {
-        const int32_t dz = (int32_t)(i / 9u) - 1, dy = (int32_t)((i / 3u) % 3u) - 1, dx = (int32_t)(i % 3u) - 1;
-        const int32_t cx = clampi((int32_t)((uint32_t)bx + (uint32_t)dx), 0, gxmax);
-        const int32_t cy = clampi((int32_t)((uint32_t)by + (uint32_t)dy), 0, gymax);
-        const int32_t cz = clampi((int32_t)((uint32_t)bz + (uint32_t)dz), 0, gzmax);
-        return (uint32_t)cx + (uint32_t)cy * gp.grid_x + (uint32_t)cz * gp.grid_x * gp.grid_y;
-    };
+    const float radius = ip.photon_radius, r2max = radius * radius, cell = gp.cell_size;
+    const int32_t bx = f2i_sat((hp.x - gp.room_min_x) / cell);
+    const int32_t by = f2i_sat((hp.y - gp.room_min_y) / cell);
+    const int32_t bz = f2i_sat((hp.z - gp.room_min_z) / cell);
+    const int32_t gx = (int32_t)gp.grid_x, gy = (int32_t)gp.grid_y, gz = (int32_t)gp.grid_z;
+    uint32_t n_runs = 0u;
+    if (job.sorted_count != 0u) {
+        // Cells may be passed over when a hit point this near the grid is farther than the radius from every
+        // photon that some other row's or plane's overflow put among theirs.
+        const float wide = (float)min(gx, min(gy, gz)) - 2.0f;
+        const bool pass = bx >= -1 && by >= -1 && bz >= -1 && bx <= gx && by <= gy && bz <= gz && wide * cell > radius * 1.01f;
+        const float far2 = pass ? r2max * (1.0f + 0x1p-18f) : __int_as_float(0x7F800000);
+        const float margin = 0x1p-19f * (fabsf(gp.room_min_x) + fabsf(gp.room_min_y) + fabsf(gp.room_min_z) +
+                                         (float)max(gx, max(gy, gz)) * cell);
+        int32_t cx[3], cy[3], cz[3];
+        float dx2[3], dy2[3], dz2[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            cx[d] = clampi((int32_t)((uint32_t)bx + (uint32_t)(d - 1)), 0, gx - 1);
+            cy[d] = clampi((int32_t)((uint32_t)by + (uint32_t)(d - 1)), 0, gy - 1);
+            cz[d] = clampi((int32_t)((uint32_t)bz + (uint32_t)(d - 1)), 0, gz - 1);
+            dx2[d] = cell_distance2(hp.x, gp.room_min_x, cell, cx[d], margin);
+            dy2[d] = cell_distance2(hp.y, gp.room_min_y, cell, cy[d], margin);
+            dz2[d] = cell_distance2(hp.z, gp.room_min_z, cell, cz[d], margin);
+        }
+        uint32_t budget = 384u;
+        uint2 run = make_uint2(0u, 0u);
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+#pragma unroll
+            for (int y = 0; y < 3; ++y) {
+                const uint2 *row = job.grid_meta + ((uint32_t)cy[y] * gp.grid_x + (uint32_t)cz[z] * gp.grid_x * gp.grid_y);
+                const float row2 = dy2[y] + dz2[z];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    const uint2 m = __ldg(row + cx[x]);
+                    const uint32_t take = min(m.y, budget);
+                    budget -= take;
+                    if (take != 0u && !(row2 + dx2[x] > far2)) {
+                        if (run.x + run.y == m.x && run.y != 0u) {
+                            run.y += take;
+                        } else {
+                            if (run.y != 0u) runs[n_runs++] = run;
+                            run = make_uint2(m.x, take);
+                        }
+                    }
+                }
+            }
+        }
+        if (run.y != 0u) runs[n_runs++] = run;
+    }
     // Photon indices are u32 and clamped to the last sorted photon (the backend's rule for an
     // out-of-range index; the grid's ranges never leave the array).
     const uint32_t last = (uint32_t)job.sorted_count - 1u;
     const float4 *posv = job.sorted_pos ? job.sorted_pos : job.sorted_photons;
     const uint32_t pstride = job.sorted_pos ? 1u : 4u;
-    uint32_t ci = 0u, k = 0u;
-    uint2 m = __ldg(job.grid_meta + cell_at(0u));
-    if (job.sorted_count == 0u) m.y = 0u, ci = 27u;
-    while (!done) {
-        if (k >= m.y) {
-            if (++ci >= 27u) break;  // also ends at once for an empty photon map
-            m = __ldg(job.grid_meta + cell_at(ci));
-            k = 0u;
-            continue;
+    f3 ph_sum = mk3(0.0f, 0.0f, 0.0f);
+    uint32_t ph_hits = 0u;
+    bool done = n_runs == 0u;
+    uint2 m = done ? make_uint2(0u, 0u) : runs[0];
+    for (uint32_t ri = 1u; !done;) {
+        if (m.y == 0u) {
+            if (ri >= n_runs) break;
+            m = runs[ri++];
         }
-        // A group of four photons: positions loaded together (from the compact position array
-        // when there is one), then tested in order with the budget and the hit cap.
-        float4 pos[4];
+        // A group of eight photons: positions loaded together (from the compact position array when there
+        // is one) and tested, then the hits among them in order, up to the hit cap.
+        float4 pos[8];
 #pragma unroll
-        for (uint32_t j = 0; j < 4u; ++j) pos[j] = __ldg(posv + (size_t)min(m.x + k + j, last) * pstride);
+        for (uint32_t j = 0; j < 8u; ++j) pos[j] = __ldg(posv + (size_t)min(m.x + j, last) * pstride);
+        const uint32_t group = min(m.y, 8u);
+        uint32_t hits = 0u;
 #pragma unroll
-        for (uint32_t j = 0; j < 4u; ++j) {
-            if (done || k + j >= m.y) break;
-            if (budget == 0u) {
+        for (uint32_t j = 0; j < 8u; ++j) {
+            const f3 dd = xyz(pos[j]) - hp;
+            const float d2 = dot(dd, dd);
+            if (j < group && d2 < r2max) hits |= 1u << j;
+        }
+        while (hits) {
+            const uint32_t j = __ffs(hits) - 1u;
+            hits &= hits - 1u;
+            const float4 *ph = job.sorted_photons + 4ull * min(m.x + j, last);
+            const f3 pw = xyz(__ldg(ph + 1));
+            const f3 inc = xyz(__ldg(ph + 2));
+            ph_sum = ph_sum + pw * fmaxf(dot(shn, -inc), 0.0f);
+            if (++ph_hits >= 64u) {
                 done = true;
                 break;
             }
-            budget -= 1u;
-            const f3 dd = xyz(pos[j]) - hp;
-            const float d2 = dot(dd, dd);
-            if (d2 < r2max) {
-                const float4 *ph = job.sorted_photons + 4ull * min(m.x + k + j, last);
-                const f3 pw = xyz(__ldg(ph + 1));
-                const f3 inc = xyz(__ldg(ph + 2));
-                ph_sum = ph_sum + pw * fmaxf(dot(shn, -inc), 0.0f);
-                ph_hits += 1u;
-                if (ph_hits >= 64u) done = true;
-            }
         }
-        k += 4u;
+        m.x += group;
+        m.y -= group;
     }
     if (ph_hits > 0u)
-        acc_add_term(p, slot, sidx,
-                     td * ph_sum * ip.photon_scale / (kPi * (float)ph_hits * ip.photon_radius * ip.photon_radius),
+        acc_add_term(p, slot, sidx, td * ph_sum * ip.photon_scale / (kPi * (float)ph_hits * ip.photon_radius * ip.photon_radius),
                      false);
     if (ip.photon_debug == 1u) {
         const float density = fminf((float)ph_hits / 64.0f, 1.0f);
