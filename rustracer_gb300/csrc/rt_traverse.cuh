@@ -246,7 +246,10 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
             key[c] = hit && n == 0u ? te : kNone;  // +inf: not a pending child
         }
     }
-    // Hit leaves into the queue, child by child in lane order.
+    uint32_t anyl = cnt[0];
+#pragma unroll
+    for (int c = 1; c < K; ++c) anyl |= cnt[c];
+    if (__any_sync(0xFFFFFFFFu, anyl != 0u))
 #pragma unroll
     for (int c = 0; c < K; ++c) {
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, cnt[c] != 0u);
@@ -279,9 +282,22 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
         }
         st.node = ref[0];
         st.te = key[0];
+        if (key[1] < kNone) {
+            if (st.sp + (K - 1) <= kTopStack) {
+                uint2 *e = top + st.sp * kBlock;
 #pragma unroll
-        for (int i = K - 1; i >= 1; --i)
-            if (key[i] < kNone) trav_push<kBlock>(st, top, deep, ref[i], key[i]);
+                for (int i = K - 1; i >= 1; --i) {
+                    const bool on = key[i] < kNone;
+                    if (on) *e = make_uint2(ref[i], __float_as_uint(key[i]));
+                    e += on ? kBlock : 0;
+                    st.sp += on ? 1u : 0u;
+                }
+            } else {
+#pragma unroll
+                for (int i = K - 1; i >= 1; --i)
+                    if (key[i] < kNone) trav_push<kBlock>(st, top, deep, ref[i], key[i]);
+            }
+        }
         visiting = trav_settle<kBlock>(st, top, deep);
     }
 }
