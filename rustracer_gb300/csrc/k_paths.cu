@@ -29,6 +29,8 @@ template <bool kMulti, bool kPhotons, bool kWhole>
 __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kernel(const __grid_constant__ WaveParams p,
                                                                                   uint32_t iter, uint32_t most) {
     extern __shared__ __align__(16) unsigned char trav_smem[];
+    grid_dependency_wait();
+    grid_launch_dependents();
     // kWhole: `most` pixel positions, 8 x 4 tiles as in generate; otherwise the paths queued for `iter`.
     const uint32_t n = kWhole ? most : p.counts[4 * iter];
     if (!kWhole && n > most) return;
@@ -225,11 +227,11 @@ cudaError_t launch_paths_frame(const WaveParams &p, uint32_t tiles, bool multi, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, int num_sms,
-                              cudaStream_t st) {
+cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, bool early,
+                              int num_sms, cudaStream_t st) {
     const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
-    paths_kernel<false>(multi, photons)<<<blocks, kPathsBlock, trav_smem_bytes(kPathsBlock, false), st>>>(p, iter, most);
-    return cudaGetLastError();
+    return launch_dependent_if(early, paths_kernel<false>(multi, photons), blocks, kPathsBlock,
+                               trav_smem_bytes(kPathsBlock, false), st, p, iter, most);
 }
 
 }  // namespace rtd

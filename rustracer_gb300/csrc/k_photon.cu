@@ -218,6 +218,7 @@ __device__ bool photon_bounce(const PhotonTraceParams &p, uint32_t photon_index,
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) ph_generate_kernel(const __grid_constant__ PhotonTraceParams p,
                                                           const PhotonWave w) {
+    grid_launch_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t photon_index = p.photon_begin + i;
     bool live = false;
@@ -236,6 +237,8 @@ __global__ void __launch_bounds__(256) ph_generate_kernel(const __grid_constant_
 
 __global__ void __launch_bounds__(128) ph_shade_kernel(const __grid_constant__ PhotonTraceParams p, const PhotonWave w,
                                                        uint32_t iter) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t n = w.counts[4 * iter];
     const uint32_t *q = w.queue[iter & 1u];
     const bool last = iter + 1u >= RT_MAX_BOUNCES;
@@ -308,7 +311,7 @@ cudaError_t launch_photon_wave(const PhotonTraceParams &p, const PhotonWave &w, 
     const uint32_t shade_grid = (uint32_t)(shade_needed < shade_cap ? shade_needed : shade_cap);
     for (uint32_t it = 0; it < RT_MAX_BOUNCES; ++it) {
         if ((e = launch_extend(wp, it, n, p.scene, num_sms, tune, st)) != cudaSuccess) return e;
-        ph_shade_kernel<<<shade_grid, 128, 0, st>>>(p, w, it);
+        if ((e = launch_dependent(ph_shade_kernel, shade_grid, 128u, 0, st, p, w, it)) != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
@@ -1133,24 +1136,6 @@ __global__ void __launch_bounds__(kOrderWarps * 32, 4) cell_gather_kernel(const 
     }
 }
 
-// Launches `kernel` as a programmatic dependent of the previous kernel in the stream: its blocks may
-// be scheduled before that kernel has finished and wait for it in grid_dependency_wait().
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t st,
-                                    Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 cudaError_t launch_grid_build(const GridBuffers &g, cudaStream_t st) {
     cudaError_t e;
     const uint32_t C = g.num_cells;
@@ -1197,19 +1182,19 @@ cudaError_t launch_grid_build(const GridBuffers &g, cudaStream_t st) {
                                                                          chunks + 1, g.total + 1);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (ct == 1u)
-            e = launch_dependent(scan_lookback_list_kernel<1>, chunks, kScanThreads, st, g.counts, C, g.scan_partials,
+            e = launch_dependent(scan_lookback_list_kernel<1>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
                                  chunks, g.meta, vec, g.cursor, g.total + 1, g.total);
         else if (ct == 2u)
-            e = launch_dependent(scan_lookback_list_kernel<2>, chunks, kScanThreads, st, g.counts, C, g.scan_partials,
+            e = launch_dependent(scan_lookback_list_kernel<2>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
                                  chunks, g.meta, vec, g.cursor, g.total + 1, g.total);
         else
-            e = launch_dependent(scan_lookback_list_kernel<4>, chunks, kScanThreads, st, g.counts, C, g.scan_partials,
+            e = launch_dependent(scan_lookback_list_kernel<4>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
                                  chunks, g.meta, vec, g.cursor, g.total + 1, g.total);
         if (e != cudaSuccess) return e;
-        if ((e = launch_dependent(scatter_rank_kernel, grid_for((n + 7) / 8, 256, 8), 256, st, g.keys,
+        if ((e = launch_dependent(scatter_rank_kernel, grid_for((n + 7) / 8, 256, 8), 256, 0, st, g.keys,
                                   (const uint32_t *)g.rank, n, (const uint2 *)g.meta, g.order)) != cudaSuccess)
             return e;
-        return launch_dependent(cell_gather_kernel, grid_for((uint64_t)C * 32, kOrderWarps * 32, 4), kOrderWarps * 32, st,
+        return launch_dependent(cell_gather_kernel, grid_for((uint64_t)C * 32, kOrderWarps * 32, 4), kOrderWarps * 32, 0, st,
                                 (const uint2 *)g.meta, (const uint32_t *)g.cursor, (const uint32_t *)(g.total + 1),
                                 g.order, g.photons, g.sorted, g.sorted_pos, wide);
     }

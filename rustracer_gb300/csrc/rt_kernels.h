@@ -94,11 +94,11 @@ cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t
                              const WaveTuning &tune, cudaStream_t st, WaveProfile *prof = nullptr);
 // The gather pass of few paths in one launch (k_paths.cu): a whole frame of at most paths_limit pixels in
 // `tiles` 8 x 4 tiles, or, if at most `most` paths are queued for iteration `iter` (traced, not yet shaded),
-// the rest of theirs.
+// the rest of theirs (early: as a programmatic dependent).
 uint32_t paths_limit(int num_sms);
 cudaError_t launch_paths_frame(const WaveParams &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st);
-cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, int num_sms,
-                              cudaStream_t st);
+cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, bool early,
+                              int num_sms, cudaStream_t st);
 void prepare_paths_kernels();
 int device_sm_count();
 // One-time kernel attributes (shared-memory opt-ins); call before capturing launches into a graph.
@@ -174,5 +174,29 @@ cudaError_t launch_denoise(const float4 *in, float4 *out, const float4 *gbuffer,
 cudaError_t launch_resolve(const float4 *frame, float4 *accum, const float4 *gbuffer, uint32_t width,
                            uint32_t height, float alpha, const float *alpha_dev, const rt_tonemap_params &tp,
                            uchar4 *out, cudaStream_t st);
+
+// Launches `kernel` as a programmatic dependent of the previous kernel in the stream: its blocks may be
+// scheduled as that kernel's blocks leave and wait for its end in grid_dependency_wait(), which every such
+// kernel calls before it touches memory.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent_if(bool early, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                                cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                             Args... args) {
+    return launch_dependent_if(true, kernel, grid, block, smem, st, args...);
+}
 
 }  // namespace rtd
