@@ -5,21 +5,18 @@
 //                         bounce body also emits the u32 cell key of every slot it stores
 //                         (photon_count.wgsl:18-23), so the grid build never re-reads positions.
 //   photon_keys_kernel    keys of a photon buffer loaded from the host (same key function).
-//   grid build            exact u32 counting sort of the slots by cell key; without per-slot ranks
-//                         (the no-allocation entry, whose scratch holds no rank array):
-//     count_kernel        histogram (photon_count.wgsl:25-34)
-//     scan_*              device exclusive scan of the counts into (start, count) pairs; replaces the
-//                         blocking read-back and host scan of lib.rs:956-1007
-//     scatter_kernel      slot index to start + cursor (photon_scatter.wgsl:61-71)
-//     multi_cells_kernel  the cells holding two or more photons
-//     order_kernel        sorts each such cell's slot indices ascending: the result is the scatter in
-//                         slot order, independent of atomic arrival order (the reference's order
-//                         within a cell is unspecified)
-//     gather_kernel       sorted[i] = photons[order[i]] (64-byte records)
-//   grid build with ranks (the renderer's and the stage entry's path): count_rank (histogram + each
-//   slot's rank in atomic order), scan_lookback_list (single-pass scan + list of occupied cells),
-//   scatter_rank (start + rank, no atomics), then cell_gather: per occupied cell the slot order
-//   restored and the records copied in one pass.  Same counts, offsets and slot order either way.
+//   grid build            exact u32 counting sort of the slots by cell key: count_rank (histogram,
+//                         photon_count.wgsl:25-34, + each slot's rank in atomic order), scan_lookback_list
+//                         (single-pass exclusive scan into (start, count) pairs + list of occupied cells;
+//                         replaces the blocking read-back and host scan of lib.rs:956-1007), scatter_rank
+//                         (start + rank, photon_scatter.wgsl:61-71 without atomics), then cell_gather: per
+//                         occupied cell the slot order restored and the records copied in one pass.
+//   small grid build      the no-allocation entry's form, for up to 2^20 slots and 2^18 cells in 9 MB of
+//                         scratch: key and rank of a slot share a word, written by the pass that reads the
+//                         photons; the same scan; then the cells' slots sorted in place (a warp's registers
+//                         up to 256 photons, a block's bitmap beyond) and one flat copy.
+// Both leave the scatter in slot order, independent of atomic arrival order (the reference's order within a
+// cell is unspecified).
 #include <algorithm>
 #include <cstring>
 
@@ -357,50 +354,6 @@ __device__ __forceinline__ uint4 load_keys4(const uint32_t *__restrict__ keys, u
     return k;
 }
 
-// Histogram: one reduction per valid key (no return value, so the adds do not hold the warp; keys of
-// one warp rarely repeat, so merging lanes first costs more than it saves).
-__global__ void __launch_bounds__(256) count_kernel(const uint32_t *__restrict__ keys, uint64_t n,
-                                                    uint32_t *__restrict__ counts) {
-    // eight keys per thread and pass, both 16-byte loads issued before the reductions
-    const uint64_t stride = 8ull * gridDim.x * blockDim.x;
-    const uint64_t start = 4ull * (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x);
-    const uint64_t half = 4ull * gridDim.x * blockDim.x;
-    const uint64_t rounds = (n + stride - 1) / stride;
-    for (uint64_t r = 0; r < rounds; ++r) {
-        const uint4 a = load_keys4(keys, start + r * stride, n);
-        const uint4 b = load_keys4(keys, start + r * stride + half, n);
-        const uint32_t kk[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (kk[j] != kInvalidKey) atomicAdd(counts + kk[j], 1u);
-    }
-}
-
-// Slot indices to start[key] + cursor[key] (positions within a cell in atomic order; the order pass
-// restores slot order).
-__global__ void __launch_bounds__(256) scatter_kernel(const uint32_t *__restrict__ keys, uint64_t n,
-                                                      const uint2 *__restrict__ meta, uint32_t *__restrict__ cursor,
-                                                      uint32_t *__restrict__ order) {
-    // eight keys per thread and pass: loads, then all atomics and meta reads, then the stores
-    const uint64_t stride = 8ull * gridDim.x * blockDim.x;
-    const uint64_t start = 4ull * (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x);
-    const uint64_t half = 4ull * gridDim.x * blockDim.x;
-    const uint64_t rounds = (n + stride - 1) / stride;
-    for (uint64_t r = 0; r < rounds; ++r) {
-        const uint64_t s0 = start + r * stride, s1 = s0 + half;
-        const uint4 a = load_keys4(keys, s0, n);
-        const uint4 b = load_keys4(keys, s1, n);
-        const uint32_t kk[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        uint32_t pos[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (kk[j] != kInvalidKey) pos[j] = atomicAdd(cursor + kk[j], 1u) + __ldg(&meta[kk[j]].x);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (kk[j] != kInvalidKey) order[pos[j]] = (uint32_t)((j < 4 ? s0 : s1) + (j & 3));
-    }
-}
-
 // Exclusive scan of counts into meta, three phases over tiles of kScanTile cells.
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanItems = 8;
@@ -473,45 +426,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(uint32_t *p
     }
 }
 
-// Rescan each tile with its offset; writes (start, count) per cell.  Items are blocked per thread
-// (thread t owns cells t*8 .. t*8+7 of the tile, two 16-byte loads, four 16-byte stores) so the
-// in-thread sums stay in cell order.
-__global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t *__restrict__ counts, uint32_t n,
-                                                                  const uint32_t *__restrict__ partials,
-                                                                  uint2 *__restrict__ meta, bool vec) {
-    __shared__ uint32_t warp_sums[kScanThreads / 32];
-    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    if (vec && base + kScanItems <= n) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(counts + base));
-        const uint4 b = __ldg(reinterpret_cast<const uint4 *>(counts + base + 4));
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else {
-#pragma unroll
-        for (uint32_t i = 0; i < kScanItems; ++i) v[i] = base + i < n ? __ldg(counts + base + i) : 0u;
-    }
-    uint32_t local = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < kScanItems; ++i) local += v[i];
-    uint32_t ex = block_exclusive_scan(local, warp_sums, nullptr) + __ldg(partials + blockIdx.x);
-    uint32_t st[kScanItems];
-#pragma unroll
-    for (uint32_t i = 0; i < kScanItems; ++i) {
-        st[i] = ex;
-        ex += v[i];
-    }
-    if (vec && base + kScanItems <= n) {
-        uint4 *m4 = reinterpret_cast<uint4 *>(meta + base);
-#pragma unroll
-        for (uint32_t i = 0; i < kScanItems; i += 2) m4[i / 2] = make_uint4(st[i], v[i], st[i + 1], v[i + 1]);
-    } else {
-#pragma unroll
-        for (uint32_t i = 0; i < kScanItems; ++i)
-            if (base + i < n) meta[base + i] = make_uint2(st[i], v[i]);
-    }
-}
-
 // Ascending sort of one cell's slot indices.  Comparators always order (lower index, higher index)
 // (the "flip" bitonic network), so positions past `count` act as +infinity and are never touched.
 template <typename Seg>
@@ -546,7 +460,7 @@ __device__ __forceinline__ void warp_bitonic(Seg seg, uint32_t count, uint32_t l
 }
 
 constexpr uint32_t kOrderWarps = 8;
-constexpr uint32_t kOrderSmem = 1024;  // per-warp shared buffer (entries)
+constexpr uint32_t kCellRegsMax = 256;  // cells up to this size are sorted in registers
 
 // Ascending bitonic sort of 32 * R values held R per lane (value e = lane * R + r).  Exchanges at
 // distance j < R stay in the lane's registers; wider ones pair lanes lane ^ (j / R) by shuffle.
@@ -578,105 +492,6 @@ __device__ __forceinline__ void warp_sort_regs(uint32_t (&v)[R], uint32_t lane) 
                     }
                 }
             }
-        }
-    }
-}
-
-// Sorts the cell's `count` (<= 32 R) slot indices order[start ..], in place or (out != null) into out.
-template <int R>
-__device__ __forceinline__ void sort_cell_regs(uint32_t *__restrict__ order, uint32_t start, uint32_t count,
-                                               uint32_t lane, uint32_t *out = nullptr) {
-    uint32_t v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t e = lane * R + r;
-        v[r] = e < count ? order[start + e] : 0xFFFFFFFFu;
-    }
-    warp_sort_regs<R>(v, lane);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t e = lane * R + r;
-        if (e < count) {
-            if (out) out[e] = v[r];
-            else order[start + e] = v[r];
-        }
-    }
-}
-
-// Cells holding two or more photons, appended to `list` (two cells per 16-byte meta load).
-__global__ void __launch_bounds__(256) multi_cells_kernel(const uint2 *__restrict__ meta, uint32_t n_cells,
-                                                          uint32_t *__restrict__ list, uint32_t *__restrict__ n_list,
-                                                          bool vec) {
-    // four cells per thread and pass (two 16-byte meta loads in flight)
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n_quads = (n_cells + 3u) / 4u;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t rounds = (n_quads + stride - 1) / stride;
-    for (uint32_t r = 0; r < rounds; ++r) {
-        const uint32_t c0 = 4u * (r * stride + blockIdx.x * blockDim.x + threadIdx.x);
-        uint32_t cnt[4] = {0u, 0u, 0u, 0u};
-        if (vec && c0 + 3u < n_cells) {
-            const uint4 m0 = __ldg(reinterpret_cast<const uint4 *>(meta + c0));
-            const uint4 m1 = __ldg(reinterpret_cast<const uint4 *>(meta + c0 + 2u));
-            cnt[0] = m0.y;
-            cnt[1] = m0.w;
-            cnt[2] = m1.y;
-            cnt[3] = m1.w;
-        } else {
-#pragma unroll
-            for (uint32_t j = 0; j < 4u; ++j)
-                if (c0 + j < n_cells) cnt[j] = __ldg(&meta[c0 + j].y);
-        }
-        uint32_t masks[4], tot = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < 4u; ++j) {
-            masks[j] = __ballot_sync(0xFFFFFFFFu, cnt[j] > 1u);
-            tot += __popc(masks[j]);
-        }
-        if (tot == 0u) continue;
-        uint32_t base = 0;
-        if (lane == 0u) base = atomicAdd(n_list, tot);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        const uint32_t lt = lanemask_lt();
-#pragma unroll
-        for (uint32_t j = 0; j < 4u; ++j) {
-            if (cnt[j] > 1u) list[base + __popc(masks[j] & lt)] = c0 + j;
-            base += __popc(masks[j]);
-        }
-    }
-}
-
-// One warp per listed cell: the cell's slot indices (in atomic order after the scatter) sorted
-// ascending, so photons of a cell keep slot order, as a sequential scatter would leave them.
-__global__ void __launch_bounds__(kOrderWarps * 32) order_kernel(const uint2 *__restrict__ meta,
-                                                                  const uint32_t *__restrict__ list,
-                                                                  const uint32_t *__restrict__ n_list,
-                                                                  uint32_t *__restrict__ order) {
-    __shared__ uint32_t buf[kOrderWarps][kOrderSmem];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t warps_total = gridDim.x * kOrderWarps;
-    const uint32_t n = *n_list;
-    for (uint32_t li = blockIdx.x * kOrderWarps + w; li < n; li += warps_total) {
-        const uint2 m = __ldg(meta + __ldg(list + li));
-        const uint32_t start = m.x, count = m.y;
-        if (count <= 1u) continue;
-        if (count <= 32u) {
-            sort_cell_regs<1>(order, start, count, lane);
-        } else if (count <= 64u) {
-            sort_cell_regs<2>(order, start, count, lane);
-        } else if (count <= 128u) {
-            sort_cell_regs<4>(order, start, count, lane);
-        } else if (count <= 256u) {
-            sort_cell_regs<8>(order, start, count, lane);
-        } else if (count <= kOrderSmem) {
-            uint32_t *sb = buf[w];
-            for (uint32_t i = lane; i < count; i += 32) sb[i] = order[start + i];
-            __syncwarp();
-            warp_bitonic(sb, count, lane);
-            for (uint32_t i = lane; i < count; i += 32) order[start + i] = sb[i];
-            __syncwarp();
-        } else {
-            warp_bitonic(order + start, count, lane);
         }
     }
 }
@@ -718,13 +533,14 @@ __global__ void __launch_bounds__(256) photon_gather_kernel(const float4 *__rest
                                                             const uint32_t *__restrict__ total, uint64_t cap,
                                                             float4 *__restrict__ sorted,
                                                             float4 *__restrict__ sorted_pos, bool wide) {
-    const uint64_t n = min((uint64_t)__ldg(total), cap);
+    grid_dependency_wait();
+    const uint64_t n = min((uint64_t)*total, cap);
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += 2 * step) {
         const uint64_t i2 = i + step;
         const bool two = i2 < n;
-        const float4 *s0 = photons + 4ull * __ldg(order + i);
-        const float4 *s1 = photons + 4ull * __ldg(order + (two ? i2 : i));
+        const float4 *s0 = photons + 4ull * order[i];
+        const float4 *s1 = photons + 4ull * order[two ? i2 : i];
         if (wide) {
             Photon8 a, b;
             load_photon_wide(s0, a);
@@ -791,7 +607,9 @@ __global__ void __launch_bounds__(256) count_rank_kernel(const uint32_t *__restr
     }
 }
 
-// scan_apply plus the list of occupied cells (count >= 1), appended with one atomic per warp.
+// Rescan each tile with its offset: (start, count) per cell and the list of occupied cells (count >= 1),
+// appended with one atomic per warp.  Items are blocked per thread (thread t owns cells t*8 .. t*8+7 of the
+// tile, two 16-byte loads, four 16-byte stores) so the in-thread sums stay in cell order.
 __global__ void __launch_bounds__(kScanThreads) scan_apply_list_kernel(const uint32_t *__restrict__ counts, uint32_t n,
                                                                        const uint32_t *__restrict__ partials,
                                                                        uint2 *__restrict__ meta, bool vec,
@@ -875,10 +693,14 @@ __device__ __forceinline__ void load_counts8(const uint32_t *counts, uint32_t ba
     }
 }
 
-template <int CT>
+//
+// kSmall (the small grid build): the counts stay, meta may be aligned to 4 bytes only (hence its type; vec is false then), and
+// the cells that need sorting are listed instead: those of 2 .. kCellRegsMax photons from the front of `list`
+// (n_list[0] of them), those of more from its end (n_list[1]).
+template <int CT, bool kSmall>
 __global__ void __launch_bounds__(kScanThreads) scan_lookback_list_kernel(uint32_t *__restrict__ counts,
                                                                           uint32_t n, uint32_t *status,
-                                                                          uint32_t chunks, uint2 *__restrict__ meta,
+                                                                          uint32_t chunks, uint32_t *__restrict__ meta,
                                                                           bool vec, uint32_t *__restrict__ list,
                                                                           uint32_t *__restrict__ n_list,
                                                                           uint32_t *__restrict__ total_out) {
@@ -943,6 +765,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_lookback_list_kernel(uint32
         }
     }
     __syncthreads();
+    auto listed = [](uint32_t count) { return kSmall ? count - 2u <= kCellRegsMax - 2u : count != 0u; };
     uint32_t carry = s_prefix;
 #pragma unroll
     for (int t = 0; t < CT; ++t) {
@@ -951,7 +774,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_lookback_list_kernel(uint32
 #pragma unroll
         for (uint32_t i = 0; i < kScanItems; ++i) {
             local += v[t][i];
-            occ += v[t][i] ? 1u : 0u;
+            occ += listed(v[t][i]) ? 1u : 0u;
         }
         uint32_t tile_total = 0;
         uint32_t ex = block_exclusive_scan(local, warp_sums, &tile_total) + carry;
@@ -962,20 +785,23 @@ __global__ void __launch_bounds__(kScanThreads) scan_lookback_list_kernel(uint32
             st[i] = ex;
             ex += v[t][i];
         }
-        // (start, count) written; the counts are cleared for the next build (meta keeps them)
+        // (start, count) written; the counts are cleared for the next build (meta keeps them; not kSmall)
         if (vec && base + kScanItems <= n) {
-            uint4 *m4 = reinterpret_cast<uint4 *>(meta + base);
+            uint4 *m4 = reinterpret_cast<uint4 *>(meta + 2u * base);
 #pragma unroll
             for (uint32_t i = 0; i < kScanItems; i += 2)
                 m4[i / 2] = make_uint4(st[i], v[t][i], st[i + 1], v[t][i + 1]);
-            reinterpret_cast<uint4 *>(counts + base)[0] = make_uint4(0u, 0u, 0u, 0u);
-            reinterpret_cast<uint4 *>(counts + base)[1] = make_uint4(0u, 0u, 0u, 0u);
+            if (!kSmall) {
+                reinterpret_cast<uint4 *>(counts + base)[0] = make_uint4(0u, 0u, 0u, 0u);
+                reinterpret_cast<uint4 *>(counts + base)[1] = make_uint4(0u, 0u, 0u, 0u);
+            }
         } else {
 #pragma unroll
             for (uint32_t i = 0; i < kScanItems; ++i)
                 if (base + i < n) {
-                    meta[base + i] = make_uint2(st[i], v[t][i]);
-                    counts[base + i] = 0u;
+                    meta[2u * (base + i)] = st[i];
+                    meta[2u * (base + i) + 1u] = v[t][i];
+                    if (!kSmall) counts[base + i] = 0u;
                 }
         }
         // warp-exclusive offsets of the occupied cells, one atomic per warp
@@ -990,8 +816,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_lookback_list_kernel(uint32
         if (lane == 0u && warp_total) wbase = atomicAdd(n_list, warp_total);
         wbase = __shfl_sync(0xFFFFFFFFu, wbase, 0) + x - occ;
 #pragma unroll
-        for (uint32_t i = 0; i < kScanItems; ++i)
-            if (v[t][i]) list[wbase++] = base + i;
+        for (uint32_t i = 0; i < kScanItems; ++i) {
+            if (listed(v[t][i])) list[wbase++] = base + i;
+            if (kSmall && v[t][i] > kCellRegsMax) list[n - 1u - atomicAdd(n_list + 1, 1u)] = base + i;
+        }
         __syncthreads();  // warp_sums is reused by the next tile's scan
     }
 }
@@ -1094,8 +922,6 @@ __device__ __forceinline__ void sort_cell_to(const uint32_t *__restrict__ order,
     for (int r = 0; r < R; ++r) buf[lane * R + r] = v[r];
 }
 
-constexpr uint32_t kCellRegsMax = 256;  // cells up to this size are sorted in registers
-
 // Per-cell slot order fused with the photon gather: one warp per listed (occupied) cell sorts the
 // cell's slot indices ascending -- photons of a cell keep slot order, as a sequential scatter would
 // leave them -- and copies the cell's records into sorted order.  Cells of more than 256 photons are
@@ -1150,77 +976,234 @@ cudaError_t launch_grid_build(const GridBuffers &g, cudaStream_t st) {
     const bool vec = (reinterpret_cast<uintptr_t>(g.counts) % 16u) == 0u && (reinterpret_cast<uintptr_t>(g.meta) % 16u) == 0u;
     const bool wide = ((reinterpret_cast<uintptr_t>(g.photons) | reinterpret_cast<uintptr_t>(g.sorted)) % 32u) == 0u;
     const uint32_t tiles = (C + kScanTile - 1) / kScanTile;
-    if (g.rank) {
-        // One scan pass with decoupled look-back while every value fits its 30 bits, else the three
-        // phases.  Chunks of up to four tiles, about two chunks per SM; the look-back's chunk status
-        // words and ticket (scan_partials[0 .. chunks], chunks <= tiles) and the count of occupied cells
-        // (total[1]; the cells are listed in the cursor array, which this path does not otherwise need)
-        // are cleared by the count launch.  The counts are zero on entry: cleared when the renderer is
-        // created and by the scan of every build once it has turned them into (start, count).
-        const bool lookback = n && n < (uint64_t)kScanValMask;
-        const uint32_t want = (tiles + 2 * sm - 1) / (2 * sm);
-        const uint32_t ct = want <= 1u ? 1u : (want <= 2u ? 2u : 4u);
-        const uint32_t chunks = (tiles + ct - 1) / ct;
-        if (!lookback) {
-            if ((e = cudaMemsetAsync(g.counts, 0, (size_t)C * 4, st)) != cudaSuccess) return e;
-            if ((e = cudaMemsetAsync(g.total + 1, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-            if (n) count_rank_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, n, g.counts, g.rank, nullptr,
-                                                                                    0u, g.total + 1);
-            scan_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g.counts, C, g.scan_partials);
-            scan_partials_kernel<<<1, kScanThreads, 0, st>>>(g.scan_partials, tiles, g.total);
-            scan_apply_list_kernel<<<tiles, kScanThreads, 0, st>>>(g.counts, C, g.scan_partials, g.meta, vec, g.cursor,
-                                                                   g.total + 1);
-            if ((e = cudaMemsetAsync(g.counts, 0, (size_t)C * 4, st)) != cudaSuccess) return e;
-            if (n) {
-                scatter_rank_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, g.rank, n, g.meta, g.order);
-                cell_gather_kernel<<<grid_for((uint64_t)C * 32, kOrderWarps * 32, 4), kOrderWarps * 32, 0, st>>>(
-                    g.meta, g.cursor, g.total + 1, g.order, g.photons, g.sorted, g.sorted_pos, wide);
-            }
-            return cudaGetLastError();
-        }
-        count_rank_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, n, g.counts, g.rank, g.scan_partials,
-                                                                         chunks + 1, g.total + 1);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if (ct == 1u)
-            e = launch_dependent(scan_lookback_list_kernel<1>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
-                                 chunks, g.meta, vec, g.cursor, g.total + 1, g.total);
-        else if (ct == 2u)
-            e = launch_dependent(scan_lookback_list_kernel<2>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
-                                 chunks, g.meta, vec, g.cursor, g.total + 1, g.total);
-        else
-            e = launch_dependent(scan_lookback_list_kernel<4>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
-                                 chunks, g.meta, vec, g.cursor, g.total + 1, g.total);
-        if (e != cudaSuccess) return e;
-        if ((e = launch_dependent(scatter_rank_kernel, grid_for((n + 7) / 8, 256, 8), 256, 0, st, g.keys,
-                                  (const uint32_t *)g.rank, n, (const uint2 *)g.meta, g.order)) != cudaSuccess)
-            return e;
-        return launch_dependent(cell_gather_kernel, grid_for((uint64_t)C * 32, kOrderWarps * 32, 4), kOrderWarps * 32, 0, st,
-                                (const uint2 *)g.meta, (const uint32_t *)g.cursor, (const uint32_t *)(g.total + 1),
-                                g.order, g.photons, g.sorted, g.sorted_pos, wide);
-    }
-    if ((e = cudaMemsetAsync(g.counts, 0, (size_t)C * 4, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(g.cursor, 0, (size_t)C * 4, st)) != cudaSuccess) return e;
-    if (n) {
-        count_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, n, g.counts);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    scan_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g.counts, C, g.scan_partials);
-    scan_partials_kernel<<<1, kScanThreads, 0, st>>>(g.scan_partials, tiles, g.total);
-    scan_apply_kernel<<<tiles, kScanThreads, 0, st>>>(g.counts, C, g.scan_partials, g.meta, vec);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (n) {
-        scatter_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, n, g.meta, g.cursor, g.order);
-        // The cells to order are listed in the cursor array (the cursors are spent after the scatter);
-        // the list length is total[1].
+    // One scan pass with decoupled look-back while every value fits its 30 bits, else the three
+    // phases.  Chunks of up to four tiles, about two chunks per SM; the look-back's chunk status
+    // words and ticket (scan_partials[0 .. chunks], chunks <= tiles) and the count of occupied cells
+    // (total[1]; the cells are listed in the cursor array, which this path does not otherwise need)
+    // are cleared by the count launch.  The counts are zero on entry: cleared when the renderer is
+    // created and by the scan of every build once it has turned them into (start, count).
+    const bool lookback = n && n < (uint64_t)kScanValMask;
+    const uint32_t want = (tiles + 2 * sm - 1) / (2 * sm);
+    const uint32_t ct = want <= 1u ? 1u : (want <= 2u ? 2u : 4u);
+    const uint32_t chunks = (tiles + ct - 1) / ct;
+    if (!lookback) {
+        if ((e = cudaMemsetAsync(g.counts, 0, (size_t)C * 4, st)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(g.total + 1, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-        multi_cells_kernel<<<grid_for((C + 3) / 4, 256, 8), 256, 0, st>>>(g.meta, C, g.cursor, g.total + 1, vec);
-        order_kernel<<<grid_for((uint64_t)C * 32, kOrderWarps * 32, 8), kOrderWarps * 32, 0, st>>>(g.meta, g.cursor,
-                                                                                                g.total + 1, g.order);
-        photon_gather_kernel<<<grid_for((n + 1) / 2, 256, 8), 256, 0, st>>>(g.photons, g.order, g.total, n, g.sorted,
-                                                                              g.sorted_pos, wide);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (n) count_rank_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, n, g.counts, g.rank, nullptr,
+                                                                                0u, g.total + 1);
+        scan_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(g.counts, C, g.scan_partials);
+        scan_partials_kernel<<<1, kScanThreads, 0, st>>>(g.scan_partials, tiles, g.total);
+        scan_apply_list_kernel<<<tiles, kScanThreads, 0, st>>>(g.counts, C, g.scan_partials, g.meta, vec, g.cursor,
+                                                               g.total + 1);
+        if ((e = cudaMemsetAsync(g.counts, 0, (size_t)C * 4, st)) != cudaSuccess) return e;
+        if (n) {
+            scatter_rank_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, g.rank, n, g.meta, g.order);
+            cell_gather_kernel<<<grid_for((uint64_t)C * 32, kOrderWarps * 32, 4), kOrderWarps * 32, 0, st>>>(
+                g.meta, g.cursor, g.total + 1, g.order, g.photons, g.sorted, g.sorted_pos, wide);
+        }
+        return cudaGetLastError();
     }
-    return cudaSuccess;
+    count_rank_kernel<<<grid_for((n + 7) / 8, 256, 8), 256, 0, st>>>(g.keys, n, g.counts, g.rank, g.scan_partials,
+                                                                     chunks + 1, g.total + 1);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (ct == 1u)
+        e = launch_dependent(scan_lookback_list_kernel<1, false>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
+                             chunks, reinterpret_cast<uint32_t *>(g.meta), vec, g.cursor, g.total + 1, g.total);
+    else if (ct == 2u)
+        e = launch_dependent(scan_lookback_list_kernel<2, false>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
+                             chunks, reinterpret_cast<uint32_t *>(g.meta), vec, g.cursor, g.total + 1, g.total);
+    else
+        e = launch_dependent(scan_lookback_list_kernel<4, false>, chunks, kScanThreads, 0, st, g.counts, C, g.scan_partials,
+                             chunks, reinterpret_cast<uint32_t *>(g.meta), vec, g.cursor, g.total + 1, g.total);
+    if (e != cudaSuccess) return e;
+    if ((e = launch_dependent(scatter_rank_kernel, grid_for((n + 7) / 8, 256, 8), 256, 0, st, g.keys,
+                              (const uint32_t *)g.rank, n, (const uint2 *)g.meta, g.order)) != cudaSuccess)
+        return e;
+    return launch_dependent(cell_gather_kernel, grid_for((uint64_t)C * 32, kOrderWarps * 32, 4), kOrderWarps * 32, 0, st,
+                            (const uint2 *)g.meta, (const uint32_t *)g.cursor, (const uint32_t *)(g.total + 1),
+                            g.order, g.photons, g.sorted, g.sorted_pos, wide);
+}
+
+// ---- small grid build -------------------------------------------------------------------------------
+// Six launches, each a programmatic dependent of the one before; its bytes take 14 us at 1M slots, the rest is
+// the chain of dependent loads of each launch and, with few slots, the launches.  1,000,003 slots in 64^3 cells
+// 137 -> 63 us, in 8^3 1,707 -> 142, 70,000 in 64^3 57 -> 30, 5,000 in 8^3 44 -> 22, against keys, histogram,
+// three-phase scan, atomic scatter and one warp's sort per cell in nine launches and three memsets.
+// A slot's word: cell in the low 18 bits, rank in its cell in the high 14; all ones: no photon.  Ranks from
+// kSmallRankMax up are stored as that: such a slot takes its place from the cell's counter in the scatter.
+constexpr uint32_t kSmallCellBits = 18, kSmallRankMax = (1u << (32 - kSmallCellBits)) - 2u;
+static_assert(RT_NOALLOC_MAX_CELLS <= 1u << kSmallCellBits, "cells of the small grid build");
+
+// The counts, the scan's status words and total[0 .. 3] start at zero.
+__global__ void __launch_bounds__(256) small_clear_kernel(uint32_t *__restrict__ counts, uint32_t n_cells, bool vec,
+                                                          uint32_t *__restrict__ status, uint32_t n_status,
+                                                          uint32_t *__restrict__ total) {
+    grid_launch_dependents();
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n_status) status[t] = 0u;
+    if (t < 4u) total[t] = 0u;
+    const uint32_t c = 4u * t;
+    if (vec && c + 4u <= n_cells) {
+        *reinterpret_cast<uint4 *>(counts + c) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+        for (uint32_t i = c; i < min(c + 4u, n_cells); ++i) counts[i] = 0u;
+    }
+}
+
+// Keys, histogram and ranks in one pass over the photons (their first 32 bytes), four slots per thread.  The
+// photons are read while the counts are still being cleared.
+__global__ void __launch_bounds__(256) small_count_kernel(const float4 *__restrict__ photons, uint32_t n,
+                                                          const rt_grid_params gp, uint32_t *__restrict__ counts,
+                                                          uint32_t *__restrict__ words) {
+    grid_launch_dependents();
+    const uint32_t s0 = blockIdx.x * 1024u + threadIdx.x;
+    uint32_t key[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j) {
+        const uint32_t s = s0 + 256u * j;
+        key[j] = kInvalidKey;
+        if (s < n) key[j] = slot_key(gp, xyz(__ldg(photons + 4ull * s)), __ldg(&photons[4ull * s + 1].x));
+    }
+    grid_dependency_wait();
+    uint32_t rank[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j)
+        if (key[j] != kInvalidKey) rank[j] = atomicAdd(counts + key[j], 1u);
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j) {
+        const uint32_t s = s0 + 256u * j;
+        if (s < n) words[s] = key[j] == kInvalidKey ? kInvalidKey : key[j] | min(rank[j], kSmallRankMax) << kSmallCellBits;
+    }
+}
+
+// order[start[cell] + rank] = slot.  The slots without a rank fill the cell from its end, counting its counter
+// down (small_order_kernel restores it from meta).
+__global__ void __launch_bounds__(256) small_scatter_kernel(const uint32_t *__restrict__ words, uint32_t n,
+                                                            const uint32_t *__restrict__ meta, uint32_t *__restrict__ counts,
+                                                            uint32_t *__restrict__ order) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const uint32_t s0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    const uint4 a = load_keys4(words, s0, n);
+    const uint32_t word[4] = {a.x, a.y, a.z, a.w};
+    uint32_t pos[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (word[j] != kInvalidKey) {
+            const uint32_t cell = word[j] & ((1u << kSmallCellBits) - 1u);
+            uint32_t rank = word[j] >> kSmallCellBits;
+            if (rank == kSmallRankMax) rank = atomicSub(counts + cell, 1u) - 1u;
+            pos[j] = __ldg(meta + 2u * cell) + rank;
+        }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (word[j] != kInvalidKey) order[pos[j]] = s0 + (uint32_t)j;
+}
+
+// Cells of 2 .. kCellRegsMax photons, one warp each, sorted in registers in place.
+template <int R>
+__device__ __forceinline__ void sort_cell(uint32_t *__restrict__ order, uint32_t count, uint32_t lane) {
+    uint32_t v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t e = lane * R + r;
+        v[r] = e < count ? order[e] : 0xFFFFFFFFu;
+    }
+    warp_sort_regs<R>(v, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t e = lane * R + r;
+        if (e < count) order[e] = v[r];
+    }
+}
+
+// Every listed cell's slots in order.  Larger cells first, one block each: the cell's slots are marked in a
+// bitmap over all slots in shared memory and written back in order, so the time hardly depends on how many there
+// are (one warp's in-place sort took 26 us for 900 photons and grew with their square).  Thread t has the bitmap's
+// words [t << words_log2, (t + 1) << words_log2), laid out with an odd stride (no bank conflicts).
+constexpr uint32_t kSmallOrderThreads = 1024;
+__global__ void __launch_bounds__(kSmallOrderThreads) small_order_kernel(const uint32_t *__restrict__ meta,
+                                                                         const uint32_t *__restrict__ list, uint32_t n_cells,
+                                                                         const uint32_t *__restrict__ n_listed,
+                                                                         uint32_t *__restrict__ counts,
+                                                                         uint32_t *__restrict__ order, uint32_t words_log2) {
+    extern __shared__ uint32_t bitmap[];
+    __shared__ uint32_t s_sum[kSmallOrderThreads / 32];
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_small = n_listed[0], n_big = n_listed[1];
+    const uint32_t words = 1u << words_log2, stride = words | 1u;
+    uint32_t *mine = bitmap + threadIdx.x * stride;
+    for (uint32_t b = blockIdx.x; b < n_big; b += gridDim.x) {
+        const uint32_t cell = list[n_cells - 1u - b], start = meta[2u * cell], count = meta[2u * cell + 1u];
+        for (uint32_t k = 0; k < words; ++k) mine[k] = 0u;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < count; i += kSmallOrderThreads) {
+            const uint32_t slot = order[start + i], w = slot >> 5;
+            atomicOr(bitmap + (w >> words_log2) * stride + (w & (words - 1u)), 1u << (slot & 31u));
+        }
+        __syncthreads();
+        uint32_t own = 0u;
+        for (uint32_t k = 0; k < words; ++k) own += __popc(mine[k]);
+        uint32_t x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (lane == 31u) s_sum[warp] = x;
+        __syncthreads();
+        uint32_t to = start + x - own + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? s_sum[lane] : 0u);
+        if (own != 0u)
+            for (uint32_t k = 0; k < words; ++k)
+                for (uint32_t bits = mine[k], slot = 32u * (threadIdx.x * words + k); bits; bits &= bits - 1u)
+                    order[to++] = slot + (uint32_t)__ffs(bits) - 1u;
+        if (threadIdx.x == 0u) counts[cell] = count;
+        __syncthreads();
+    }
+    // (the blocks without a larger cell come first)
+    const uint32_t warps = gridDim.x * (kSmallOrderThreads / 32);
+    for (uint32_t li = (gridDim.x - 1u - blockIdx.x) + gridDim.x * warp; li < n_small; li += warps) {
+        const uint32_t cell = list[li], count = meta[2u * cell + 1u];
+        uint32_t *at = order + meta[2u * cell];
+        if (count <= 32u) sort_cell<1>(at, count, lane);
+        else if (count <= 64u) sort_cell<2>(at, count, lane);
+        else if (count <= 128u) sort_cell<4>(at, count, lane);
+        else sort_cell<8>(at, count, lane);
+    }
+}
+
+cudaError_t launch_small_grid(const SmallGrid &g, const rt_grid_params &gp, cudaStream_t st) {
+    const uint32_t C = gp.num_cells, n = (uint32_t)gp.photon_slots, sm = (uint32_t)num_sms();
+    const bool vec = (reinterpret_cast<uintptr_t>(g.counts) % 16u) == 0u && (reinterpret_cast<uintptr_t>(g.meta) % 16u) == 0u;
+    const bool wide = ((reinterpret_cast<uintptr_t>(g.photons) | reinterpret_cast<uintptr_t>(g.sorted)) % 32u) == 0u;
+    const uint32_t chunks = (C + kScanTile - 1) / kScanTile;  // at most 128: one tile per block
+    auto blocks = [](uint32_t items, uint32_t per_block) { return (items + per_block - 1u) / per_block; };
+    cudaError_t e;
+    small_clear_kernel<<<blocks(C, 1024u), 256, 0, st>>>(g.counts, C, vec, g.status, chunks + 1u, g.total);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (n && (e = launch_dependent(small_count_kernel, blocks(n, 1024u), 256u, 0, st, g.photons, n, gp, g.counts,
+                                   g.words)) != cudaSuccess)
+        return e;
+    if ((e = launch_dependent(scan_lookback_list_kernel<1, true>, chunks, kScanThreads, 0, st, g.counts, C, g.status, chunks,
+                              g.meta, vec, g.list, g.total + 1, g.total)) != cudaSuccess || !n)
+        return e;
+    if ((e = launch_dependent(small_scatter_kernel, blocks(n, 1024u), 256u, 0, st, g.words, n, g.meta, g.counts,
+                              g.order)) != cudaSuccess)
+        return e;
+    // One block per SM (its registers allow no more), with a bitmap of n slots if a cell may need it (at most 132 KB).
+    uint32_t words_log2 = 0u;
+    while ((32u * kSmallOrderThreads << words_log2) < n) ++words_log2;
+    const size_t bytes = n > kCellRegsMax ? kSmallOrderThreads * ((1u << words_log2) | 1u) * sizeof(uint32_t) : 0u;
+    if (bytes > 48u * 1024u && (e = cudaFuncSetAttribute(small_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)bytes)) != cudaSuccess)
+        return e;
+    const uint32_t order_blocks = std::max(blocks(n / 2u, kSmallOrderThreads / 32u), blocks(n, kCellRegsMax + 1u));
+    if ((e = launch_dependent(small_order_kernel, std::min(order_blocks, sm), kSmallOrderThreads, bytes, st, g.meta, g.list, C,
+                              g.total + 1, g.counts, g.order, words_log2)) != cudaSuccess)
+        return e;
+    return launch_dependent(photon_gather_kernel, std::min(blocks(blocks(n, 2u), 256u), sm * 8u), 256u, 0, st, g.photons,
+                            g.order, g.total, (uint64_t)n, g.sorted, (float4 *)nullptr, wide);
 }
 
 }  // namespace rtd

@@ -149,17 +149,27 @@ struct GridBuffers {
     float4 *sorted_pos;     // slot_count positions (the sorted photons' first float4), or null
     uint32_t *scan_partials;  // grid_scan_partials(num_cells) entries
     uint32_t *total;          // 4 entries: [0] binned photons, [1] listed cells
-    // Optional per-slot rank within its cell (null: count and an atomic scatter, then a pass that
-    // lists the multi-photon cells, a per-cell order pass and the gather).  With ranks the count pass
-    // records them, the scan lists the occupied cells, the scatter needs no atomics and one pass per
-    // occupied cell restores slot order and copies the records.
-    uint32_t *rank;
+    uint32_t *rank;           // slot_count: each slot's rank within its cell
 };
 uint32_t grid_scan_partials(uint32_t num_cells);
 cudaError_t launch_photon_keys(const float4 *photons, uint64_t slot_count, const rt_grid_params &gp, uint32_t *keys,
                                cudaStream_t st);
-// count -> scan -> scatter -> per-cell slot order -> photon gather.  counts/cursor are cleared here.
+// count with ranks -> scan -> scatter -> per-cell slot order and copy.
 cudaError_t launch_grid_build(const GridBuffers &g, cudaStream_t st);
+// The small grid build: at most RT_NOALLOC_MAX_SLOTS slots and RT_NOALLOC_MAX_CELLS cells.
+struct SmallGrid {
+    const float4 *photons;
+    uint32_t *counts;  // num_cells
+    uint32_t *meta;    // 2 num_cells: start and count per cell (4-byte aligned)
+    float4 *sorted;    // as many photons as are binned
+    // scratch
+    uint32_t *words;   // photon_slots
+    uint32_t *order;   // photon_slots
+    uint32_t *list;    // num_cells
+    uint32_t *status;  // grid_scan_partials(num_cells)
+    uint32_t *total;   // 4: binned photons, cells listed from the front, cells listed from the end
+};
+cudaError_t launch_small_grid(const SmallGrid &g, const rt_grid_params &gp, cudaStream_t st);
 
 // Image kernels.
 // alpha_dev, when not null, is read on the device in place of p.alpha (a CUDA graph replays the

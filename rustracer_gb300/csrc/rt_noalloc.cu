@@ -6,7 +6,7 @@
 // framework's pool that owns every byte the process may touch), and processes running close to the
 // memory limit, where an allocation could fail in the middle of a frame.  For them,
 // rt_stage_photon_grid_noalloc takes device pointers for its input and outputs and keeps its scratch
-// -- per-slot cell keys and slot order, per-cell cursors, the scan's tile sums and the binned total --
+// -- a word per slot, the slot order, the list of cells to sort, the scan's status words and the totals --
 // in one file-scope __device__ array of fixed size.  Every GPU that loads this library holds that
 // array (RT_NOALLOC_SCRATCH_BYTES, 9,438,208 bytes) until the process exits.
 #include <cuda_runtime.h>
@@ -19,12 +19,12 @@ using rt::set_error;
 namespace {
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-constexpr size_t kKeysOff = 0;
-constexpr size_t kOrderOff = align256(kKeysOff + 4 * (size_t)RT_NOALLOC_MAX_SLOTS);
-constexpr size_t kCursorOff = align256(kOrderOff + 4 * (size_t)RT_NOALLOC_MAX_SLOTS);
-constexpr size_t kPartialsOff = align256(kCursorOff + 4 * (size_t)RT_NOALLOC_MAX_CELLS);
-constexpr size_t kPartialsMax = RT_NOALLOC_MAX_CELLS / 2048 + 2;  // the scan's tile sums (+ grand total)
-constexpr size_t kTotalOff = align256(kPartialsOff + 4 * kPartialsMax);
+constexpr size_t kWordsOff = 0;
+constexpr size_t kOrderOff = align256(kWordsOff + 4 * (size_t)RT_NOALLOC_MAX_SLOTS);
+constexpr size_t kListOff = align256(kOrderOff + 4 * (size_t)RT_NOALLOC_MAX_SLOTS);
+constexpr size_t kStatusOff = align256(kListOff + 4 * (size_t)RT_NOALLOC_MAX_CELLS);
+constexpr size_t kStatusMax = RT_NOALLOC_MAX_CELLS / 2048 + 2;  // the scan's status words and ticket
+constexpr size_t kTotalOff = align256(kStatusOff + 4 * kStatusMax);
 constexpr size_t kScratchBytes = align256(kTotalOff + 16);
 static_assert(kScratchBytes <= RT_NOALLOC_SCRATCH_BYTES, "scratch layout exceeds the declared size");
 
@@ -53,8 +53,8 @@ extern "C" int rt_stage_photon_grid_noalloc(const rt_photon *d_photons, const rt
                   gp->photon_slots, gp->num_cells, (unsigned)RT_NOALLOC_MAX_SLOTS, (unsigned)RT_NOALLOC_MAX_CELLS);
         return RT_ERR_INVALID_ARGUMENT;
     }
-    if (rtd::grid_scan_partials(gp->num_cells) > kPartialsMax) {
-        set_error("rt_stage_photon_grid_noalloc: scan tile sums exceed the scratch layout");
+    if (rtd::grid_scan_partials(gp->num_cells) > kStatusMax) {
+        set_error("rt_stage_photon_grid_noalloc: scan status words exceed the scratch layout");
         return RT_ERR_INVALID_ARGUMENT;
     }
     int dev = 0;
@@ -75,23 +75,11 @@ extern "C" int rt_stage_photon_grid_noalloc(const rt_photon *d_photons, const rt
     }
     unsigned char *b = static_cast<unsigned char *>(base);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint32_t *keys = reinterpret_cast<uint32_t *>(b + kKeysOff);
-    rtd::GridBuffers g;
-    g.photons = reinterpret_cast<const float4 *>(d_photons);
-    g.keys = keys;
-    g.slot_count = gp->photon_slots;
-    g.num_cells = gp->num_cells;
-    g.counts = d_counts;  // cleared by the build (with the cursors); the scan totals are written whole
-    g.meta = reinterpret_cast<uint2 *>(d_meta);
-    g.cursor = reinterpret_cast<uint32_t *>(b + kCursorOff);
-    g.order = reinterpret_cast<uint32_t *>(b + kOrderOff);
-    g.sorted = reinterpret_cast<float4 *>(d_sorted);
-    g.sorted_pos = nullptr;
-    g.rank = nullptr;  // the scratch holds no rank array: count, atomic scatter, multi-photon cell pass
-    g.scan_partials = reinterpret_cast<uint32_t *>(b + kPartialsOff);
-    g.total = reinterpret_cast<uint32_t *>(b + kTotalOff);
-    if ((e = rtd::launch_photon_keys(g.photons, g.slot_count, *gp, keys, st)) != cudaSuccess ||
-        (e = rtd::launch_grid_build(g, st)) != cudaSuccess) {
+    auto words = [&](size_t off) { return reinterpret_cast<uint32_t *>(b + off); };
+    const rtd::SmallGrid g{reinterpret_cast<const float4 *>(d_photons), d_counts, d_meta,
+                           reinterpret_cast<float4 *>(d_sorted), words(kWordsOff), words(kOrderOff), words(kListOff),
+                           words(kStatusOff), words(kTotalOff)};
+    if ((e = rtd::launch_small_grid(g, *gp, st)) != cudaSuccess) {
         set_error("rt_stage_photon_grid_noalloc: launch failed: %s", cudaGetErrorString(e));
         return RT_ERR_CUDA;
     }
