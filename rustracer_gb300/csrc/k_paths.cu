@@ -26,7 +26,7 @@ constexpr uint32_t kPathsShare = 4;
 }  // namespace
 
 template <bool kMulti, bool kPhotons, bool kWhole>
-__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kernel(const __grid_constant__ WaveParams p,
+__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kernel(const __grid_constant__ WaveJob p,
                                                                                   uint32_t iter, uint32_t most) {
     extern __shared__ __align__(16) unsigned char trav_smem[];
     grid_dependency_wait();
@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
         uint32_t slot = 0u, jid = 0u;
         if (kWhole) {
             const uint32_t at = min(base + lane, n - 1u), gtile = at >> 5;
-            if (kMulti) jid = job_of(p, gtile, [](const DevJob &j) { return j.tile0; });
-            const DevJob &job = p.jobs[jid];
+            jid = job_of<kMulti>(p, gtile, [](const DevJob &j) { return j.tile0; });
+            const DevJob &job = job_at<kMulti>(p, jid);
             const uint32_t W = job.ip.width, tiles_x = (W + 7u) / 8u, tile = gtile - job.tile0;
             const uint32_t px = tile % tiles_x * 8u + (at & 7u), py = tile / tiles_x * 4u + (at >> 3 & 3u);
             alive = alive && px < W && py < job.ip.height;
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
             if (kMulti) jid = __float_as_uint(p.thr[slot].w);
         }
         const bool mine = alive;
-        const DevJob &job = p.jobs[jid];
+        const DevJob &job = job_at<kMulti>(p, jid);
         const DevScene &sc = job.scene;
         const float4 *records = kMulti ? sc.wnodes : p.records0, *tris = kMulti ? sc.tri_ord : p.tris0;
         const bool empty = kMulti ? sc.cnode_count == 0u : p.empty0 != 0u;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                                 continue;
                             const unsigned long long hit = w.best[lane];
                             if (occ) {
-                                clear = cut_out_lit(p.jobs[occ_job].scene, w.ro[lane], w.rd[lane], w.limit[lane], hit);
+                                clear = cut_out_lit(job_at<kMulti>(p, occ_job).scene, w.ro[lane], w.rd[lane], w.limit[lane], hit);
                             } else {
                                 hit_dist = hit_t(hit);
                                 hit_slot = (uint32_t)hit;
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                     prim = __float_as_uint(__ldg(tris + 3ull * hit_slot).w);
                     word = __float_as_uint(__ldg(tris + 3ull * hit_slot + 1).w);
                 }
-                out = shade_path<kPhotons, false>(p, slot, hit_dist, prim, word >> 2, lit);
+                out = shade_path<kPhotons, false, kMulti>(p, slot, hit_dist, prim, word >> 2, lit);
                 if (kPhotons && out.photon)
                     photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td, runs);
                 alive = out.keep;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
 }
 
 namespace {
-using PathsKernel = void (*)(const WaveParams, uint32_t, uint32_t);
+using PathsKernel = void (*)(const WaveJob, uint32_t, uint32_t);
 template <bool kWhole>
 PathsKernel paths_kernel(bool multi, bool photons) {
     if (multi) return photons ? wf_paths_kernel<true, true, kWhole> : wf_paths_kernel<true, false, kWhole>;
@@ -221,13 +221,13 @@ void prepare_paths_kernels() {
 // foliage 0.71 against 0.91; at 400 x 300 0.43 against 0.45; at 480 x 270 1.32 against 1.14.
 uint32_t paths_limit(int num_sms) { return (uint32_t)num_sms * kPathsBlocksPerSm * kPathsBlock; }
 
-cudaError_t launch_paths_frame(const WaveParams &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st) {
+cudaError_t launch_paths_frame(const WaveJob &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st) {
     const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
     paths_kernel<true>(multi, photons)<<<blocks, kPathsBlock, trav_smem_bytes(kPathsBlock, false), st>>>(p, 0u, 32u * tiles);
     return cudaGetLastError();
 }
 
-cudaError_t launch_paths_rest(const WaveParams &p, uint32_t iter, uint32_t most, bool multi, bool photons, bool early,
+cudaError_t launch_paths_rest(const WaveJob &p, uint32_t iter, uint32_t most, bool multi, bool photons, bool early,
                               int num_sms, cudaStream_t st) {
     const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
     return launch_dependent_if(early, paths_kernel<false>(multi, photons), blocks, kPathsBlock,

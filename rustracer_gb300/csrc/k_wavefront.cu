@@ -30,13 +30,14 @@ namespace rtd {
 // generate: 8 x 4 pixel tiles, one per warp, so the first queue is tile-coherent.  One launch over
 // every job's tiles (job j's start at its tile0).
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) wf_generate_kernel(const __grid_constant__ WaveParams p, uint32_t n_tiles) {
+template <bool kMulti>
+__global__ void __launch_bounds__(128) wf_generate_kernel(const __grid_constant__ WaveJob p, uint32_t n_tiles) {
     grid_launch_dependents();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t gtile = blockIdx.x * 4u + warp;
     if (gtile >= n_tiles) return;  // whole warps: warp_append below is warp-uniform
-    const uint32_t jid = job_of(p, gtile, [](const DevJob &j) { return j.tile0; });
-    const DevJob &job = p.jobs[jid];
+    const uint32_t jid = job_of<kMulti>(p, gtile, [](const DevJob &j) { return j.tile0; });
+    const DevJob &job = job_at<kMulti>(p, jid);
     const uint32_t W = job.ip.width, H = job.ip.height;
     const uint32_t tiles_x = (W + 7u) / 8u;
     const uint32_t tile = gtile - job.tile0;
@@ -66,7 +67,8 @@ constexpr uint32_t kShadeKeys = 5;  // miss, dielectric, Lambertian / emissive, 
 // The entry's order key; for a hit also its triangle and material word, read from the hit prim
 // slot's record (the traversal stores the slot: `orig` = the triangle's index, `word` = key | material
 // << 2, filled at scene upload).
-__device__ __forceinline__ uint32_t shade_key(const WaveParams &p, const uint32_t *q, uint32_t i, uint32_t n,
+template <bool kMulti>
+__device__ __forceinline__ uint32_t shade_key(const WaveJob &p, const uint32_t *q, uint32_t i, uint32_t n,
                                               uint32_t &slot, uint32_t &orig, uint32_t &word) {
     slot = 0u;
     orig = 0u;
@@ -75,7 +77,8 @@ __device__ __forceinline__ uint32_t shade_key(const WaveParams &p, const uint32_
     slot = q[i];
     const float2 h = p.hit[slot];
     if (h.x >= kInf) return 0u;
-    const float4 *rec = p.jobs[__float_as_uint(p.thr[slot].w)].scene.tri_ord + 3ull * __float_as_uint(h.y);
+    const float4 *tris = kMulti ? p.jobs[__float_as_uint(p.thr[slot].w)].scene.tri_ord : p.job0.scene.tri_ord;
+    const float4 *rec = tris + 3ull * __float_as_uint(h.y);
     orig = __float_as_uint(__ldg(rec).w);
     word = __float_as_uint(__ldg(rec + 1).w);
     return word & 3u;
@@ -85,8 +88,8 @@ __device__ __forceinline__ uint32_t shade_key(const WaveParams &p, const uint32_
 // registers with 62 bytes of spills; 6: 80 registers, ~200 bytes of spills, the default: the extra
 // warps hide the kernel's dependent loads, config-2 shade 7.04 -> 6.56 -> 6.41 ms per frame), chosen
 // per launch by the tuning's shade_blocks.
-template <bool kPhotons, bool kDebug, int kBlocks>
-__global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_constant__ WaveParams p, uint32_t iter,
+template <bool kPhotons, bool kDebug, bool kMulti, int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_constant__ WaveJob p, uint32_t iter,
                                                                uint32_t most) {
     __shared__ uint32_t s_count[4][kShadeKeys];  // entries per warp and key
     __shared__ uint32_t s_order[128];
@@ -112,7 +115,7 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         const uint32_t round_base = r * stride + blockIdx.x * blockDim.x;
         const uint32_t i_own = round_base + threadIdx.x;
         uint32_t slot_own, orig_own, word_own;
-        const uint32_t key = shade_key(p, q, i_own, n, slot_own, orig_own, word_own);
+        const uint32_t key = shade_key<kMulti>(p, q, i_own, n, slot_own, orig_own, word_own);
         uint32_t same = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kShadeKeys; ++k) {
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         uint32_t slot = 0;
         if (valid) {
             slot = q[i];
-            out = shade_path<kPhotons, kDebug>(p, slot, p.hit[slot].x, s_orig[threadIdx.x], s_word[threadIdx.x] >> 2, false);
+            out = shade_path<kPhotons, kDebug, kMulti>(p, slot, p.hit[slot].x, s_orig[threadIdx.x], s_word[threadIdx.x] >> 2, false);
         }
         // Queue positions by original order: each thread appends for the entry it keyed, then the
         // thread that shaded it writes its records there.
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         }
         if (kPhotons && out.photon) {
             float4 *rec = p.preq + 3ull * s_ppos[li];
-            const uint32_t jid = __float_as_uint(p.thr[slot].w);
+            const uint32_t jid = kMulti ? __float_as_uint(p.thr[slot].w) : 0u;
             rec[0] = make_float4(out.ph_hp.x, out.ph_hp.y, out.ph_hp.z, __uint_as_float(slot));
             rec[1] = make_float4(out.ph_n.x, out.ph_n.y, out.ph_n.z, __uint_as_float(out.ph_sidx));
             rec[2] = make_float4(out.ph_td.x, out.ph_td.y, out.ph_td.z, __uint_as_float(jid));
@@ -189,7 +192,8 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
 // divergent cell loops.  Runs after shade(iter) and before the occlusion rays of iter, so a pixel's
 // terms arrive in the order the inline lookup added them.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ WaveParams p, uint32_t iter) {
+template <bool kMulti>
+__global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ WaveJob p, uint32_t iter) {
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t n = p.counts[4 * iter + 3];
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ 
     const LookupRuns runs{mine, mine + 32u * kRunsA, 32u};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 r0 = p.preq[3ull * i], r1 = p.preq[3ull * i + 1], r2 = p.preq[3ull * i + 2];
-        photon_lookup(p, p.jobs[__float_as_uint(r2.w)], __float_as_uint(r0.w), __float_as_uint(r1.w), xyz(r0), xyz(r1),
+        photon_lookup(p, job_at<kMulti>(p, __float_as_uint(r2.w)), __float_as_uint(r0.w), __float_as_uint(r1.w), xyz(r0), xyz(r1),
                       xyz(r2), runs);
     }
 }
@@ -428,12 +432,13 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
 // ------------------------------------------------------------------------------------------------
 // finalize: one launch over every job's slots.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) wf_finalize_kernel(const __grid_constant__ WaveParams p, uint32_t n_slots) {
+template <bool kMulti>
+__global__ void __launch_bounds__(256) wf_finalize_kernel(const __grid_constant__ WaveJob p, uint32_t n_slots) {
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= n_slots) return;
-    finalize_slot(p, p.jobs[job_of(p, slot, [](const DevJob &j) { return j.base; })], slot);
+    finalize_slot(p, job_at<kMulti>(p, job_of<kMulti>(p, slot, [](const DevJob &j) { return j.base; })), slot);
 }
 
 // Segments (paths queued per iteration) and shadow rays of the pass, added to the 64-bit counters.
@@ -552,7 +557,9 @@ cudaError_t launch_extend(const WaveParams &params, uint32_t iter, uint64_t max_
 cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uint32_t n_jobs, uint32_t iters, int num_sms,
                              const WaveTuning &tune, cudaStream_t st, WaveProfile *prof) {
     cudaError_t e;
-    WaveParams p = params;
+    WaveJob p;
+    std::memset(&p, 0, sizeof(p));
+    static_cast<WaveParams &>(p) = params;
     uint64_t slots = 0;
     uint32_t stack_need = 0, wide_need = 0;
     bool wide = n_jobs > 0;  // four-wide records when every job's scene has them
@@ -567,6 +574,8 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         cut = cut || jobs[j].scene->any_hit_shadows == 0u;
     }
     if (n_jobs == 1u) set_scene0(p, *jobs[0].scene, wide);
+    const bool one = n_jobs == 1u && jobs[0].job != nullptr;  // the launches carry the job
+    if (one) p.job0 = *jobs[0].job;
     bool photons = false, debug = false;
     for (uint32_t j = 0; j < n_jobs; ++j) {
         photons = photons || jobs[j].photons != 0u;
@@ -579,9 +588,11 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     // a limit of half as many paths measures 18.9, 4.44, 1.50 and 0.81.  Both need the four-wide records, no
     // debug view and no per-launch profile.
     const uint32_t most = wide && !debug && !prof && !p.work ? paths_limit(num_sms) : 0u;
-    if (iters && slots <= most) return launch_paths_frame(p, (uint32_t)tiles, n_jobs > 1u, photons, num_sms, st);
+    if (iters && slots <= most) return launch_paths_frame(p, (uint32_t)tiles, !one, photons, num_sms, st);
     if ((e = cudaMemsetAsync(p.counts, 0, sizeof(uint32_t) * 4 * (size_t)(iters + 1), st)) != cudaSuccess) return e;
-    if (tiles) wf_generate_kernel<<<(unsigned)((tiles + 3u) / 4u), 128, 0, st>>>(p, (uint32_t)tiles);
+    if (tiles)
+        (one ? wf_generate_kernel<false> : wf_generate_kernel<true>)<<<(unsigned)((tiles + 3u) / 4u), 128, 0, st>>>(
+            p, (uint32_t)tiles);
     WaveTuning t = tune;
     normalize_tuning(t, wide ? wide_need : stack_need);
     const TraceKernel trc = trace_kernel(t, wide, p.work != nullptr, n_jobs > 1u, cut);
@@ -597,16 +608,18 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     // extend(0), shade(0), then per iteration one trace launch with the occlusion rays of the
     // iteration before and the closest-hit rays of this one, then its shade; the last occlusion rays
     // close the pass.
-    void (*shade)(const WaveParams, uint32_t, uint32_t);
-    if (t.shade_blocks == 6u)
-        shade = photons ? (debug ? wf_shade_kernel<true, true, 6> : wf_shade_kernel<true, false, 6>)
-                        : (debug ? wf_shade_kernel<false, true, 6> : wf_shade_kernel<false, false, 6>);
+    void (*shade)(const WaveJob, uint32_t, uint32_t);
+    if (one && !debug && t.shade_blocks == 6u)
+        shade = photons ? wf_shade_kernel<true, false, false, 6> : wf_shade_kernel<false, false, false, 6>;
+    else if (t.shade_blocks == 6u)
+        shade = photons ? (debug ? wf_shade_kernel<true, true, true, 6> : wf_shade_kernel<true, false, true, 6>)
+                        : (debug ? wf_shade_kernel<false, true, true, 6> : wf_shade_kernel<false, false, true, 6>);
     else if (t.shade_blocks == 5u)
-        shade = photons ? (debug ? wf_shade_kernel<true, true, 5> : wf_shade_kernel<true, false, 5>)
-                        : (debug ? wf_shade_kernel<false, true, 5> : wf_shade_kernel<false, false, 5>);
+        shade = photons ? (debug ? wf_shade_kernel<true, true, true, 5> : wf_shade_kernel<true, false, true, 5>)
+                        : (debug ? wf_shade_kernel<false, true, true, 5> : wf_shade_kernel<false, false, true, 5>);
     else
-        shade = photons ? (debug ? wf_shade_kernel<true, true, 4> : wf_shade_kernel<true, false, 4>)
-                        : (debug ? wf_shade_kernel<false, true, 4> : wf_shade_kernel<false, false, 4>);
+        shade = photons ? (debug ? wf_shade_kernel<true, true, true, 4> : wf_shade_kernel<true, false, true, 4>)
+                        : (debug ? wf_shade_kernel<false, true, true, 4> : wf_shade_kernel<false, false, true, 4>);
     // In a small pass each launch's blocks are scheduled while the one before drains (gather 1.05 against 1.10 ms
     // at 480 x 270, 0.56 against 0.59 at 640 x 360 with a photon map).  In a large one that keeps traversal and
     // shade on the same SMs and with them the traversal's split of L1 for both (19.2 against 18.3 ms on config 2,
@@ -619,7 +632,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     };
     for (uint32_t it = 0; it < iters; ++it) {
         mark(prof ? prof->trace_ev : nullptr, n_trc, 0);
-        if ((e = launch_dependent_if(early, trc, grid, t.block_threads, smem, st, p, it, it ? it - 1u : kNoIter, t.chunk,
+        if ((e = launch_dependent_if(early, trc, grid, t.block_threads, smem, st, static_cast<const WaveParams &>(p), it, it ? it - 1u : kNoIter, t.chunk,
                                   trace_steps(t))) != cudaSuccess)
             return e;
         mark(prof ? prof->trace_ev : nullptr, n_trc++, 1);
@@ -627,19 +640,19 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         uint32_t rest = 0u;
         if (most && it && (photons ? it % 2u == 1u && iters - it >= 2u : it % 3u == 0u && iters - it >= 3u)) {
             rest = most;
-            if ((e = launch_paths_rest(p, it, rest, n_jobs > 1u, photons, early, num_sms, st)) != cudaSuccess) return e;
+            if ((e = launch_paths_rest(p, it, rest, !one, photons, early, num_sms, st)) != cudaSuccess) return e;
         }
         if ((e = launch_dependent_if(early, shade, shade_grid, 128u, 0, st, p, it, rest)) != cudaSuccess) return e;
         mark(prof ? prof->shade_ev : nullptr, n_shd++, 1);
         if (photons) {
             mark(prof ? prof->photon_ev : nullptr, n_pho, 0);
-            if ((e = launch_dependent_if(early, wf_photon_kernel, photon_grid, 128u, 0, st, p, it)) != cudaSuccess) return e;
+            if ((e = launch_dependent_if(early, one ? wf_photon_kernel<false> : wf_photon_kernel<true>, photon_grid, 128u, 0, st, p, it)) != cudaSuccess) return e;
             mark(prof ? prof->photon_ev : nullptr, n_pho++, 1);
         }
     }
     if (iters) {
         mark(prof ? prof->trace_ev : nullptr, n_trc, 0);
-        if ((e = launch_dependent_if(early, trc, grid, t.block_threads, smem, st, p, kNoIter, iters - 1u, t.chunk, trace_steps(t))) !=
+        if ((e = launch_dependent_if(early, trc, grid, t.block_threads, smem, st, static_cast<const WaveParams &>(p), kNoIter, iters - 1u, t.chunk, trace_steps(t))) !=
             cudaSuccess)
             return e;
         mark(prof ? prof->trace_ev : nullptr, n_trc++, 1);
@@ -649,10 +662,10 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         prof->shade_launches = n_shd;
         prof->photon_launches = n_pho;
     }
-    if (slots && (e = launch_dependent_if(early, wf_finalize_kernel, (unsigned)((slots + 255u) / 256u), 256u, 0, st, p,
+    if (slots && (e = launch_dependent_if(early, one ? wf_finalize_kernel<false> : wf_finalize_kernel<true>, (unsigned)((slots + 255u) / 256u), 256u, 0, st, p,
                                        (uint32_t)slots)) != cudaSuccess)
         return e;
-    return launch_dependent_if(early, wf_count_kernel, 1u, 32u, 0, st, p, iters);
+    return launch_dependent_if(early, wf_count_kernel, 1u, 32u, 0, st, static_cast<const WaveParams &>(p), iters);
 }
 
 }  // namespace rtd

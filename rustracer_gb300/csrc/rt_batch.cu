@@ -116,7 +116,8 @@ std::vector<unsigned char> BatchEngine::signature(rt_renderer *const *rs, uint32
     return s;
 }
 
-int BatchEngine::enqueue(rt_renderer *const *rs, uint32_t n, uint32_t iters, const float *alpha, bool dev_alpha) {
+int BatchEngine::enqueue(rt_renderer *const *rs, uint32_t n, uint32_t iters, const float *alpha, bool dev_alpha,
+                         const rtd::DevJob *table) {
     std::vector<rtd::JobShape> shapes(n);
     for (uint32_t j = 0; j < n; ++j) {
         const rt_renderer *r = rs[j];
@@ -124,7 +125,8 @@ int BatchEngine::enqueue(rt_renderer *const *rs, uint32_t n, uint32_t iters, con
                                   r->scene.stack_cap, r->cfg.enable_photon_map ? 1u : 0u,
                                   r->cfg.debug_view != 0u ? 1u : 0u, r->scene.wnodes ? 1u : 0u,
                                   r->scene.wide_stack,
-                                  &r->scene};
+                                  &r->scene,
+                                  dev_alpha ? nullptr : table + j};  // (a captured frame reads the job table)
     }
     const rtd::WaveParams wp = path.params(jobs.device(), n, counters.as<unsigned long long>());
     RT_CK(rtd::launch_wavefront(wp, shapes.data(), n, iters, num_sms, tuning, stream));
@@ -191,7 +193,7 @@ int BatchEngine::frame(rt_renderer *const *rs, uint32_t n) {
             }
             cudaGraph_t g = nullptr;
             RT_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            int st = enqueue(rs, n, iters, alpha.data(), true);
+            int st = enqueue(rs, n, iters, alpha.data(), true, table.data());
             cudaError_t ce = cudaStreamEndCapture(stream, &g);
             if (st != RT_OK) {
                 if (g) cudaGraphDestroy(g);
@@ -209,7 +211,7 @@ int BatchEngine::frame(rt_renderer *const *rs, uint32_t n) {
         }
     }
     if (replay) RT_CK(cudaGraphLaunch(exec, stream));
-    else if (int st = enqueue(rs, n, iters, alpha.data(), false)) return st;
+    else if (int st = enqueue(rs, n, iters, alpha.data(), false, table.data())) return st;
     if (fe[1]) RT_CK(cudaEventRecord(fe[1], stream));
     // Later work on each member's own stream (read-backs, solo frames, destroy) waits for this frame.
     RT_CK(cudaEventRecord(done, stream));

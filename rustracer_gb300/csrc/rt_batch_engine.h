@@ -51,7 +51,8 @@ struct BatchEngine {
 
   private:
     std::vector<unsigned char> signature(rt_renderer *const *rs, uint32_t n, uint32_t iters) const;
-    int enqueue(rt_renderer *const *rs, uint32_t n, uint32_t iters, const float *alpha, bool dev_alpha);
+    int enqueue(rt_renderer *const *rs, uint32_t n, uint32_t iters, const float *alpha, bool dev_alpha,
+                const rtd::DevJob *table);
 };
 
 }  // namespace rt

@@ -213,8 +213,9 @@ __device__ __forceinline__ uint32_t pack_sb(uint32_t s, uint32_t b) { return (s 
 
 // The last job whose first index (`first` of DevJob: base slot or first tile) is at or below i; jobs
 // are laid out in order, so their first indices ascend.
-template <typename First>
+template <bool kMulti, typename First>
 __device__ __forceinline__ uint32_t job_of(const WaveParams &p, uint32_t i, First first) {
+    if (!kMulti) return 0u;
     uint32_t lo = 0u, hi = p.n_jobs;
     while (hi - lo > 1u) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -256,8 +257,8 @@ struct ShadeOut {
 // One loop body of gather.wgsl:299-537 for the path in `slot`, whose ray hit triangle `prim` at hit_t (a miss:
 // kInf); hmat: the hit's material, known before its triangle, or kNoMat.  lit: the light of the slot's
 // pending NEE term is visible (also if its word says so).
-template <bool kPhotons, bool kDebug>
-__device__ __forceinline__ ShadeOut shade_path(const WaveParams &p, uint32_t slot, float hit_t, uint32_t prim,
+template <bool kPhotons, bool kDebug, bool kMulti>
+__device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, float hit_t, uint32_t prim,
                                                uint32_t hmat, bool lit) {
     ShadeOut out;
     out.sh_o = out.sh_d = out.ph_hp = out.ph_n = out.ph_td = mk3(0.0f, 0.0f, 0.0f);
@@ -265,7 +266,7 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveParams &p, uint32_t slo
     out.ph_sidx = 0u;
     const float4 o4 = p.ro[slot], d4 = p.rd[slot], t4 = p.thr[slot];
     const uint32_t jid = __float_as_uint(t4.w);
-    const DevJob &job = p.jobs[jid];
+    const DevJob &job = job_at<kMulti>(p, jid);
     const DevScene &s = job.scene;
     const rt_image_params &ip = job.ip;
     const uint32_t W = ip.width;

@@ -666,7 +666,8 @@ extern "C" int rt_render_frame(rt_renderer *r) {
                                   c.debug_view != 0u ? 1u : 0u,
                                   r->scene.wnodes ? 1u : 0u,
                                   r->scene.wide_stack,
-                                  &r->scene};
+                                  &r->scene,
+                                  &job};
         if (r->prof_flags) {
             if (int st = rt::profiled_gather(r, wp, shape, iters)) return st;
         } else {
