@@ -38,9 +38,12 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     uint2 *top = reinterpret_cast<uint2 *>(trav_smem) + threadIdx.x;
     uint2 deep[kMaxStack - kTopStack];
     WarpTrav &w = reinterpret_cast<WarpTrav *>(trav_smem + sizeof(uint2) * kTopStack * kPathsBlock)[threadIdx.x >> 5];
-    // Between walks the warp's traversal state and stacks hold the photon lookups' runs.
-    const LookupRuns runs{reinterpret_cast<uint2 *>(&w) + lane, top, kPathsBlock};
-    static_assert(sizeof(WarpTrav) >= 32 * kRunsA * sizeof(uint2) && kTopStack >= kLookupCells - kRunsA, "lookup runs");
+    // Between walks the warp's traversal state holds the photon lookups' runs and hits.
+    constexpr uint32_t kRunsA = 5;
+    uint2 rest[kLookupCells - kRunsA];
+    const LookupRuns<kRunsA> runs{reinterpret_cast<uint2 *>(&w) + lane, rest};
+    uint32_t *hit_list = reinterpret_cast<uint32_t *>(runs.a - lane + 32u * kRunsA) + lane;
+    static_assert(sizeof(WarpTrav) >= 32 * (kRunsA * sizeof(uint2) + kHitList * sizeof(uint32_t)), "lookup state");
     const Treelet tree{nullptr, nullptr, 0u};
     LaneWalk r;
     r.busy = r.visiting = r.any_hit = r.careful = r.held = false;
@@ -182,7 +185,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                 }
                 out = shade_path<kPhotons, false, kMulti>(p, slot, hit_dist, prim, word >> 2, lit);
                 if (kPhotons && out.photon)
-                    photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td, runs);
+                    photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td, runs, hit_list);
                 alive = out.keep;
             }
             if (kPhotons) __syncwarp();

@@ -69,13 +69,15 @@ constexpr uint32_t kShadeKeys = 5;  // miss, dielectric, Lambertian / emissive, 
 // << 2, filled at scene upload).
 template <bool kMulti>
 __device__ __forceinline__ uint32_t shade_key(const WaveJob &p, const uint32_t *q, uint32_t i, uint32_t n,
-                                              uint32_t &slot, uint32_t &orig, uint32_t &word) {
+                                              uint32_t &slot, uint32_t &orig, uint32_t &word, float &t) {
+    t = kInf;
     slot = 0u;
     orig = 0u;
     word = 0u;
     if (i >= n) return 4u;
     slot = q[i];
     const float2 h = p.hit[slot];
+    t = h.x;
     if (h.x >= kInf) return 0u;
     const float4 *tris = kMulti ? p.jobs[__float_as_uint(p.thr[slot].w)].scene.tri_ord : p.job0.scene.tri_ord;
     const float4 *rec = tris + 3ull * __float_as_uint(h.y);
@@ -96,7 +98,8 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
     __shared__ uint8_t s_emit[128];   // by original position: 1 survives, 2 shadow ray, 4 photon lookup
     __shared__ uint32_t s_spos[128];  // by original position: shadow record index
     __shared__ uint32_t s_ppos[128];  // by original position: photon-lookup record index
-    __shared__ uint32_t s_orig[128], s_word[128];  // by shading position: the hit's triangle and material word
+    __shared__ uint32_t s_orig[128], s_word[128];
+    __shared__ float2 s_own[128];  // by shading position: the hit's triangle and material word
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t n = p.counts[4 * iter];
@@ -115,7 +118,8 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         const uint32_t round_base = r * stride + blockIdx.x * blockDim.x;
         const uint32_t i_own = round_base + threadIdx.x;
         uint32_t slot_own, orig_own, word_own;
-        const uint32_t key = shade_key<kMulti>(p, q, i_own, n, slot_own, orig_own, word_own);
+        float t_own;
+        const uint32_t key = shade_key<kMulti>(p, q, i_own, n, slot_own, orig_own, word_own, t_own);
         uint32_t same = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kShadeKeys; ++k) {
@@ -131,6 +135,7 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
             for (uint32_t w = 0; w < 4; ++w)
                 if (k < key || (k == key && w < warp)) pos += s_count[w][k];
         s_order[pos] = i_own;
+        s_own[pos] = make_float2(__uint_as_float(slot_own), t_own);
         s_orig[pos] = orig_own;
         s_word[pos] = word_own;
         __syncthreads();
@@ -139,8 +144,9 @@ __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_con
         ShadeOut out;
         uint32_t slot = 0;
         if (valid) {
-            slot = q[i];
-            out = shade_path<kPhotons, kDebug, kMulti>(p, slot, p.hit[slot].x, s_orig[threadIdx.x], s_word[threadIdx.x] >> 2, false);
+            const float2 own = s_own[threadIdx.x];
+            slot = __float_as_uint(own.x);
+            out = shade_path<kPhotons, kDebug, kMulti>(p, slot, own.y, s_orig[threadIdx.x], s_word[threadIdx.x] >> 2, false);
         }
         // Queue positions by original order: each thread appends for the entry it keyed, then the
         // thread that shaded it writes its records there.
@@ -197,13 +203,16 @@ __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ 
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t n = p.counts[4 * iter + 3];
-    __shared__ uint2 s_runs[4][kLookupCells * 32];
-    uint2 *mine = s_runs[threadIdx.x >> 5] + (threadIdx.x & 31u);
-    const LookupRuns runs{mine, mine + 32u * kRunsA, 32u};
+    constexpr uint32_t kRunsA = 10;
+    __shared__ uint2 s_runs[4][kRunsA * 32];
+    uint2 rest[kLookupCells - kRunsA];
+    __shared__ uint32_t s_hits[4][kHitList * 32];
+    const LookupRuns<kRunsA> runs{s_runs[threadIdx.x >> 5] + (threadIdx.x & 31u), rest};
+    uint32_t *hit_list = s_hits[threadIdx.x >> 5] + (threadIdx.x & 31u);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 r0 = p.preq[3ull * i], r1 = p.preq[3ull * i + 1], r2 = p.preq[3ull * i + 2];
         photon_lookup(p, job_at<kMulti>(p, __float_as_uint(r2.w)), __float_as_uint(r0.w), __float_as_uint(r1.w), xyz(r0), xyz(r1),
-                      xyz(r2), runs);
+                      xyz(r2), runs, hit_list);
     }
 }
 

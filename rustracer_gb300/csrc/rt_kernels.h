@@ -16,7 +16,7 @@ struct DevJob {
     rt_image_params ip;
     rt_grid_params gp;
     const float4 *sorted_photons;  // 4 x float4 per photon
-    const float4 *sorted_pos;      // position of each sorted photon (its first float4), 16 B apart
+    const float4 *sorted_pos;      // position of each sorted photon (its first float4), 16 B apart; at least two
     uint64_t sorted_count;
     const uint2 *grid_meta;        // (start, count) per cell
     uint32_t max_bounces, npix, base, spp;  // base: first path slot; spp = max(1, ip.spp)

@@ -496,15 +496,14 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
     return out;
 }
 
-// The photons a lookup may examine, as runs of the sorted array: at most one run per cell of the 27.  Lane l
-// of a warp keeps run i at a[32 i + l] for i < kRunsA, the rest at b[b_stride (i - kRunsA)].
-constexpr uint32_t kLookupCells = 27u, kRunsA = 16u;
+// The photons a lookup may examine, as runs of the sorted array: at most one run per cell of the 27, hardly ever
+// more than one per row of three.  A lane keeps run i at a[32 i] in shared memory for i < kRunsA, the others in b
+// (local memory).  Its list of hits that wait to be added: entry i at [32 i].
+constexpr uint32_t kLookupCells = 27u, kHitList = 24u, kMaxHits = 64u;
+template <uint32_t kRunsA>
 struct LookupRuns {
     uint2 *a, *b;
-    uint32_t b_stride;
-    __device__ __forceinline__ uint2 &operator[](uint32_t i) const {
-        return i < kRunsA ? a[32u * i] : b[b_stride * (i - kRunsA)];
-    }
+    __device__ __forceinline__ uint2 &operator[](uint32_t i) const { return i < kRunsA ? a[32u * i] : b[i - kRunsA]; }
 };
 
 // Squared distance along one axis from x to the photons of cell c: none lie nearer than its faces, less
@@ -524,12 +523,15 @@ __device__ __forceinline__ float cell_distance2(float x, float grid_min, float c
 // farther than the radius only use up the budget, neighbouring cells of a row merge.  With radius = cell / 2
 // on a surface, four of its nine occupied cells remain.  Then the runs are tested as one flat loop over
 // groups of eight photons, so a thread moves to its next run by itself.  Bound by the latency of the photon
-// loads (issue 35% busy), so a group's tests come before its hits: 1920 x 1080 at 4 spp, 2^20 photons in 128^3
-// cells, 3.19 ms of lookups per frame before (every cell tested, a hit's loads between the tests of a group of
-// four), 2.38 with the runs, 2.07 with the hits after the tests, 1.79 with groups of eight (sixteen: 1.76, and
-// slower for few lookups).
+// loads and by lanes that wait for the warp's longest lookup (11 of 32 active), so hits only go into a list of the
+// lane; the warp adds them, four loaded at a time, when a list is nearly full.  1920 x 1080 at 4 spp, 2^20 photons
+// in 128^3 cells, 3.19 ms of lookups per frame with every cell tested and a hit's loads between the tests, 2.38
+// with the runs, 1.79 with groups of eight.  Relight and frame, then a batch of twelve: 4.67 and 9.30 ms with the
+// 27 runs in shared memory, 4.51 and 9.15 with ten (its rest is L1) and positions loaded in pairs, 4.38 and 8.53
+// with the lists (16 long: 4.40 and 8.55; eight hits at a time 4.60 and 8.62, two 4.62 and 9.05).
+template <typename Runs>
 __device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob &job, uint32_t slot, uint32_t sidx, f3 hp,
-                                              f3 shn, f3 td, const LookupRuns &runs) {
+                                              f3 shn, f3 td, const Runs &runs, uint32_t *hit_list) {
     const rt_image_params &ip = job.ip;
     const rt_grid_params &gp = job.gp;
     const float radius = ip.photon_radius, r2max = radius * radius, cell = gp.cell_size;
@@ -586,45 +588,61 @@ __device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob 
     // Photon indices are u32 and clamped to the last sorted photon (the backend's rule for an
     // out-of-range index; the grid's ranges never leave the array).
     const uint32_t last = (uint32_t)job.sorted_count - 1u;
-    const float4 *posv = job.sorted_pos ? job.sorted_pos : job.sorted_photons;
-    const uint32_t pstride = job.sorted_pos ? 1u : 4u;
+    const float4 *posv = job.sorted_pos;
     f3 ph_sum = mk3(0.0f, 0.0f, 0.0f);
-    uint32_t ph_hits = 0u;
-    bool done = n_runs == 0u;
-    uint2 m = done ? make_uint2(0u, 0u) : runs[0];
-    for (uint32_t ri = 1u; !done;) {
-        if (m.y == 0u) {
-            if (ri >= n_runs) break;
-            m = runs[ri++];
-        }
-        // A group of eight photons: positions loaded together (from the compact position array when there
-        // is one) and tested, then the hits among them in order, up to the hit cap.
-        float4 pos[8];
+    uint32_t ph_hits = 0u, waiting = 0u;  // hits added, hits in the lane's list
+    auto add_hits = [&]() {
+        for (uint32_t k = 0u; k < waiting; k += 4u) {
+            float4 pw[4], inc[4];
 #pragma unroll
-        for (uint32_t j = 0; j < 8u; ++j) pos[j] = __ldg(posv + (size_t)min(m.x + j, last) * pstride);
-        const uint32_t group = min(m.y, 8u);
-        uint32_t hits = 0u;
+            for (uint32_t j = 0; j < 4u; ++j) {
+                const float4 *ph = job.sorted_photons + 4ull * hit_list[32u * min(k + j, waiting - 1u)];
+                pw[j] = __ldg(ph + 1);
+                inc[j] = __ldg(ph + 2);
+            }
 #pragma unroll
-        for (uint32_t j = 0; j < 8u; ++j) {
-            const f3 dd = xyz(pos[j]) - hp;
-            const float d2 = dot(dd, dd);
-            if (j < group && d2 < r2max) hits |= 1u << j;
+            for (uint32_t j = 0; j < 4u; ++j)
+                if (k + j < waiting) ph_sum = ph_sum + xyz(pw[j]) * fmaxf(dot(shn, -xyz(inc[j])), 0.0f);
         }
-        while (hits) {
-            const uint32_t j = __ffs(hits) - 1u;
-            hits &= hits - 1u;
-            const float4 *ph = job.sorted_photons + 4ull * min(m.x + j, last);
-            const f3 pw = xyz(__ldg(ph + 1));
-            const f3 inc = xyz(__ldg(ph + 2));
-            ph_sum = ph_sum + pw * fmaxf(dot(shn, -inc), 0.0f);
-            if (++ph_hits >= 64u) {
-                done = true;
-                break;
+        ph_hits += waiting;
+        waiting = 0u;
+    };
+    const uint32_t lanes = __activemask();
+    bool more = n_runs != 0u;
+    uint2 m = more ? runs[0] : make_uint2(0u, 0u);
+    uint32_t ri = 1u;
+    while (__any_sync(lanes, more)) {
+        if (more) {
+            // A group of up to eight photons: the four pairs of positions that hold the first are loaded together.
+            float4 pos[8];
+            const uint32_t first = m.x & ~1u, skip = m.x & 1u;
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; j += 2u) ldg32(posv + min(first + j, last & ~1u), pos[j], pos[j + 1]);
+            const uint32_t group = min(m.y, 8u - skip);
+            uint32_t hits = 0u;
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) {
+                const f3 dd = xyz(pos[j]) - hp;
+                const float d2 = dot(dd, dd);
+                if (d2 < r2max) hits |= 1u << j;
+            }
+            hits &= ((1u << group) - 1u) << skip;
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j)
+                if (hits >> j & 1u) hit_list[32u * waiting++] = min(first + j, last);
+            m.x += group;
+            m.y -= group;
+            if (ph_hits + waiting >= kMaxHits) {
+                waiting = kMaxHits - ph_hits;
+                more = false;
+            } else if (m.y == 0u) {
+                more = ri < n_runs;
+                if (more) m = runs[ri++];
             }
         }
-        m.x += group;
-        m.y -= group;
+        if (__any_sync(lanes, waiting > kHitList - 8u)) add_hits();
     }
+    add_hits();
     if (ph_hits > 0u)
         acc_add_term(p, slot, sidx, td * ph_sum * ip.photon_scale / (kPi * (float)ph_hits * ip.photon_radius * ip.photon_radius),
                      false);

@@ -146,6 +146,9 @@ int check_config(const rt_render_config *cfg, const char *fn) {
 uint64_t photon_slots_of(const rt_render_config &c) {
     return c.enable_photon_map ? std::max<uint64_t>((uint64_t)c.photon_count * RT_MAX_BOUNCES, 1) : 1;
 }
+// The lookups load positions in pairs (beyond one slot their number is even).
+uint64_t sorted_pos_bytes(uint64_t slots) { return std::max<uint64_t>(slots, 2) * 16; }
+static_assert(RT_MAX_BOUNCES % 2u == 0u, "photon slots come in pairs");
 
 // The renderer's own buffers on a resident scene (Renderer::new after the scene upload).
 int create_on(rt_resident_scene *res, const rt_render_config *cfg, rt_renderer **out) {
@@ -217,7 +220,7 @@ int create_on(rt_resident_scene *res, const rt_render_config *cfg, rt_renderer *
     r->cfg.photon_radius = radius;
     const uint64_t S = r->photon_slots, C = r->gp.num_cells;
     if (r->d_photons.alloc(S * 64) != cudaSuccess || r->d_sorted.alloc(S * 64) != cudaSuccess ||
-        r->d_sorted_pos.alloc(S * 16) != cudaSuccess || r->d_rank.alloc(S * 4) != cudaSuccess ||
+        r->d_sorted_pos.alloc(sorted_pos_bytes(S)) != cudaSuccess || r->d_rank.alloc(S * 4) != cudaSuccess ||
         r->d_keys.alloc(S * 4) != cudaSuccess || r->d_order.alloc(S * 4) != cudaSuccess ||
         r->d_counts.alloc(C * 4) != cudaSuccess || r->d_cursor.alloc(C * 4) != cudaSuccess ||
         r->d_meta.alloc(C * 8) != cudaSuccess ||
@@ -461,7 +464,7 @@ uint64_t renderer_create_bytes(const rt_render_config &c, uint64_t num_cells, ui
     // frame or photon rebuild).
     const uint64_t npix = (uint64_t)c.width * c.height;
     const uint64_t S = photon_slots_of(c);
-    return npix * (5 * 16 + 4) + S * (64 + 64 + 16 + 4 + 4 + 4) + num_cells * 16 +
+    return npix * (5 * 16 + 4) + S * (64 + 64 + 4 + 4 + 4) + sorted_pos_bytes(S) + num_cells * 16 +
            (uint64_t)rtd::grid_scan_partials((uint32_t)num_cells) * 4 + 16 + 64 +
            sizeof(rt_light) * std::max<uint64_t>(n_lights, 1);
 }
