@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
             if (kMulti) jid = __float_as_uint(p.thr[slot].w);
         }
         const bool mine = alive;
+        bool lookup = false;  // a photon lookup waits in the slot's record of preq
         const DevJob &job = job_at<kMulti>(p, jid);
         const DevScene &sc = job.scene;
         const float4 *records = kMulti ? sc.wnodes : p.records0, *tris = kMulti ? sc.tri_ord : p.tris0;
@@ -184,11 +185,27 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                     word = __float_as_uint(__ldg(tris + 3ull * hit_slot + 1).w);
                 }
                 out = shade_path<kPhotons, false, kMulti>(p, slot, hit_dist, prim, word >> 2, lit);
-                if (kPhotons && out.photon)
-                    photon_lookup(p, job, slot, out.ph_sidx, out.ph_hp, out.ph_n, out.ph_td, runs, hit_list);
+                if (kPhotons && out.photon) {
+                    float4 *req = p.preq + 3ull * slot;
+                    req[0] = make_float4(out.ph_hp.x, out.ph_hp.y, out.ph_hp.z, __uint_as_float(out.ph_sidx));
+                    req[1] = make_float4(out.ph_n.x, out.ph_n.y, out.ph_n.z, 0.0f);
+                    req[2] = make_float4(out.ph_td.x, out.ph_td.y, out.ph_td.z, 0.0f);
+                    lookup = true;
+                }
                 alive = out.keep;
             }
-            if (kPhotons) __syncwarp();
+            // A lookup's term comes before the next one added to its slot: the lookups wait until a lane that
+            // has one goes on, or no lane does, and run together (640 x 360 with a photon map, four frames: 2.15 ms
+            // with each lookup right after its shade step, 2.03 together).
+            if (kPhotons && (__any_sync(0xFFFFFFFFu, lookup && alive) || !__any_sync(0xFFFFFFFFu, alive))) {
+                if (lookup) {
+                    const float4 *req = p.preq + 3ull * slot;
+                    const float4 r0 = req[0], r1 = req[1], r2 = req[2];
+                    photon_lookup(p, job, slot, __float_as_uint(r0.w), xyz(r0), xyz(r1), xyz(r2), runs, hit_list);
+                    lookup = false;
+                }
+                __syncwarp();
+            }
         }
         if (kWhole && mine) finalize_slot(p, job, slot);
     }
