@@ -37,7 +37,8 @@ struct WaveParams {
     float4 *rd;        // direction, .w = sample index | segment index << 16
     float4 *thr;       // throughput, .w = job index
     float2 *hit;       // closest t, the hit's prim slot
-    float4 *acc;       // 4 per slot: (col, lum_sum), (lum2_sum, first_depth, -, -), sample_lum[0..8]
+    float4 *acc;       // 4 per slot: (col, lum_sum), (lum2_sum, first_depth, the current sample's luminance, -),
+                       // luminance of each ended sample [0..8]
     float4 *nrm;       // first-hit shading normal
     uint32_t *queue[2];
     uint32_t *counts;  // per iteration: [0] paths queued, [1] shadow rays, [2] trace cursor, [3] photon lookups
