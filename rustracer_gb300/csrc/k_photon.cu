@@ -102,7 +102,7 @@ __device__ bool photon_emit(const PhotonTraceParams &p, uint32_t photon_index, R
         float v = u2 * su;
         float w = 1.0f - u - v;
         origin = tri.v0 * u + tri.v1 * v + tri.v2 * w;
-        f3 n = triangle_normal(tri.v0, tri.v1, tri.v2);
+        f3 n = tri.gn;
         f3 local = sample_cosine_hemisphere(rng);
         dir = to_world(local, n);
         power = light.color * light.intensity;
@@ -138,7 +138,7 @@ __device__ bool photon_bounce(const PhotonTraceParams &p, uint32_t photon_index,
     Mat mat = load_mat(s, tri.material_id);
     f3 hit_pos = origin + dir * hit.t;
     Bary bb = barycentric(tri, origin, dir, hit.t);
-    f3 normal = triangle_normal(tri.v0, tri.v1, tri.v2);
+    f3 normal = tri.gn;
     bool front = dot(dir, normal) < 0.0f;
     f3 sn_geom = smooth_normal(tri, bb, normal);
     f3 face_normal = front ? sn_geom : -sn_geom;

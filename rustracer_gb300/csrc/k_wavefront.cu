@@ -26,6 +26,26 @@
 
 namespace rtd {
 
+__global__ void __launch_bounds__(256) triangle_terms_kernel(float4 *__restrict__ tris, uint64_t n) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float4 *p = tris + 8ull * i;
+    const f3 v0 = xyz(p[0]), v1 = xyz(p[1]), v2 = xyz(p[2]), e1 = v1 - v0, e2 = v2 - v0, gn = triangle_normal(v0, v1, v2);
+    const float d00 = dot(e1, e1), d01 = dot(e1, e2), d11 = dot(e2, e2);
+    p[0].w = gn.x;
+    p[1].w = gn.y;
+    p[2].w = gn.z;
+    p[3].w = d00;
+    p[4].w = d01;
+    p[5].w = d11;
+    p[7].w = d00 * d11 - d01 * d01;
+}
+
+cudaError_t launch_triangle_terms(float4 *tris, uint64_t n, cudaStream_t st) {
+    triangle_terms_kernel<<<(unsigned)((n + 255u) / 256u), 256, 0, st>>>(tris, n);
+    return cudaGetLastError();
+}
+
 // ------------------------------------------------------------------------------------------------
 // generate: 8 x 4 pixel tiles, one per warp, so the first queue is tile-coherent.  One launch over
 // every job's tiles (job j's start at its tile0).

@@ -190,16 +190,19 @@ struct DevScene {
 // Index clamped into [0, n) (n == 0 maps to element 0, which every scene array has).
 __device__ __forceinline__ uint32_t clampi_u(uint32_t i, uint32_t n) { return i < n ? i : (n ? n - 1u : 0u); }
 
+// A triangle's record on the device carries terms of its vertices in its spare words, filled at scene upload
+// (launch_triangle_terms): the geometric normal and the products barycentric() starts with.
 struct Tri {
-    f3 v0, v1, v2;
+    f3 v0, v1, v2, gn;
 };
 __device__ __forceinline__ Tri load_tri_verts(const DevScene &s, uint32_t i) {
     const float4 *p = s.tris + 8ull * clampi_u(i, s.tri_count);
     float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-    return Tri{xyz(a), xyz(b), xyz(c)};
+    return Tri{xyz(a), xyz(b), xyz(c), mk3(a.w, b.w, c.w)};
 }
 struct TriFull {
-    f3 v0, v1, v2, n0, n1, n2;
+    f3 v0, v1, v2, n0, n1, n2, gn;
+    float d00, d01, d11, denom;
     float uv0x, uv0y, uv1x, uv1y, uv2x, uv2y;
     uint32_t material_id;
 };
@@ -212,6 +215,8 @@ __device__ __forceinline__ TriFull load_tri(const DevScene &s, uint32_t i) {
     t.n0 = xyz(d); t.n1 = xyz(e); t.n2 = xyz(f);
     t.uv0x = g.x; t.uv0y = g.y; t.uv1x = g.z; t.uv1y = g.w; t.uv2x = h.x; t.uv2y = h.y;
     t.material_id = __float_as_uint(h.z);
+    t.gn = mk3(a.w, b.w, c.w);
+    t.d00 = d.w; t.d01 = e.w; t.d11 = f.w; t.denom = h.w;
     return t;
 }
 struct Mat {
@@ -320,13 +325,11 @@ __device__ __forceinline__ Bary barycentric(const TriFull &tri, f3 ro, f3 rd, fl
     f3 e1 = tri.v1 - tri.v0;
     f3 e2 = tri.v2 - tri.v0;
     f3 p = ro + rd * t - tri.v0;
-    float d00 = dot(e1, e1), d01 = dot(e1, e2), d11 = dot(e2, e2);
     float d20 = dot(p, e1), d21 = dot(p, e2);
-    float denom = d00 * d11 - d01 * d01;
     float u = 0.0f, v = 0.0f;
-    if (denom != 0.0f) {
-        u = (d11 * d20 - d01 * d21) / denom;
-        v = (d00 * d21 - d01 * d20) / denom;
+    if (tri.denom != 0.0f) {
+        u = (tri.d11 * d20 - tri.d01 * d21) / tri.denom;
+        v = (tri.d00 * d21 - tri.d01 * d20) / tri.denom;
     }
     float w = 1.0f - u - v;
     return Bary{tri.uv0x * w + tri.uv1x * u + tri.uv2x * v, tri.uv0y * w + tri.uv1y * u + tri.uv2y * v, u, v};

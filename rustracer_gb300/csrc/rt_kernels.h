@@ -115,6 +115,8 @@ cudaError_t launch_paths_rest(const WaveJob &p, uint32_t iter, uint32_t most, bo
                               int num_sms, cudaStream_t st);
 void prepare_paths_kernels();
 int device_sm_count();
+// Fills the spare words of n uploaded triangle records (see load_tri).
+cudaError_t launch_triangle_terms(float4 *tris, uint64_t n, cudaStream_t st);
 // One-time kernel attributes (shared-memory opt-ins); call before capturing launches into a graph.
 void prepare_kernels();
 void prepare_wavefront_kernels();

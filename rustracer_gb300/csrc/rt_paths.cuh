@@ -95,22 +95,33 @@ __device__ __forceinline__ f3 spec_ggx(f3 wo, f3 n, f3 wi, float a, f3 f0) {
     f3 F = fresnel_schlick(fmaxf(dot(wo, h), 0.0f), f0);
     return F * (D * smith_g1(ndl, a) * smith_g1(ndv, a) / (4.0f * ndl * ndv));
 }
-__device__ __forceinline__ f3 sample_spec_dir(f3 rd, f3 n, float a, Rng &rng) {
-    f3 up = fabsf(n.y) < 0.999f ? mk3(0.0f, 1.0f, 0.0f) : mk3(1.0f, 0.0f, 0.0f);
-    f3 bt = normalize(cross(up, n));
-    f3 bb = cross(n, bt);
+// What the two lobes' direction samples have in common: the frame around n, the two random numbers, one's
+// square root (r; w: the square root of its complement) and the other's angle.
+struct DirSample {
+    f3 t, b;
+    float r, w, sp, cp;
+};
+__device__ __forceinline__ DirSample dir_sample(f3 n, bool spec, Rng &rng) {
+    DirSample d;
+    const f3 up = fabsf(n.y) < 0.999f ? mk3(0.0f, 1.0f, 0.0f) : mk3(1.0f, 0.0f, 0.0f);
+    d.t = normalize(cross(up, n));
+    d.b = cross(n, d.t);
+    const float u1 = rng_f32(rng), u2 = rng_f32(rng);
+    d.r = sqrtf(spec ? u1 : u2);
+    d.w = sqrtf(1.0f - (spec ? u1 : u2));
+    sincos_fixed(2.0f * kPi * (spec ? u2 : u1), d.sp, d.cp);
+    return d;
+}
+__device__ __forceinline__ f3 sample_spec_dir(f3 rd, f3 n, float a, const DirSample &d) {
+    const f3 bt = d.t, bb = d.b;
     f3 mrd = -rd;
     f3 v = mk3(dot(bt, mrd), dot(bb, mrd), dot(n, mrd));
     f3 vh = normalize(mk3(a * v.x, a * v.y, fmaxf(v.z, 1e-4f)));
     float l2 = vh.x * vh.x + vh.y * vh.y;
     f3 t1 = l2 > 0.0f ? mk3(-vh.y, vh.x, 0.0f) * (1.0f / sqrtf(l2)) : mk3(1.0f, 0.0f, 0.0f);
     f3 t2 = cross(vh, t1);
-    float r = sqrtf(rng_f32(rng));
-    float phi = 2.0f * kPi * rng_f32(rng);
-    float sp, cp;
-    sincos_fixed(phi, sp, cp);
-    float x = r * cp;
-    float y = r * sp;
+    float x = d.r * d.cp;
+    float y = d.r * d.sp;
     float s = 0.5f * (1.0f + vh.z);
     float yy = (1.0f - s) * sqrtf(fmaxf(0.0f, 1.0f - x * x)) + s * y;
     f3 hh = x * t1 + yy * t2 + sqrtf(fmaxf(0.0f, 1.0f - x * x - yy * yy)) * vh;
@@ -183,8 +194,7 @@ __device__ __forceinline__ LightSample light_sample(const DevJob &job, f3 hp, f3
         ls.wi = ld;
         float ndl = dot(sn, ld);
         if (ndl <= 0.0f) return ls;
-        f3 ln = triangle_normal(tri.v0, tri.v1, tri.v2);
-        float ndl_l = dot(ln, -ld);
+        float ndl_l = dot(tri.gn, -ld);
         if (ndl_l <= 0.0f) return ls;
         float area = 0.5f * len3(cross(tri.v1 - tri.v0, tri.v2 - tri.v0));
         ls.e = le * l.intensity * ndl * ndl_l * area * fn / (r2 + 0.01f);
@@ -274,7 +284,6 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
     const f3 env_color = mk3(s.env_color[0], s.env_color[1], s.env_color[2]);
     const f3 env_horizon = mk3(s.env_horizon[0], s.env_horizon[1], s.env_horizon[2]);
     const uint32_t pix = slot - job.base;
-    const uint32_t px = pix % W, py = pix / W;
     f3 ro = xyz(o4), rd = xyz(d4), thr = xyz(t4);
     Rng rng{__float_as_uint(o4.w)};
     const uint32_t sb = __float_as_uint(d4.w);
@@ -309,7 +318,7 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
             done_step = true;
         }
         if (!done_step) {
-            const f3 gn = triangle_normal(tr.v0, tr.v1, tr.v2);
+            const f3 gn = tr.gn;
             const bool ff = dot(rd, gn) < 0.0f;
             const f3 sn_geom = smooth_normal(tr, bb, gn);
             const f3 sn = ff ? sn_geom : -sn_geom;
@@ -356,7 +365,7 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
                     case 5: A.col = emis; break;
                     case 8:
                     case 9: {
-                        float pu = (float)px / (float)ip.width, pv = (float)py / (float)ip.height;
+                        float pu = (float)(pix % W) / (float)ip.width, pv = (float)(pix / W) / (float)ip.height;
                         float4 t =
                             tex_sample(s.tex[debug_view == 8 ? RT_TEX_EMISSIVE : RT_TEX_ALBEDO], pu, pv, 0);
                         A.col = mk3(t.x, t.y, t.z);
@@ -417,15 +426,16 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
                 f3 dscale = diffuse_weight / (1.0f - spec_prob);
 
                 LightSample ls = light_sample(job, hp, shn, rng);
-                f3 c_nee;
+                // (What both lobes compute alike stands outside the branches: most warps have paths of both.)
+                f3 lobe = dscale;
                 if (!do_spec) {
                     if (env_intensity > 0.0f)
                         add_radiance(A, thr * dscale * sky_color(shn, env_color, env_horizon, env_intensity));
-                    c_nee = thr * dscale * ls.e / kPi;
                     add_radiance(A, thr * albedo * ip.ambient);
                 } else {
-                    c_nee = thr * spec_ggx(wo, shn, ls.wi, a, f0) * ls.e / spec_prob;
+                    lobe = spec_ggx(wo, shn, ls.wi, a, f0);
                 }
+                const f3 c_nee = thr * lobe * ls.e / (do_spec ? spec_prob : kPi);
                 bool nee_luma_only = false;
                 if (kPhotons && ip.use_photons == 1u && !do_spec) {  // gather.wgsl:473-514
                     // The lookup runs in wf_photon_kernel right after this pass; its term
@@ -448,16 +458,15 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
                                               __uint_as_float((sidx & 0xFFFFu) | kNeePending |
                                                               (nee_luma_only ? kNeeLumaOnly : 0u)));
                 }
+                const DirSample ds = dir_sample(shn, do_spec, rng);
+                ro = hp + shn * 0.001f;
                 if (do_spec) {
-                    rd = sample_spec_dir(rd, shn, a, rng);
-                    ro = hp + shn * 0.001f;
+                    rd = sample_spec_dir(rd, shn, a, ds);
                     f3 h = normalize(wo + rd);
                     float ndl = fmaxf(dot(shn, rd), 0.0f);
                     thr = thr * fresnel_schlick(fmaxf(dot(wo, h), 0.0f), f0) * smith_g1(ndl, a) / spec_prob;
                 } else {
-                    f3 local = sample_cosine_hemisphere(rng);
-                    rd = to_world(local, shn);
-                    ro = hp + shn * 0.001f;
+                    rd = ds.t * (ds.cp * ds.w) + shn * ds.r + ds.b * (ds.sp * ds.w);
                     thr = thr * dscale;
                     if (kPhotons && ip.use_photons == 1u) alive = false;
                 }
@@ -475,7 +484,7 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveJob &p, uint32_t slot, 
     if (!alive) {
         sidx += 1u;
         if (sidx < spp) {
-            camera_ray(job, px, py, rng, ro, rd);
+            camera_ray(job, pix % W, pix / W, rng, ro, rd);
             thr = mk3(1.0f, 1.0f, 1.0f);
             b = 0u;
             out.keep = true;

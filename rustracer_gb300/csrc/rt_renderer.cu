@@ -363,6 +363,10 @@ int resident_scene_create(const rt_scene_desc *sd, rt_resident_scene **out) {
     int st;
     // Scene upload (Renderer::new, lib.rs:234-266).
     if ((st = upload(res->d_tris, sd->triangles, sd->triangle_count, s)) != RT_OK) return fail(st);
+    if (rtd::launch_triangle_terms(res->d_tris.as<float4>(), std::max<uint64_t>(sd->triangle_count, 1), s) != cudaSuccess) {
+        set_error("rt_resident_scene_create: kernel launch failed");
+        return fail(RT_ERR_CUDA);
+    }
     rt::TraversalLayout lay;
     if (!rt::build_traversal_layout(sd->bvh_nodes, sd->bvh_node_count, sd->bvh_prims, sd->bvh_prim_count,
                                     sd->triangles, sd->triangle_count, lay))
