@@ -568,6 +568,16 @@ void set_scene0(WaveParams &p, const DevScene &scene, bool wide) {
 }
 }  // namespace
 
+bool one_job_reads_table(const JobShape &shape, const WaveTuning &tune, bool profiled) {
+    WaveTuning t = tune;
+    normalize_tuning(t, 0u);
+    return profiled || shape.wide == 0u || shape.debug != 0u || shape.scene->any_hit_shadows == 0u || t.treelet != 0u ||
+           t.shade_blocks != 6u;
+}
+bool photon_pass_reads_table(const DevScene &scene, const WaveTuning &tune) {
+    return scene.wnodes == nullptr || tune.treelet != 0u;
+}
+
 cudaError_t launch_extend(const WaveParams &params, uint32_t iter, uint64_t max_items, const DevScene &scene, int num_sms,
                           const WaveTuning &tune, cudaStream_t st) {
     const bool wide = scene.wnodes != nullptr;

@@ -106,6 +106,13 @@ struct WaveProfile {
 // generate (per job), iters x (extend, shade, shadow) over all jobs, finalize (per job), counters.
 cudaError_t launch_wavefront(const WaveParams &p, const JobShape *jobs, uint32_t n_jobs, uint32_t iters, int num_sms,
                              const WaveTuning &tune, cudaStream_t st, WaveProfile *prof = nullptr);
+// Whether the kernels of a pass over one job that its launches carry (launch_wavefront with shape.job), or of a
+// photon pass (launch_photon_wave), read the job table all the same: the two-wide, treelet and profiling
+// traversals, debug views, other shade variants than the default, and the alpha rule of cut-out scenes do.  Else
+// the caller need not upload it, which takes a copy and its gap out of every frame (16 frames of
+// 256 x 256 2.39 -> 2.25 ms).
+bool one_job_reads_table(const JobShape &shape, const WaveTuning &tune, bool profiled);
+bool photon_pass_reads_table(const DevScene &scene, const WaveTuning &tune);
 // The gather pass of few paths in one launch (k_paths.cu): a whole frame of at most paths_limit pixels in
 // `tiles` 8 x 4 tiles, or, if at most `most` paths are queued for iteration `iter` (traced, not yet shaded),
 // the rest of theirs (early: as a programmatic dependent).

@@ -658,11 +658,20 @@ extern "C" int rt_render_frame(rt_renderer *r) {
         }
         cudaEvent_t fe[4] = {nullptr, nullptr, nullptr, nullptr};
         for (auto &e : fe) RT_CK(r->ring.next(&e));
-        RT_CK(cudaEventRecord(r->events.ev[EV_FRAME0], s));
-        if (fe[3]) RT_CK(cudaEventRecord(fe[0], s));
+        if (!fe[3]) {  // no more events in the ring
+            fe[0] = r->events.ev[EV_FRAME0];
+            fe[1] = r->events.ev[EV_GATHER1];
+            fe[2] = r->events.ev[EV_DENOISE1];
+            fe[3] = r->events.ev[EV_RESOLVE1];
+        } else {
+            r->ring_denoised.resize(r->ring.used / 4, c.enable_denoise != 0);
+        }
+        // (an event record takes 2 us of the stream; a frame without denoise has three)
+        if (!c.enable_denoise) fe[2] = fe[1];
+        for (int i = 0; i < 4; ++i) r->frame_ev[i] = fe[i];
+        RT_CK(cudaEventRecord(fe[0], s));
         const rtd::DevJob job = rt::make_job(r, 0u);
         if (int st = rt::ensure_job_table(r)) return st;
-        RT_CK(r->jobs.upload(&job, 1, s));
         const rtd::WaveParams wp = r->path.params(r->jobs.device(), 1u, r->d_counters.as<unsigned long long>());
         const rtd::JobShape shape{c.width,
                                   c.height,
@@ -675,20 +684,18 @@ extern "C" int rt_render_frame(rt_renderer *r) {
                                   r->scene.wide_stack,
                                   &r->scene,
                                   &job};
+        if (rtd::one_job_reads_table(shape, r->tuning, r->prof_flags != 0u)) RT_CK(r->jobs.upload(&job, 1, s));
         if (r->prof_flags) {
             if (int st = rt::profiled_gather(r, wp, shape, iters)) return st;
         } else {
             RT_CK(rtd::launch_wavefront(wp, &shape, 1u, iters, r->num_sms, r->tuning, s));
         }
-        RT_CK(cudaEventRecord(r->events.ev[EV_GATHER1], s));
-        if (fe[3]) RT_CK(cudaEventRecord(fe[1], s));
+        RT_CK(cudaEventRecord(fe[1], s));
         float4 *result = nullptr;
         if (int st = rt::enqueue_denoise(r, alpha, nullptr, s, &result)) return st;
-        RT_CK(cudaEventRecord(r->events.ev[EV_DENOISE1], s));
-        if (fe[3]) RT_CK(cudaEventRecord(fe[2], s));
+        if (fe[2] != fe[1]) RT_CK(cudaEventRecord(fe[2], s));
         if (int st = rt::enqueue_resolve(r, result, alpha, nullptr, s)) return st;
-        RT_CK(cudaEventRecord(r->events.ev[EV_RESOLVE1], s));
-        if (fe[3]) RT_CK(cudaEventRecord(fe[3], s));
+        RT_CK(cudaEventRecord(fe[3], s));
         r->frames += 1;
         r->have_frame_timing = true;
         return RT_OK;
@@ -897,9 +904,11 @@ int rt::enqueue_photon_rebuild(rt_renderer *r) {
         return RT_ERR_STATE;
     }
     const rtd::PhotonWave w = rtd::photon_wave_at(r->d_sorted.p, (uint32_t)traced);
-    const rtd::DevJob job = rt::make_job(r, 0u);
-    if (int st = rt::ensure_job_table(r)) return st;
-    RT_CK(r->jobs.upload(&job, 1, s));
+    if (rtd::photon_pass_reads_table(r->scene, r->tuning)) {
+        const rtd::DevJob job = rt::make_job(r, 0u);
+        if (int st = rt::ensure_job_table(r)) return st;
+        RT_CK(r->jobs.upload(&job, 1, s));
+    }
     RT_CK(cudaEventRecord(r->events.ev[EV_TRACE0], s));
     RT_CK(rtd::launch_photon_wave(tp, w, r->jobs.device(), r->num_sms, r->tuning, s));
     RT_CK(cudaEventRecord(r->events.ev[EV_TRACE1], s));
@@ -1038,23 +1047,24 @@ extern "C" int rt_get_stats(rt_renderer *r, rt_frame_stats *out) {
         out->segments = ctr[0];
         out->shadow_rays = ctr[1];
         out->photons_stored = total;
-        auto ms = [&](int a, int b) {
+        auto ms = [&](cudaEvent_t a, cudaEvent_t b) {
             float v = 0.0f;
-            if (cudaEventElapsedTime(&v, r->events.ev[a], r->events.ev[b]) != cudaSuccess) {
+            if (cudaEventElapsedTime(&v, a, b) != cudaSuccess) {
                 cudaGetLastError();
                 return 0.0f;
             }
             return v;
         };
         if (r->have_frame_timing) {
-            out->ms_gather = ms(EV_FRAME0, EV_GATHER1);
-            out->ms_denoise = ms(EV_GATHER1, EV_DENOISE1);
-            out->ms_resolve = ms(EV_DENOISE1, EV_RESOLVE1);
-            out->ms_frame = ms(EV_FRAME0, EV_RESOLVE1);
+            const cudaEvent_t *e = r->frame_ev;
+            out->ms_gather = ms(e[0], e[1]);
+            out->ms_denoise = ms(e[1], e[2]);
+            out->ms_resolve = ms(e[2], e[3]);
+            out->ms_frame = ms(e[0], e[3]);
         }
         if (r->have_photon_timing) {
-            out->ms_photon_trace = ms(EV_TRACE0, EV_TRACE1);
-            out->ms_grid_build = ms(EV_TRACE1, EV_GRID1);
+            out->ms_photon_trace = ms(r->events.ev[EV_TRACE0], r->events.ev[EV_TRACE1]);
+            out->ms_grid_build = ms(r->events.ev[EV_TRACE1], r->events.ev[EV_GRID1]);
         }
         // Drain the per-frame ring: complete groups of four events.
         auto el = [](cudaEvent_t a, cudaEvent_t b) {
@@ -1067,14 +1077,15 @@ extern "C" int rt_get_stats(rt_renderer *r, rt_frame_stats *out) {
         };
         const size_t groups = r->ring.used / 4;
         for (size_t g = 0; g < groups; ++g) {
-            cudaEvent_t *e = &r->ring.pool[4 * g];
+            cudaEvent_t *e = &r->ring.pool[4 * g], denoised = e[r->ring_denoised[g] ? 2 : 1];
             out->ms_gather_sum += el(e[0], e[1]);
-            out->ms_denoise_sum += el(e[1], e[2]);
-            out->ms_resolve_sum += el(e[2], e[3]);
+            out->ms_denoise_sum += el(e[1], denoised);
+            out->ms_resolve_sum += el(denoised, e[3]);
             out->ms_frame_sum += el(e[0], e[3]);
         }
         out->timed_frames = groups;
         r->ring.used = 0;
+        r->ring_denoised.clear();
         return RT_OK;
     });
 }

@@ -239,6 +239,8 @@ struct rt_renderer {
     uint32_t last_denoise_passes = 0;
     rt::Events events;
     rt::FrameEventRing ring;
+    std::vector<bool> ring_denoised;  // per frame in the ring: its denoise end is recorded (else it is its gather end)
+    cudaEvent_t frame_ev[4] = {};  // the last solo frame's events (of the ring, or of events when it is full)
     // Gather-pass profiling (rt_set_profiling): flags, events around the profiled launches (2 per
     // launch of each kind, plus the pass bounds), the counting kernels' work counters, the sums.
     uint32_t prof_flags = 0;
