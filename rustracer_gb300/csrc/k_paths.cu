@@ -19,7 +19,7 @@
 namespace rtd {
 
 namespace {
-constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 4;  // 128 registers
+constexpr int kPathsBlock = 256, kPathsBlocksPerSm = 2;  // 128 registers
 // Paths per warp when they are too few for 32 each: below this a warp's idle lanes gain nothing (measured at
 // 64 x 64: 2, 4 and 8 alike, 16 10% slower, 32 28%).
 constexpr uint32_t kPathsShare = 4;
@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     // Few paths are spread over all warps.
     const uint32_t warps = gridDim.x * (kPathsBlock / 32);
     const uint32_t share = min(32u, max(kPathsShare, (n + warps - 1u) / warps));
-    for (uint32_t base = share * (blockIdx.x * (kPathsBlock / 32) + (threadIdx.x >> 5)); base < n; base += share * warps) {
+    for (uint32_t first = 0u; first < n; first += share * warps) {  // (the same rounds for a block's warps)
+        const uint32_t base = first + share * (blockIdx.x * (kPathsBlock / 32) + (threadIdx.x >> 5));
         bool alive = lane < share && base + lane < n;
         uint32_t slot = 0u, jid = 0u;
         if (kWhole) {
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                 if (lit) p.nee[slot].w = __uint_as_float(__float_as_uint(p.nee[slot].w) | kNeeLit);
                 out.shadow = false;
             }
-            if (!__any_sync(0xFFFFFFFFu, alive)) break;
+            if (kPhotons ? !__any_sync(0xFFFFFFFFu, alive) : !__syncthreads_or(alive)) break;
             if (alive) {
                 uint32_t prim = 0u, word = 0u;
                 if (hit_dist < kInf) {
