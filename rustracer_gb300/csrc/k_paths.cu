@@ -44,6 +44,12 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     const LookupRuns<kRunsA> runs{reinterpret_cast<uint2 *>(&w) + lane, rest};
     uint32_t *hit_list = reinterpret_cast<uint32_t *>(runs.a - lane + 32u * kRunsA) + lane;
     static_assert(sizeof(WarpTrav) >= 32 * (kRunsA * sizeof(uint2) + kHitList * sizeof(uint32_t)), "lookup state");
+    // A step is some 3,000 instructions without a loop, which the warps of a scheduler would each fetch at another
+    // place (40% of their cycles), so a block's warps start each shade step together: 16 Cornell frames of
+    // 256 x 256 2.07 -> 1.71 ms (blocks of four warps 1.79, of sixteen 1.73).  Not with photon maps and several
+    // samples in every pixel, where lookups that cannot wait keep the others waiting (relight at 4 spp 4.28 against
+    // 4.25 ms; one sample, 640 x 360, four frames: 1.88 against 1.95).
+    const bool lockstep = !kPhotons || p.lockstep != 0u;
     const Treelet tree{nullptr, nullptr, 0u};
     LaneWalk r;
     r.busy = r.visiting = r.any_hit = r.careful = r.held = false;
@@ -73,6 +79,15 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
         bool lookup = false;  // a photon lookup waits in the slot's record of preq
         const DevJob &job = job_at<kMulti>(p, jid);
         const DevScene &sc = job.scene;
+        auto look_up = [&]() {
+            if (lookup) {
+                const float4 *req = p.preq + 3ull * slot;
+                const float4 r0 = req[0], r1 = req[1], r2 = req[2];
+                photon_lookup(p, job, slot, __float_as_uint(r0.w), xyz(r0), xyz(r1), xyz(r2), runs, hit_list);
+                lookup = false;
+            }
+            __syncwarp();
+        };
         const float4 *records = kMulti ? sc.wnodes : p.records0, *tris = kMulti ? sc.tri_ord : p.tris0;
         const bool empty = kMulti ? sc.cnode_count == 0u : p.empty0 != 0u;
         const bool any = kMulti ? sc.any_hit_shadows != 0u : p.any_hit0 != 0u;
@@ -178,7 +193,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                 if (lit) p.nee[slot].w = __uint_as_float(__float_as_uint(p.nee[slot].w) | kNeeLit);
                 out.shadow = false;
             }
-            if (kPhotons ? !__any_sync(0xFFFFFFFFu, alive) : !__syncthreads_or(alive)) break;
+            if (lockstep ? !__syncthreads_or(alive) : !__any_sync(0xFFFFFFFFu, alive)) break;
             if (alive) {
                 uint32_t prim = 0u, word = 0u;
                 if (hit_dist < kInf) {
@@ -196,18 +211,11 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                 alive = out.keep;
             }
             // A lookup's term comes before the next one added to its slot: the lookups wait until a lane that
-            // has one goes on, or no lane does, and run together (640 x 360 with a photon map, four frames: 2.15 ms
-            // with each lookup right after its shade step, 2.03 together).
-            if (kPhotons && (__any_sync(0xFFFFFFFFu, lookup && alive) || !__any_sync(0xFFFFFFFFu, alive))) {
-                if (lookup) {
-                    const float4 *req = p.preq + 3ull * slot;
-                    const float4 r0 = req[0], r1 = req[1], r2 = req[2];
-                    photon_lookup(p, job, slot, __float_as_uint(r0.w), xyz(r0), xyz(r1), xyz(r2), runs, hit_list);
-                    lookup = false;
-                }
-                __syncwarp();
-            }
+            // has one goes on, or the block's paths have all ended (without lockstep the warp's), and run together
+            // (640 x 360 with a photon map, four frames: 2.15 ms with each lookup right after its shade step).
+            if (kPhotons && __any_sync(0xFFFFFFFFu, lookup && alive)) look_up();
         }
+        if (kPhotons) look_up();
         if (kWhole && mine) finalize_slot(p, job, slot);
     }
     segments = __reduce_add_sync(0xFFFFFFFFu, segments);

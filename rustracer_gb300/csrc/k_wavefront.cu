@@ -611,6 +611,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         wide_need = jobs[j].wide_stack > wide_need ? jobs[j].wide_stack : wide_need;
         wide = wide && jobs[j].wide != 0u;
         cut = cut || jobs[j].scene->any_hit_shadows == 0u;
+        if (jobs[j].spp <= 1u) p.lockstep = 1u;
     }
     if (n_jobs == 1u) set_scene0(p, *jobs[0].scene, wide);
     const bool one = n_jobs == 1u && jobs[0].job != nullptr;  // the launches carry the job
