@@ -602,7 +602,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     uint64_t slots = 0;
     uint32_t stack_need = 0, wide_need = 0;
     bool wide = n_jobs > 0;  // four-wide records when every job's scene has them
-    bool cut = false;
+    bool cut = false, few_records = true;
     uint64_t tiles = 0;
     for (uint32_t j = 0; j < n_jobs; ++j) {
         tiles += ((jobs[j].width + 7u) / 8u) * ((jobs[j].height + 3u) / 4u);
@@ -612,6 +612,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         wide = wide && jobs[j].wide != 0u;
         cut = cut || jobs[j].scene->any_hit_shadows == 0u;
         if (jobs[j].spp <= 1u) p.lockstep = 1u;
+        few_records = few_records && jobs[j].scene->wnode_count <= 64u;
     }
     if (n_jobs == 1u) set_scene0(p, *jobs[0].scene, wide);
     const bool one = n_jobs == 1u && jobs[0].job != nullptr;  // the launches carry the job
@@ -621,14 +622,17 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         photons = photons || jobs[j].photons != 0u;
         debug = debug || jobs[j].debug != 0u;
     }
-    // Few pixels: the whole pass in one launch.  Few paths left: the rest of them in one launch, tried at
+    // Few pixels: the whole pass in one launch, with trees of a few dozen records, whose walks hardly differ, up to
+    // 8/5 as many (Cornell box at 400 x 300, 1 and 4 spp: 189 and 653 us against 222 and 699, 20 leaf cards 204 / 265;
+    // a 20k-triangle room 491 / 462; 512 x 300 at 3 spp 576 / 547).  Few paths left: the rest of them in one launch, tried at
     // every third iteration, with photon maps (which end most paths at once) at every second (an idle try
     // costs 2.5 us).  Gather with and without the tries: config 2 18.7 / 19.1 ms, 640 x 480 at 4 spp in a
     // 328k-triangle room 4.39 / 4.71, cut-out foliage 1.51 / 1.57, 640 x 480 with a photon map 0.81 / 1.13;
     // a limit of half as many paths measures 18.9, 4.44, 1.50 and 0.81.  Both need the four-wide records, no
     // debug view and no per-launch profile.
     const uint32_t most = wide && !debug && !prof && !p.work ? paths_limit(num_sms) : 0u;
-    if (iters && slots <= most) return launch_paths_frame(p, (uint32_t)tiles, !one, photons, num_sms, st);
+    const uint32_t whole = few_records ? most + most / 5u * 3u : most;
+    if (iters && slots <= whole) return launch_paths_frame(p, (uint32_t)tiles, !one, photons, num_sms, st);
     if ((e = cudaMemsetAsync(p.counts, 0, sizeof(uint32_t) * 4 * (size_t)(iters + 1), st)) != cudaSuccess) return e;
     if (tiles)
         (one ? wf_generate_kernel<false> : wf_generate_kernel<true>)<<<(unsigned)((tiles + 3u) / 4u), 128, 0, st>>>(
