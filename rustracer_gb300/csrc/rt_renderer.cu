@@ -1179,6 +1179,20 @@ extern "C" int rt_read_photon_grid(rt_renderer *r, uint32_t *counts, uint32_t *m
 // ================================================================================================
 // Stage entry points (host buffers in and out; the default stream; temporaries freed on return)
 // ================================================================================================
+namespace {
+// The device buffers of an image stage, `n` of the same size in one allocation: 40 us to take and 40 to give back,
+// each, whatever its size (640 x 360 through both stages 1.26 ms with an allocation per buffer, 0.85 with one).
+struct StageBuffers {
+    DevBuf mem;
+    size_t size = 0;
+    cudaError_t alloc(size_t bytes, size_t n) {
+        size = (bytes + 255) & ~(size_t)255;
+        return mem.alloc(size * n);
+    }
+    float4 *part(size_t i) const { return reinterpret_cast<float4 *>(mem.as<unsigned char>() + i * size); }
+};
+}  // namespace
+
 extern "C" int rt_stage_denoise(const float *frame_rgba, const float *gbuffer, const float *moments, uint32_t width,
                                 uint32_t height, float alpha, uint32_t passes, float *out_rgba) {
     return rt::guarded("rt_stage_denoise", [&]() -> int {
@@ -1188,15 +1202,12 @@ extern "C" int rt_stage_denoise(const float *frame_rgba, const float *gbuffer, c
             return RT_ERR_INVALID_ARGUMENT;
         }
         const size_t bytes = (size_t)width * height * 16;
-        DevBuf a, b, g, m;
-        RT_CK(a.alloc(bytes));
-        RT_CK(b.alloc(bytes));
-        RT_CK(g.alloc(bytes));
-        RT_CK(m.alloc(bytes));
-        RT_CK(cudaMemcpy(a.p, frame_rgba, bytes, cudaMemcpyHostToDevice));
-        RT_CK(cudaMemcpy(g.p, gbuffer, bytes, cudaMemcpyHostToDevice));
-        RT_CK(cudaMemcpy(m.p, moments, bytes, cudaMemcpyHostToDevice));
-        float4 *cur = a.as<float4>(), *nxt = b.as<float4>();
+        StageBuffers mem;
+        RT_CK(mem.alloc(bytes, 4));
+        float4 *cur = mem.part(0), *nxt = mem.part(1), *g = mem.part(2), *m = mem.part(3);
+        RT_CK(cudaMemcpy(cur, frame_rgba, bytes, cudaMemcpyHostToDevice));
+        RT_CK(cudaMemcpy(g, gbuffer, bytes, cudaMemcpyHostToDevice));
+        RT_CK(cudaMemcpy(m, moments, bytes, cudaMemcpyHostToDevice));
         for (uint32_t it = 0; it < passes; ++it) {
             rt_denoise_params dp;
             std::memset(&dp, 0, sizeof(dp));
@@ -1207,7 +1218,7 @@ extern "C" int rt_stage_denoise(const float *frame_rgba, const float *gbuffer, c
             dp.phi_normal = 12.0f;
             dp.phi_depth = 0.05f;
             dp.alpha = alpha;
-            RT_CK(rtd::launch_denoise(cur, nxt, g.as<float4>(), m.as<float4>(), dp, nullptr, 0));
+            RT_CK(rtd::launch_denoise(cur, nxt, g, m, dp, nullptr, 0));
             std::swap(cur, nxt);
         }
         RT_CK(cudaMemcpy(out_rgba, cur, bytes, cudaMemcpyDeviceToHost));
@@ -1224,23 +1235,21 @@ extern "C" int rt_stage_resolve(const float *frame_rgba, float *accum_inout, con
             return RT_ERR_INVALID_ARGUMENT;
         }
         const size_t bytes = (size_t)width * height * 16;
-        DevBuf f, a, g, o;
-        RT_CK(f.alloc(bytes));
-        RT_CK(a.alloc(bytes));
-        RT_CK(o.alloc(bytes / 4));
-        RT_CK(cudaMemcpy(f.p, frame_rgba, bytes, cudaMemcpyHostToDevice));
-        RT_CK(cudaMemcpy(a.p, accum_inout, bytes, cudaMemcpyHostToDevice));
+        StageBuffers mem;
+        RT_CK(mem.alloc(bytes, gbuffer ? 4 : 3));
+        float4 *f = mem.part(0), *a = mem.part(1), *o = mem.part(2);
+        RT_CK(cudaMemcpy(f, frame_rgba, bytes, cudaMemcpyHostToDevice));
+        RT_CK(cudaMemcpy(a, accum_inout, bytes, cudaMemcpyHostToDevice));
         const float4 *gp = nullptr;
         if (gbuffer) {
-            RT_CK(g.alloc(bytes));
-            RT_CK(cudaMemcpy(g.p, gbuffer, bytes, cudaMemcpyHostToDevice));
-            gp = g.as<float4>();
+            RT_CK(cudaMemcpy(mem.part(3), gbuffer, bytes, cudaMemcpyHostToDevice));
+            gp = mem.part(3);
         }
         rt_tonemap_params t = *tp;
         t.width = width;
-        RT_CK(rtd::launch_resolve(f.as<float4>(), a.as<float4>(), gp, width, height, alpha, nullptr, t, o.as<uchar4>(), 0));
-        RT_CK(cudaMemcpy(accum_inout, a.p, bytes, cudaMemcpyDeviceToHost));
-        RT_CK(cudaMemcpy(out_rgba8, o.p, bytes / 4, cudaMemcpyDeviceToHost));
+        RT_CK(rtd::launch_resolve(f, a, gp, width, height, alpha, nullptr, t, reinterpret_cast<uchar4 *>(o), 0));
+        RT_CK(cudaMemcpy(accum_inout, a, bytes, cudaMemcpyDeviceToHost));
+        RT_CK(cudaMemcpy(out_rgba8, o, bytes / 4, cudaMemcpyDeviceToHost));
         return RT_OK;
     });
 }
