@@ -107,9 +107,11 @@ __device__ __forceinline__ uint32_t shade_key(const WaveJob &p, const uint32_t *
 }
 
 // kBlocks: resident blocks per SM the register allocation aims at (4: ~123 registers; 5: 96
-// registers with 62 bytes of spills; 6: 80 registers, ~200 bytes of spills, the default: the extra
-// warps hide the kernel's dependent loads, config-2 shade 7.04 -> 6.56 -> 6.41 ms per frame), chosen
-// per launch by the tuning's shade_blocks.
+// registers with 62 bytes of spills; 6: 80 registers, 100 to 200 bytes of spills, the default: the extra
+// warps hide the kernel's dependent loads), chosen per launch by the tuning's shade_blocks.  Bound by divergence
+// (16 of 32 lanes), those loads and a long body (10% of a warp's cycles wait for instructions).  1080p room frame
+// with the job in the launch: 19.17 ms with 5 blocks, 18.14 with 6, 18.68 with 7; with the state prefetched to L1
+// while the entries are ordered, blocks of 64, 256 or 384, or the texture fetch out of line: the same to 2% slower.
 template <bool kPhotons, bool kDebug, bool kMulti, int kBlocks>
 __global__ void __launch_bounds__(128, kBlocks) wf_shade_kernel(const __grid_constant__ WaveJob p, uint32_t iter,
                                                                uint32_t most) {
@@ -628,7 +630,8 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     // every third iteration, with photon maps (which end most paths at once) at every second (an idle try
     // costs 2.5 us).  Gather with and without the tries: config 2 18.7 / 19.1 ms, 640 x 480 at 4 spp in a
     // 328k-triangle room 4.39 / 4.71, cut-out foliage 1.51 / 1.57, 640 x 480 with a photon map 0.81 / 1.13;
-    // a limit of half as many paths measures 18.9, 4.44, 1.50 and 0.81.  Both need the four-wide records, no
+    // a limit of half as many paths measures 18.9, 4.44, 1.50 and 0.81, later 1080p room frames 17.99 against 17.83, with
+    // twice as many 17.98.  Both need the four-wide records, no
     // debug view and no per-launch profile.
     const uint32_t most = wide && !debug && !prof && !p.work ? paths_limit(num_sms) : 0u;
     const uint32_t whole = few_records ? most + most / 5u * 3u : most;
