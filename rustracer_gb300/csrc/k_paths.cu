@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     uint2 deep[kMaxStack - kTopStack];
     WarpTrav &w = reinterpret_cast<WarpTrav *>(trav_smem + sizeof(uint2) * kTopStack * kPathsBlock)[threadIdx.x >> 5];
     // Between walks the warp's traversal state holds the photon lookups' runs and hits.
-    constexpr uint32_t kRunsA = 5;
+    constexpr uint32_t kRunsA = 4;
     uint2 rest[kLookupCells - kRunsA];
     const LookupRuns<kRunsA> runs{reinterpret_cast<uint2 *>(&w) + lane, rest};
     uint32_t *hit_list = reinterpret_cast<uint32_t *>(runs.a - lane + 32u * kRunsA) + lane;
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     const bool lockstep = !kPhotons || p.lockstep != 0u;
     const Treelet tree{nullptr, nullptr, 0u};
     LaneWalk r;
-    r.busy = r.visiting = r.any_hit = r.careful = r.held = false;
+    r.busy = r.visiting = r.any_hit = false;
     r.st.sp = 0u;
     uint32_t segments = 0u, shadow_rays = 0u;
     // Few paths are spread over all warps.
@@ -126,7 +126,6 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                     r.st.cap = kMaxStack;
                     r.any_hit = false;
                     r.st.t = kInf;
-                    if (kMulti) w.margin[lane] = sc.tie_margin;
                     walk_begin(r, w, xyz(o), xyz(d), mk3(1.0f, 1.0f, 1.0f) / xyz(d), tris);
                     r.visiting = !empty;
                     segments += 1u;
@@ -150,7 +149,6 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                                 r.st.records = os.wnodes;
                                 otris = os.tri_ord;
                                 oany = os.any_hit_shadows != 0u;
-                                w.margin[lane] = os.tie_margin;
                             }
                             // (see wf_trace_kernel)
                             r.any_hit = oany;
@@ -165,14 +163,13 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                         at = min(at + (uint32_t)__popc(idle), n_occ);
                     }
                     uint32_t visits = 0u, tests = 0u;
-                    walk_records<true, 0, kPathsBlock, kMulti, false>(r, w, top, deep, tree, p.records0, p.tris0, 3u, 0,
+                    // (a refill costs little here: three records between them 1.73 ms for the 16 frames, two 1.66,
+                    // one 1.57)
+                    walk_records<true, 0, kPathsBlock, kMulti, false>(r, w, top, deep, tree, p.records0, p.tris0, 1u, 0,
                                                                       visits, tests);
-                    if (r.busy && !r.visiting) do {
+                    if (r.busy && !r.visiting) {
                         bool clear = !r.found && r.st.t == r.st.t;  // (a NaN limit counts as occluded)
                         if (!r.any_hit) {
-                            if (walk_again<kMulti>(r, w, p.tris0, kMulti ? w.margin[lane] : p.tie_margin0,
-                                                   occ ? search_limit(w.limit[lane]) : kInf))
-                                continue;
                             const unsigned long long hit = w.best[lane];
                             if (occ) {
                                 clear = cut_out_lit(job_at<kMulti>(p, occ_job).scene, w.ro[lane], w.rd[lane], w.limit[lane], hit);
@@ -183,7 +180,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                         }
                         if (occ && clear) atomicOr(&w.coming, 1u << owner);
                         r.busy = false;
-                    } while (false);
+                    }
                 }
                 __syncwarp();
                 lit = (w.coming >> lane & 1u) != 0u;

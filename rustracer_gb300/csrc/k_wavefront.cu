@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
     request();
 
     LaneWalk r;
-    r.busy = r.visiting = r.any_hit = r.careful = r.held = false;
+    r.busy = r.visiting = r.any_hit = false;
     r.st.sp = 0u;
     uint32_t id = 0u;
     uint32_t work[4] = {0u, 0u, 0u, 0u};  // kCount: records closest / occlusion, tests closest / occlusion
@@ -401,7 +401,6 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
                         tris = sc.tri_ord;
                         any = sc.any_hit_shadows;
                         empty = sc.cnode_count == 0u;
-                        w.margin[lane] = sc.tie_margin;
                     }
                     // An occlusion ray asks for hits below the limit: any one without cut-out materials, the
                     // closest with them (the reference's closest-hit-then-alpha rule; looked for a little
@@ -430,14 +429,11 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
             work[(id & kOcclusion) ? 1 : 0] += visits;
             work[(id & kOcclusion) ? 3 : 2] += tests;
         }
-        if (r.busy && !r.visiting) do {
+        if (r.busy && !r.visiting) {
             const uint32_t slot = id & ~kOcclusion;
             const bool occ = (id & kOcclusion) != 0u;
             bool lit = !r.found && r.st.t == r.st.t;  // (a NaN limit counts as occluded)
             if (!r.any_hit) {
-                if (walk_again<kMulti>(r, w, p.tris0, kMulti ? w.margin[lane] : p.tie_margin0,
-                                       kCut && occ ? search_limit(w.limit[lane]) : kInf))
-                    continue;
                 const unsigned long long hit = w.best[lane];
                 if (kCut && occ)
                     lit = cut_out_lit(p.jobs[__float_as_uint(p.thr[slot].w)].scene, w.ro[lane], w.rd[lane], w.limit[lane],
@@ -447,7 +443,7 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
             }
             if (occ && lit) atomicOr(reinterpret_cast<uint32_t *>(&p.nee[slot].w), kNeeLit);
             r.busy = false;
-        } while (false);
+        }
     }
     if (kCount && p.work) {
 #pragma unroll
@@ -566,7 +562,6 @@ void set_scene0(WaveParams &p, const DevScene &scene, bool wide) {
     p.tris0 = scene.tri_ord;
     p.any_hit0 = scene.any_hit_shadows;
     p.empty0 = scene.cnode_count == 0u ? 1u : 0u;
-    p.tie_margin0 = scene.tie_margin;
 }
 }  // namespace
 

@@ -107,7 +107,6 @@ std::vector<unsigned char> BatchEngine::signature(rt_renderer *const *rs, uint32
         put(s, r->scene.tri_ord);
         put(s, r->scene.cnode_count);
         put(s, r->scene.any_hit_shadows);
-        put(s, r->scene.tie_margin);
         put(s, r->scene.wide_stack);
         put(s, r->glow);
         put(s, r->marker);

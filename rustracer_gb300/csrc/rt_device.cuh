@@ -172,9 +172,6 @@ struct DevScene {
     // entries (wide_stack); otherwise wnodes is null and only the two-wide records are used.
     const float4 *wnodes;
     uint32_t wnode_count, wide_stack;
-    // Absolute part of the distance below which a ray's two nearest hits count as tied (see rt_traverse.cuh):
-    // 2^-17 of the scene's largest coordinate, a hundred times a hit's rounding error there.
-    float tie_margin;
     uint32_t any_hit_shadows;  // 1: no alpha-cutout material, shadow rays may stop at the first hit
     const float4 *tris;      // 8 x float4 per TriangleGpu
     const float4 *mats;      // 4 x float4 per MaterialGpu

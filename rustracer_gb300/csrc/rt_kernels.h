@@ -50,10 +50,9 @@ struct WaveParams {
     // by closest-hit / occlusion rays, then their leaf triangle tests.
     unsigned long long *work;
     // A one-job launch's scene: its records, leaf-ordered triangles, whether its occlusion rays may stop at
-    // any hit, whether it has no triangles, and its tie margin; filled by the launchers.
+    // any hit and whether it has no triangles; filled by the launchers.
     const float4 *records0, *tris0;
     uint32_t any_hit0, empty0;
-    float tie_margin0;
     uint32_t lockstep;  // the few-path kernel's blocks with photon lookups shade together too (set by launch_wavefront)
 };
 // The parameters of the kernels that read a job's tables.  A launch over one job whose values are known when it

@@ -418,9 +418,6 @@ int resident_scene_create(const rt_scene_desc *sd, rt_resident_scene **out) {
     ds.wide_stack = wide.nodes.empty() ? 0u : wide.stack_need;
     // A near-first traversal holds at most one pending entry per tree level.
     ds.stack_cap = lay.max_depth < 32u ? 32u : 63u;
-    for (int a = 0; a < 3 && sd->bvh_node_count; ++a)
-        ds.tie_margin = std::max({ds.tie_margin, 0x1p-17f * std::fabs(sd->bvh_nodes[0].bbox_min[a]),
-                                  0x1p-17f * std::fabs(sd->bvh_nodes[0].bbox_max[a])});
     ds.any_hit_shadows = 1u;
     for (uint64_t i = 0; i < sd->material_count; ++i)
         if ((sd->materials[i].flags & RT_MAT_FLAG_ALPHA_CUTOUT) && sd->materials[i].tex_albedo != RT_TEX_NONE)

@@ -4,23 +4,21 @@
 // step.  A record fetch tests the children's boxes with the reference's slab test (gather.wgsl:71-75:
 // (bmin - ro) / d, te <= ta && ta > 0 && te < t); hit internal children are visited nearest entry
 // first, the others pushed.  Hit leaves are not tested by the lane that met them: they go into the
-// warp's leaf queue, and whenever eight are waiting the warp tests them together, four lanes per leaf,
-// one triangle per lane.  The tree is the reference's, so the closest hit is the reference's.
+// warp's leaf list, which the warp tests together before it goes on, four lanes per leaf, one triangle
+// per lane.  The tree is the reference's, so the closest hit is the reference's.
 //
 // Triangles hit at exactly equal t resolve to the lowest prim slot: leaves hold consecutive slot ranges
 // with the left child's below the right's (bvh.rs:159-219), so the reference's left-first walk, where
 // the first strictly smaller t wins, meets the lowest slot first.  The best hit of a lane's ray is one
 // 64-bit word, t's bits above the prim slot (t is positive, so the words order as (t, slot) pairs), and a
-// test that hits lowers it with an atomic minimum, whatever order the tests come in.
+// test that hits lowers it with an atomic minimum, whatever order a step's tests come in.
 //
-// The order could matter in one case.  A walk that tests leaves as it meets them never tests a leaf it
-// enters at or beyond the hit it already has; with its leaves still queued, a lane may.  Such a leaf can
-// only change the result if the nearest hit lies nearer than its own leaf's box is entered, and a second
-// hit fits in between.  Both distances are rounded values of nearly the same number, so the walk keeps the
-// second nearest hit's t too, and when the two nearest hits are closer than kTieRelative of t plus
-// DevScene.tie_margin, a bound on the entry decides (hit_entry_bound); a ray it does not clear (about one
-// in a million) is walked again, waiting for the tests of each record's leaves before it goes on.  Results
-// do not depend on which rays share a warp.
+// A leaf is tested only if its box is entered before the nearest hit so far, and a hit's computed distance
+// can lie before its own leaf's box: by rounding, or by far more on a sliver.  So which leaves have been
+// tested when a box is looked at can decide between two overlapping surfaces.  Every ray's leaves are
+// therefore tested before its next record, and the result is its own: it does not depend on which rays share
+// the warp or on the launch.  (Waiting until eight leaves are listed keeps more lanes busy, 1080p frame of the
+// 1.31M-triangle room 18.28 against 18.42 ms, but leaves a walk unaware of a hit for a record or two.)
 #pragma once
 #include "rt_kernels.h"
 
@@ -30,10 +28,8 @@ namespace rtd {
 // there) in local memory.  11 let 7 blocks of 128 threads share an SM with 28 KB of L1 left; 8 measure
 // 2% slower, 14 0.5%, 16 (6 blocks) 9%.
 constexpr uint32_t kTopStack = 11, kMaxStack = 64;
-// Leaves a warp's queue holds: up to 7 wait from earlier steps, and a step adds up to 4 per lane.
-// Two hits farther apart than this part of their distance (and tie_margin) are no tie.
-constexpr float kTieRelative = 0x1p-10f;
-constexpr uint32_t kLeafCap = 7 + 4 * 32 + 1;
+// Leaves a step can meet: up to 4 per lane.
+constexpr uint32_t kLeafCap = 4 * 32;
 
 // A warp's shared state.
 struct __align__(16) WarpTrav {
@@ -49,10 +45,8 @@ struct __align__(16) WarpTrav {
     uint32_t at, ready;       // rays [at, ready) of the copied ones are unclaimed
     uint32_t coming;          // rays being copied
     unsigned long long best[32];  // t bits << 32 | prim slot
-    uint32_t second[32];          // bits of the second nearest hit's t
     float limit[32];              // occlusion rays that look for the closest hit: hits below it count
-    float margin[32];             // the scene's tie margin (launches over several scenes)
-    uint2 leaf[kLeafCap];         // queued leaves: first prim slot, count << 5 | owner lane
+    uint2 leaf[kLeafCap];         // the step's leaves: first prim slot, count << 5 | owner lane
 };
 
 __device__ __forceinline__ unsigned long long hit_word(float t, uint32_t prim) {
@@ -92,8 +86,8 @@ __device__ __forceinline__ float hit_distance(f3 ro, f3 rd, float4 v0, float4 e1
     return fabsf(a) < 1e-7f || u < 0.0f || u > 1.0f || v < 0.0f || u + v > 1.0f ? 0.0f : t;
 }
 
-// Tests the triangles of queued leaves [first, first + n), n <= 8: lane l takes triangles l % 4,
-// l % 4 + 4, ... of leaf l / 4, against the ray of the lane that queued it.
+// Tests the triangles of listed leaves [first, first + n), n <= 8: lane l takes triangles l % 4,
+// l % 4 + 4, ... of leaf l / 4, against the ray of the lane that met it.
 // tris: the scene's leaf-ordered triangles (kMulti: each ray's own, from its record).
 template <bool kMulti>
 __device__ __forceinline__ void test_leaves(WarpTrav &w, uint32_t first, uint32_t n, const float4 *tris) {
@@ -108,11 +102,7 @@ __device__ __forceinline__ void test_leaves(WarpTrav &w, uint32_t first, uint32_
         const float4 *tp = tris + 3ull * (ref + k);
         const float4 v0 = __ldg(tp), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
         const float t = hit_distance(ro, rd, v0, e1, e2);
-        // (a hit beyond the second nearest one changes nothing)
-        if (t > kEps && __float_as_uint(t) <= w.second[o]) {
-            const unsigned long long word = hit_word(t, ref + k), old = atomicMin(&w.best[o], word);
-            atomicMin(&w.second[o], (uint32_t)((word < old ? old : word) >> 32));
-        }
+        if (t > kEps) atomicMin(&w.best[o], hit_word(t, ref + k));
     }
 }
 
@@ -134,19 +124,6 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
-}
-
-// An upper bound on where a ray enters the leaf box of the triangle in `prim`: the entry into the
-// triangle's own box, which lies inside, with its corners rebuilt from the edges and moved by delta (more
-// than their rounding).
-__device__ __forceinline__ float hit_entry_bound(const float4 *tris, uint32_t prim, f3 ro, f3 rd, float delta) {
-    const float4 *tp = tris + 3ull * prim;
-    const f3 v0 = xyz(__ldg(tp)), v1 = v0 + xyz(__ldg(tp + 1)), v2 = v0 + xyz(__ldg(tp + 2));
-    const f3 lo = vmin(v0, vmin(v1, v2)) - ro, hi = vmax(v0, vmax(v1, v2)) - ro;
-    const float x = (rd.x > 0.0f ? lo.x + delta : hi.x - delta) / rd.x, y = (rd.y > 0.0f ? lo.y + delta : hi.y - delta) / rd.y,
-                z = (rd.z > 0.0f ? lo.z + delta : hi.z - delta) / rd.z;
-    const float te = fmax3f(x, y, z);
-    return te + fabsf(te) * 0x1p-20f;
 }
 
 // One ray's walk, kept by its lane.
@@ -193,17 +170,17 @@ struct Treelet {
     uint32_t count;
 };
 
-// One step of every lane of a warp: `visiting` lanes test the child boxes of their record, queue the
-// hit leaves behind the `queued` ones in w, and move on to the next record (visiting ends when none is
-// left).  records: the scene's (kMulti: each ray's own, st.records).  tests: the lane's queued triangles
-// are added.  Every lane calls it.
+// One step of every lane of a warp: `visiting` lanes test the child boxes of their record, list the hit
+// leaves in w (`leaves` of them) and move on to the next record (visiting ends when none is left).
+// records: the scene's (kMulti: each ray's own, st.records).  tests: the lane's listed triangles are
+// added.  Every lane calls it.
 //
 // A child is 32 bytes, one load: four-wide (min.x, max.x, min.y, max.y), (min.z, max.z, ref, count), so
 // that both planes of an axis go through one packed subtraction and one packed product; two-wide
 // (min, ref), (max, count).
 template <bool kWide, int kTree, int kBlock, bool kMulti>
 __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep, bool &visiting, WarpTrav &w,
-                                          uint32_t &queued, const Treelet &tree, const float4 *records,
+                                          uint32_t &leaves, const Treelet &tree, const float4 *records,
                                           uint32_t &tests) {
     constexpr int K = kWide ? 4 : 2;
     if (kMulti) records = st.records;
@@ -254,11 +231,11 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
     for (int c = 0; c < K; ++c) {
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, cnt[c] != 0u);
         if (cnt[c] != 0u) {
-            w.leaf[queued + __popc(m & lanemask_lt())] =
+            w.leaf[leaves + __popc(m & lanemask_lt())] =
                 make_uint2(ref[c], cnt[c] << 5 | (threadIdx.x & 31u));
             tests += cnt[c];
         }
-        queued += __popc(m);
+        leaves += __popc(m);
     }
     if (visiting) {
         auto cswap = [&](int i, int j) {
@@ -306,69 +283,47 @@ __device__ __forceinline__ void trav_step(TravLane &st, uint2 *top, uint2 *deep,
 struct LaneWalk {
     TravLane st;
     bool busy, visiting;
-    bool any_hit;        // an occlusion ray that may stop at its first hit below st.t
-    bool found;          // a hit below the starting st.t
-    bool careful, held;  // walked again; waits for its leaves' tests
+    bool any_hit;  // an occlusion ray that may stop at its first hit below st.t
+    bool found;    // a hit below the starting st.t
 };
 
-// The ray at the root with st.t, and no hit yet.
-__device__ __forceinline__ void walk_root(LaneWalk &r, WarpTrav &w) {
-    const uint32_t lane = threadIdx.x & 31u;
-    w.best[lane] = hit_word(r.st.t, 0u);
-    // (an occlusion ray that may stop early takes no interest in hits beyond its limit)
-    w.second[lane] = r.any_hit ? __float_as_uint(r.st.t) : 0x7F800000u;
-    r.st.node = 0u;
-    r.st.te = -kInf;
-    r.st.sp = 0u;
-}
-// Gives the lane a ray to walk (r.st.t, records and cap and r.any_hit are set): origin o, direction d, the
-// scene's triangles.
+// Gives the lane a ray to walk from the root (r.st.t, records and cap and r.any_hit are set): origin o,
+// direction d, the scene's triangles.
 __device__ __forceinline__ void walk_begin(LaneWalk &r, WarpTrav &w, f3 o, f3 d, f3 inv, const float4 *tris) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long tp = (unsigned long long)tris;
     w.ro[lane] = make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)tp));
     w.rd[lane] = make_float4(d.x, d.y, d.z, __uint_as_float((uint32_t)(tp >> 32)));
+    w.best[lane] = hit_word(r.st.t, 0u);
     r.st.minus_ro[0] = pack2(-o.x, -o.x);
     r.st.minus_ro[1] = pack2(-o.y, -o.y);
     r.st.minus_ro[2] = pack2(-o.z, -o.z);
     r.st.inv[0] = pack2(inv.x, inv.x);
     r.st.inv[1] = pack2(inv.y, inv.y);
     r.st.inv[2] = pack2(inv.z, inv.z);
-    walk_root(r, w);
-    r.found = r.careful = false;
+    r.st.node = 0u;
+    r.st.te = -kInf;
+    r.st.sp = 0u;
+    r.found = false;
     r.busy = true;
 }
 
-// Up to max_steps records for every lane of a warp (fewer once `few` or less lanes still walk), the queued
-// leaves tested eight at a time; then the rest of them, so that a lane that is no longer visiting has its
-// result.  visits and tests (kCount) count the lane's records and triangles.
+// Up to max_steps records for every lane of a warp (fewer once `few` or less lanes still walk), with the
+// tests of their leaves.  visits and tests (kCount) count the lane's records and triangles.
 template <bool kWide, int kTree, int kBlock, bool kMulti, bool kCount>
 __device__ __forceinline__ void walk_records(LaneWalk &r, WarpTrav &w, uint2 *top, uint2 *deep, const Treelet &tree,
                                              const float4 *records, const float4 *tris, uint32_t max_steps, int few,
                                              uint32_t &visits, uint32_t &tests) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t queued = 0u;
     for (uint32_t k = 0;;) {
-        uint32_t n = 0u;
+        uint32_t leaves = 0u, n = 0u;
         if (kCount && r.visiting) visits += 1u;
-        trav_step<kWide, kTree, kBlock, kMulti>(r.st, top, deep, r.visiting, w, queued, tree, records, n);
+        trav_step<kWide, kTree, kBlock, kMulti>(r.st, top, deep, r.visiting, w, leaves, tree, records, n);
         if (kCount) tests += n;
-        if (r.careful && n != 0u) {
-            r.held = r.visiting;
-            r.visiting = false;
-        }
-        const bool end = ++k >= max_steps || __popc(__ballot_sync(0xFFFFFFFFu, r.visiting)) <= few;
-        if (queued >= 8u || (end && queued != 0u)) {
-            const uint32_t tested = end ? queued : queued & ~7u, left = queued - tested;
+        if (leaves != 0u) {
             __syncwarp();
-            for (uint32_t g = 0u; g < tested; g += 8u) test_leaves<kMulti>(w, g, min(8u, tested - g), tris);
-            if (left != 0u) {  // the leaves left over move to the front
-                const uint2 leaf = w.leaf[tested + (lane & 7u)];
-                __syncwarp();
-                if (lane < left) w.leaf[lane] = leaf;
-            }
+            for (uint32_t g = 0u; g < leaves; g += 8u) test_leaves<kMulti>(w, g, min(8u, leaves - g), tris);
             __syncwarp();
-            queued = left;
             if (r.busy) {
                 const float t = hit_t(w.best[lane]);
                 if (t < r.st.t) {
@@ -376,29 +331,11 @@ __device__ __forceinline__ void walk_records(LaneWalk &r, WarpTrav &w, uint2 *to
                     if (r.any_hit) r.visiting = false;
                 }
                 r.st.t = t;
-                if (r.visiting || r.held) r.visiting = trav_settle<kBlock>(r.st, top, deep);
-                r.held = false;
+                if (r.visiting) r.visiting = trav_settle<kBlock>(r.st, top, deep);
             }
         }
-        if (end) break;
+        if (++k >= max_steps || __popc(__ballot_sync(0xFFFFFFFFu, r.visiting)) <= few) break;
     }
-}
-
-// Whether a ray that looked for its closest hit and is done has to be walked again, carefully (see the top of
-// this file); `start` is the t it started with.
-template <bool kMulti>
-__device__ __forceinline__ bool walk_again(LaneWalk &r, WarpTrav &w, const float4 *tris, float margin, float start) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long hit = w.best[lane];
-    const float t = hit_t(hit), second = __uint_as_float(w.second[lane]);
-    if (r.careful || !(second <= t + (t * kTieRelative + margin))) return false;
-    const float4 ro = w.ro[lane], rd = w.rd[lane];
-    if (kMulti) tris = ray_triangles(ro, rd);
-    if (hit_entry_bound(tris, (uint32_t)hit, xyz(ro), xyz(rd), margin * 0x1p-5f) < second) return false;
-    r.st.t = start;
-    walk_root(r, w);
-    r.careful = r.visiting = true;
-    return true;
 }
 
 // Dynamic shared memory of a traversal block: the lane-interleaved stack tops, one WarpTrav per warp, then

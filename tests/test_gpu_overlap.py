@@ -2,10 +2,13 @@
 surfaces a ray hits depends on the order its walk meets them in.  That order is the tree's alone: the image is
 the same bit for bit whatever the shape of the launch.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import rustracer_gb300 as rt
+from rustracer_gb300 import _abi as A
 
 from test_gpu_traverse import CAM, lit, width  # noqa: F401
 
@@ -73,3 +76,87 @@ def test_which_lane_walks_a_ray_does_not_matter(overlapping, width):  # noqa: F8
     ref = image(overlapping, steps=1)
     for tuning in (dict(block_threads=64), dict(block_threads=256, chunk=64), dict(refill_idle=12)):
         assert np.array_equal(image(overlapping, steps=1, **tuning), ref), tuning
+
+
+def test_the_rays_of_a_warp_do_not_matter(overlapping, width):  # noqa: F811
+    """How often a warp takes new rays, and solo frames against batches and the one-launch form."""
+    ref = image(overlapping)
+    for tuning in (dict(), dict(steps=1), dict(steps=7, chunk=64), dict(steps=64), dict(block_threads=64, blocks_per_sm=2),
+                   dict(block_threads=256, blocks_per_sm=1, chunk=256)):
+        assert np.array_equal(image(overlapping, **tuning), ref), tuning
+    small = image(overlapping, 201, 133)
+    cfg = rt.RenderConfig(width=201, height=133, spp=1, accumulate_frames=1, enable_denoise=False, max_bounces=2)
+    rs = [rt.Renderer(overlapping, cfg) for _ in range(5)]
+    for r in rs:
+        r.update_camera(CAM)
+    rs[0].set_profiling(A.PROFILE_EVENTS)
+    rs[0].record_frame()
+    b = rt.Batch(rs[1:], use_graphs=False)
+    b.render_frame()
+    for r in rs:
+        assert np.array_equal(r.read_accumulation(), small)
+    b.close()
+
+
+def deep_scene(live, passed):
+    """A chain of `passed` + `live` nodes towards -z, each with a side subtree that a ray along -z enters, nearer
+    ones deeper, so that all of them wait on the stack.  Only the last side's quad (green) lies on the ray, and a red
+    one at 200, a leaf of the root.  The `passed` sides lie behind that: a walk that knows its hit leaves them out."""
+    s = rt.Scene()
+    red, green = s.add_material(rt.emissive((1, 0, 0), 1.0)), s.add_material(rt.emissive((0, 1, 0), 1.0))
+    boxes = []
+
+    def tri(z, x, m):
+        s.add_mesh([[x - 1, -1, z], [x + 1, -1, z], [x, 1.5, z]], [0, 1, 2], m)
+        boxes.append(((x - 1, -1, z), (x + 1, 1.5, z)))
+
+    tri(-200.0, 0.0, red)
+    dist = [300.0 - i for i in range(passed)] + [190.0 - 2 * i for i in range(live)]
+    for d in dist:
+        tri(-d, -40.0, green)
+        tri(-d, 0.0 if d == dist[-1] else 40.0, green)
+    tri(-30.0, -40.0, green)
+    tri(-30.0, 40.0, green)
+    nodes = []
+
+    def leaf(p):
+        nodes.append((boxes[p][0], boxes[p][1], p, 0, 1))
+        return len(nodes) - 1
+
+    def inner(left, right):
+        nodes.append((np.minimum(nodes[left][0], nodes[right][0]), np.maximum(nodes[left][1], nodes[right][1]), left,
+                      right, 0))
+        return len(nodes) - 1
+
+    nodes.append(None)  # the root
+    below = inner(leaf(len(boxes) - 2), leaf(len(boxes) - 1))
+    for k in reversed(range(len(dist))):
+        below = inner(inner(leaf(1 + 2 * k), leaf(2 + 2 * k)), below)
+    inner(leaf(0), below)
+    nodes[0] = nodes.pop()
+    arr = np.zeros(len(nodes), A.np_dtype(A.BVHNode))
+    for n, (lo, hi, left, right, count) in zip(arr, nodes):
+        n["bbox_min"], n["bbox_max"], n["left_first"], n["right_child"], n["prim_count"] = lo, hi, left, right, count
+    prims = np.arange(len(boxes), dtype=np.uint32)
+    desc = A.SceneDesc.from_buffer_copy(s.describe())
+    desc.bvh_nodes, desc.bvh_node_count = C.cast(arr.ctypes.data, C.POINTER(A.BVHNode)), len(arr)
+    desc.bvh_prims, desc.bvh_prim_count = C.cast(prims.ctypes.data, C.POINTER(C.c_uint32)), len(prims)
+    desc.keep = (s, arr, prims)
+    return desc
+
+
+@pytest.mark.parametrize("steps", [1, 3, 64])
+@pytest.mark.parametrize("live,passed", [(61, 2), (62, 2), (63, 40), (63, 0)])
+def test_full_stack(gpu, live, passed, steps):
+    """Two-wide records drop what goes beyond 63 waiting entries: boxes behind a hit the walk has met are none."""
+    rt.set_traversal_width(2)
+    try:
+        r = rt.Renderer(deep_scene(live, passed), rt.RenderConfig(width=1, height=1, spp=1, max_bounces=1,
+                                                                   accumulate_frames=1, enable_denoise=False))
+    finally:
+        rt.set_traversal_width(4)
+    r.update_camera(rt.Camera((0, 0, 0), (0, 0, -1), (0, 1, 0), 0.01))
+    r.tuning = dict(r.tuning, steps=steps)
+    r.record_frame()
+    red, green, _ = r.read_accumulation().reshape(-1)[:3]
+    assert green > red
