@@ -28,11 +28,14 @@ constexpr uint32_t kPathsShare = 4;
 
 template <bool kMulti, bool kPhotons, bool kWhole>
 __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kernel(const __grid_constant__ WaveJob p,
-                                                                                  uint32_t iter, uint32_t most) {
+                                                                                  uint32_t iter, uint32_t most,
+                                                                                  uint32_t steps) {
     extern __shared__ __align__(16) unsigned char trav_smem[];
     grid_dependency_wait();
     grid_launch_dependents();
-    // kWhole: `most` pixel positions, 8 x 4 tiles as in generate; otherwise the paths queued for `iter`.
+    // kWhole: `most` pixel positions, 8 x 4 tiles as in generate; otherwise the paths queued for `iter`.  steps: the
+    // shade steps a path may take, the wavefront's iterations (a path's 16-bit sample and segment numbers wrap around
+    // before 65,537 samples or segments are done, so they alone would not end it).
     const uint32_t n = kWhole ? most : p.counts[4 * iter];
     if (!kWhole && n > most) return;
     const uint32_t lane = threadIdx.x & 31u;
@@ -95,6 +98,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
         ShadeOut out;
         out.sh_o = out.sh_d = mk3(0.0f, 0.0f, 0.0f);
         out.sh_max = 0.0f;
+        uint32_t left = steps;
         for (bool traced = !kWhole;; traced = false) {
             float hit_dist = kInf;
             uint32_t hit_slot = 0u;
@@ -206,8 +210,9 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                     req[2] = make_float4(out.ph_td.x, out.ph_td.y, out.ph_td.z, 0.0f);
                     lookup = true;
                 }
-                alive = out.keep;
+                alive = out.keep && left > 1u;
             }
+            left -= 1u;
             // A lookup's term comes before the next one added to its slot: the lookups wait until a lane that
             // has one goes on, or the block's paths have all ended (without lockstep the warp's), and run together
             // (640 x 360 with a photon map, four frames: 2.15 ms with each lookup right after its shade step).
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
 }
 
 namespace {
-using PathsKernel = void (*)(const WaveJob, uint32_t, uint32_t);
+using PathsKernel = void (*)(const WaveJob, uint32_t, uint32_t, uint32_t);
 template <bool kWhole>
 PathsKernel paths_kernel(bool multi, bool photons) {
     if (multi) return photons ? wf_paths_kernel<true, true, kWhole> : wf_paths_kernel<true, false, kWhole>;
@@ -248,17 +253,19 @@ void prepare_paths_kernels() {
 // foliage 0.71 against 0.91; at 400 x 300 0.43 against 0.45; at 480 x 270 1.32 against 1.14.
 uint32_t paths_limit(int num_sms) { return (uint32_t)num_sms * kPathsBlocksPerSm * kPathsBlock; }
 
-cudaError_t launch_paths_frame(const WaveJob &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st) {
+cudaError_t launch_paths_frame(const WaveJob &p, uint32_t tiles, uint32_t steps, bool multi, bool photons, int num_sms,
+                               cudaStream_t st) {
     const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
-    paths_kernel<true>(multi, photons)<<<blocks, kPathsBlock, trav_smem_bytes(kPathsBlock, false), st>>>(p, 0u, 32u * tiles);
+    paths_kernel<true>(multi, photons)<<<blocks, kPathsBlock, trav_smem_bytes(kPathsBlock, false), st>>>(p, 0u, 32u * tiles,
+                                                                                                        steps);
     return cudaGetLastError();
 }
 
-cudaError_t launch_paths_rest(const WaveJob &p, uint32_t iter, uint32_t most, bool multi, bool photons, bool early,
-                              int num_sms, cudaStream_t st) {
+cudaError_t launch_paths_rest(const WaveJob &p, uint32_t iter, uint32_t most, uint32_t steps, bool multi, bool photons,
+                              bool early, int num_sms, cudaStream_t st) {
     const uint32_t blocks = (uint32_t)num_sms * kPathsBlocksPerSm;
     return launch_dependent_if(early, paths_kernel<false>(multi, photons), blocks, kPathsBlock,
-                               trav_smem_bytes(kPathsBlock, false), st, p, iter, most);
+                               trav_smem_bytes(kPathsBlock, false), st, p, iter, most, steps);
 }
 
 }  // namespace rtd

@@ -630,7 +630,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     // debug view and no per-launch profile.
     const uint32_t most = wide && !debug && !prof && !p.work ? paths_limit(num_sms) : 0u;
     const uint32_t whole = few_records ? most + most / 5u * 3u : most;
-    if (iters && slots <= whole) return launch_paths_frame(p, (uint32_t)tiles, !one, photons, num_sms, st);
+    if (iters && slots <= whole) return launch_paths_frame(p, (uint32_t)tiles, iters, !one, photons, num_sms, st);
     if ((e = cudaMemsetAsync(p.counts, 0, sizeof(uint32_t) * 4 * (size_t)(iters + 1), st)) != cudaSuccess) return e;
     if (tiles)
         (one ? wf_generate_kernel<false> : wf_generate_kernel<true>)<<<(unsigned)((tiles + 3u) / 4u), 128, 0, st>>>(
@@ -682,7 +682,7 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         uint32_t rest = 0u;
         if (most && it && (photons ? it % 2u == 1u && iters - it >= 2u : it % 3u == 0u && iters - it >= 3u)) {
             rest = most;
-            if ((e = launch_paths_rest(p, it, rest, !one, photons, early, num_sms, st)) != cudaSuccess) return e;
+            if ((e = launch_paths_rest(p, it, rest, iters - it, !one, photons, early, num_sms, st)) != cudaSuccess) return e;
         }
         if ((e = launch_dependent_if(early, shade, shade_grid, 128u, 0, st, p, it, rest)) != cudaSuccess) return e;
         mark(prof ? prof->shade_ev : nullptr, n_shd++, 1);

@@ -115,11 +115,12 @@ bool one_job_reads_table(const JobShape &shape, const WaveTuning &tune, bool pro
 bool photon_pass_reads_table(const DevScene &scene, const WaveTuning &tune);
 // The gather pass of few paths in one launch (k_paths.cu): a whole frame of at most paths_limit pixels in
 // `tiles` 8 x 4 tiles, or, if at most `most` paths are queued for iteration `iter` (traced, not yet shaded),
-// the rest of theirs (early: as a programmatic dependent).
+// the rest of theirs (early: as a programmatic dependent); a path takes at most `steps` shade steps.
 uint32_t paths_limit(int num_sms);
-cudaError_t launch_paths_frame(const WaveJob &p, uint32_t tiles, bool multi, bool photons, int num_sms, cudaStream_t st);
-cudaError_t launch_paths_rest(const WaveJob &p, uint32_t iter, uint32_t most, bool multi, bool photons, bool early,
-                              int num_sms, cudaStream_t st);
+cudaError_t launch_paths_frame(const WaveJob &p, uint32_t tiles, uint32_t steps, bool multi, bool photons, int num_sms,
+                               cudaStream_t st);
+cudaError_t launch_paths_rest(const WaveJob &p, uint32_t iter, uint32_t most, uint32_t steps, bool multi, bool photons,
+                              bool early, int num_sms, cudaStream_t st);
 void prepare_paths_kernels();
 int device_sm_count();
 // Fills the spare words of n uploaded triangle records (see load_tri).
