@@ -419,6 +419,7 @@ __global__ void __launch_bounds__(kBlock, 896 / kBlock) wf_trace_kernel(const __
                 at += min((uint32_t)__popc(idle), avail);
                 __syncwarp();
                 if (lane == 0u) w.at = at;
+                __syncwarp();  // (every lane reads it and w.ready next time round)
                 if (at == ready) request();
             }
         }
