@@ -84,10 +84,11 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
         const DevJob &job = job_at<kMulti>(p, jid);
         const DevScene &sc = job.scene;
         auto look_up = [&]() {
+            const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, lookup);
             if (lookup) {
                 const float4 *req = p.preq + 3ull * slot;
                 const float4 r0 = req[0], r1 = req[1], r2 = req[2];
-                photon_lookup(p, job, slot, __float_as_uint(r0.w), xyz(r0), xyz(r1), xyz(r2), runs, hit_list);
+                photon_lookup(p, job, slot, __float_as_uint(r0.w), xyz(r0), xyz(r1), xyz(r2), lanes, runs, hit_list);
                 lookup = false;
             }
             __syncwarp();

@@ -231,10 +231,14 @@ __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ 
     __shared__ uint32_t s_hits[4][kHitList * 32];
     const LookupRuns<kRunsA> runs{s_runs[threadIdx.x >> 5] + (threadIdx.x & 31u), rest};
     uint32_t *hit_list = s_hits[threadIdx.x >> 5] + (threadIdx.x & 31u);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 r0 = p.preq[3ull * i], r1 = p.preq[3ull * i + 1], r2 = p.preq[3ull * i + 2];
-        photon_lookup(p, job_at<kMulti>(p, __float_as_uint(r2.w)), __float_as_uint(r0.w), __float_as_uint(r1.w), xyz(r0), xyz(r1),
-                      xyz(r2), runs, hit_list);
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + lane, lanes = __ballot_sync(0xFFFFFFFFu, i < n);
+        if (i < n) {
+            const float4 r0 = p.preq[3ull * i], r1 = p.preq[3ull * i + 1], r2 = p.preq[3ull * i + 2];
+            photon_lookup(p, job_at<kMulti>(p, __float_as_uint(r2.w)), __float_as_uint(r0.w), __float_as_uint(r1.w), xyz(r0),
+                          xyz(r1), xyz(r2), lanes, runs, hit_list);
+        }
     }
 }
 

@@ -526,7 +526,7 @@ __device__ __forceinline__ float cell_distance2(float x, float grid_min, float c
 }
 
 // The photon-map lookup (gather.wgsl:473-514) of sample sidx of the path in `slot`: hit point hp, shading normal
-// shn, throughput x diffuse weight td.
+// shn, throughput x diffuse weight td.  lanes: the lanes of the warp that call it together.
 //
 // The reference examines the 27 cells around the hit point in order (dz, then dy, then dx), at most 384
 // photons, and adds the first 64 within the radius.  First the photons to test are laid out as runs: cells
@@ -541,7 +541,7 @@ __device__ __forceinline__ float cell_distance2(float x, float grid_min, float c
 // with the lists (16 long: 4.40 and 8.55; eight hits at a time 4.60 and 8.62, two 4.62 and 9.05).
 template <typename Runs>
 __device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob &job, uint32_t slot, uint32_t sidx, f3 hp,
-                                              f3 shn, f3 td, const Runs &runs, uint32_t *hit_list) {
+                                              f3 shn, f3 td, uint32_t lanes, const Runs &runs, uint32_t *hit_list) {
     const rt_image_params &ip = job.ip;
     const rt_grid_params &gp = job.gp;
     const float radius = ip.photon_radius, r2max = radius * radius, cell = gp.cell_size;
@@ -617,7 +617,6 @@ __device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob 
         ph_hits += waiting;
         waiting = 0u;
     };
-    const uint32_t lanes = __activemask();
     bool more = n_runs != 0u;
     uint2 m = more ? runs[0] : make_uint2(0u, 0u);
     uint32_t ri = 1u;
