@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                             r.st.t = o.w - 0.001f;
                             if (!oany) {
                                 w.limit[lane] = r.st.t;
-                                r.st.t = search_limit(r.st.t);
+                                r.st.t = kInf;
                             }
                             walk_begin(r, w, xyz(o), xyz(d), mk3(1.0f, 1.0f, 1.0f) / xyz(d), otris);
                             r.visiting = r.st.t > kEps;

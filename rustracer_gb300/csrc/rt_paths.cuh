@@ -677,10 +677,6 @@ static __device__ __noinline__ bool cut_out_lit(const DevScene &s, float4 ro, fl
     return tex_sample(s.tex[RT_TEX_ALBEDO], b.uvx, b.uvy, (int32_t)bm.tex_albedo).w < 0.5f;
 }
 
-// How far a ray that looks for its closest hit below a limit searches: a little beyond it, so that
-// rounding in a box's entry cannot lose a hit before it.
-__device__ __forceinline__ float search_limit(float limit) { return limit > kEps ? limit * 1.001f : kInf; }
-
 // The pixel in `slot`: the last NEE term, the firefly sigma clamp and the frame outputs (gather.wgsl:548-593).
 __device__ __forceinline__ void finalize_slot(const WaveParams &p, const DevJob &job, uint32_t slot) {
     const uint32_t pix = slot - job.base;

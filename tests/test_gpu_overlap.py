@@ -3,6 +3,7 @@ surfaces a ray hits depends on the order its walk meets them in.  That order is 
 the same bit for bit whatever the shape of the launch.
 """
 import ctypes as C
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -160,3 +161,45 @@ def test_full_stack(gpu, live, passed, steps):
     r.record_frame()
     red, green, _ = r.read_accumulation().reshape(-1)[:3]
     assert green > red
+
+
+def cut_out_scene(thin, scale):
+    """A floor under a point light, a cut-out leaf, and slivers whose boxes begin a little beyond the light."""
+    n = 4000
+    rng = np.random.default_rng(2)
+    s = rt.Scene()
+    tex = np.full((1, 8, 8, 4), 255, np.uint8)
+    tex[0, ::2, ::2, 3] = 0
+    s.set_textures(A.TEX_ALBEDO, tex)
+    floor, needle = s.add_material(rt.lambertian((0.8, 0.8, 0.8))), s.add_material(rt.lambertian((0.2, 0.9, 0.2)))
+    leaf = s.add_material(rt.material(A.MAT_LAMBERTIAN, (0.5, 0.9, 0.4), alpha_cutout=True, tex_albedo=0))
+    quad = np.array([[-3, -3, 0], [3, -3, 0], [3, 3, 0], [-3, 3, 0]], np.float32)
+    s.add_mesh(quad * scale, [0, 1, 2, 0, 2, 3], floor)
+    s.add_mesh((0.1 * quad + np.float32([2, 2, 0.2])) * scale, [0, 1, 2, 0, 2, 3], leaf, uvs=[[0, 0], [1, 0], [1, 1], [0, 1]])
+    a, along = rng.uniform(0, np.pi, (n, 1)), rng.uniform(0.2, 1.0, (n, 1))
+    u, v = along * np.concatenate([-np.ones((n, 1)), np.ones((n, 1)), rng.uniform(-1, 1, (n, 1))], 1), thin * rng.uniform(-1, 1, (n, 3))
+    c = rng.uniform(-0.01, 0.01, (n, 2))
+    p = np.stack([c[:, :1] + np.cos(a) * u - np.sin(a) * v, c[:, 1:] + np.sin(a) * u + np.cos(a) * v,
+                  np.repeat(0.5 + rng.uniform(0.25e-3, 1e-3, (n, 1)), 3, axis=1)], axis=-1)
+    s.add_mesh((p * scale).reshape(-1, 3), np.arange(3 * n), needle)
+    s.add_light(rt.point_light((0.0, 0.0, 0.5 * scale), (1, 1, 1), 20.0 * scale * scale))
+    return s
+
+
+def cut_out_lit(thin, scale):
+    """The pixels whose light is visible."""
+    r = rt.Renderer(cut_out_scene(thin, scale), rt.RenderConfig(width=150, height=150, spp=1, accumulate_frames=1,
+                                                                enable_denoise=False, max_bounces=1))
+    r.update_camera(rt.Camera((0, 0, 4.0 * scale), (0, 0, 0), (0, 1, 0), 60.0))
+    r.record_frame()
+    return r.read_accumulation()[..., 0] > 0.03
+
+
+@pytest.mark.parametrize("thin", [1e-3, 1e-5])
+@pytest.mark.parametrize("scale", [1.0, 100.0])
+def test_slivers_behind_a_light_with_cut_outs(gpu, width, thin, scale):  # noqa: F811
+    """With cut-out materials in the scene a light is hidden by the closest hit before it: also by a sliver whose
+    box begins beyond the light.  Compared with the pixels that were lit when occlusion rays had no limit and leaves
+    no queue (commit 8f6a6e2)."""
+    packed = np.load(Path(__file__).parent / "golden" / "cut_slivers.npz")[f"{width}_{thin:g}_{scale:g}"]
+    assert np.array_equal(np.packbits(cut_out_lit(thin, scale)), packed)
