@@ -539,8 +539,8 @@ __global__ void __launch_bounds__(256) photon_gather_kernel(const float4 *__rest
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += 2 * step) {
         const uint64_t i2 = i + step;
         const bool two = i2 < n;
-        const float4 *s0 = photons + 4ull * order[i];
-        const float4 *s1 = photons + 4ull * order[two ? i2 : i];
+        const float4 *s0 = photons + 4ull * __ldcg(order + i);
+        const float4 *s1 = photons + 4ull * __ldcg(order + (two ? i2 : i));
         if (wide) {
             Photon8 a, b;
             load_photon_wide(s0, a);
@@ -574,7 +574,8 @@ __global__ void __launch_bounds__(256) photon_gather_kernel(const float4 *__rest
 
 // ---- grid build with per-slot ranks ---------------------------------------------------------------
 // The kernels after the count are launched as programmatic dependents of the one before (their blocks
-// may be scheduled while it finishes and wait for it in grid_dependency_wait).
+// may be scheduled while it finishes and wait for it in grid_dependency_wait).  What that launch writes they read
+// with __ldcg: a read-only load (__ldg) is for data that does not change while the kernel is there.
 
 // Histogram with ranks: counts[key] += 1 and rank[slot] = the count found before the add (the slot's
 // position within its cell, in atomic order).
@@ -851,7 +852,7 @@ __global__ void __launch_bounds__(256) scatter_rank_kernel(const uint32_t *__res
         uint32_t pos[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (kk[j] != kInvalidKey) pos[j] = __ldg(&meta[kk[j]].x) + __ldg(rank + (j < 4 ? s0 : s1) + (j & 3));
+            if (kk[j] != kInvalidKey) pos[j] = __ldcg(&meta[kk[j]].x) + __ldg(rank + (j < 4 ? s0 : s1) + (j & 3));
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             if (kk[j] != kInvalidKey) order[pos[j]] = (uint32_t)((j < 4 ? s0 : s1) + (j & 3));
@@ -915,7 +916,7 @@ __device__ __forceinline__ void sort_cell_to(const uint32_t *__restrict__ order,
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const uint32_t e = lane * R + r;
-        v[r] = e < count ? __ldg(order + start + e) : 0xFFFFFFFFu;
+        v[r] = e < count ? __ldcg(order + start + e) : 0xFFFFFFFFu;
     }
     if (count > 1u) warp_sort_regs<R>(v, lane);
 #pragma unroll
@@ -1093,7 +1094,7 @@ __global__ void __launch_bounds__(256) small_scatter_kernel(const uint32_t *__re
             const uint32_t cell = word[j] & ((1u << kSmallCellBits) - 1u);
             uint32_t rank = word[j] >> kSmallCellBits;
             if (rank == kSmallRankMax) rank = atomicSub(counts + cell, 1u) - 1u;
-            pos[j] = __ldg(meta + 2u * cell) + rank;
+            pos[j] = __ldcg(meta + 2u * cell) + rank;
         }
 #pragma unroll
     for (int j = 0; j < 4; ++j)

@@ -296,25 +296,6 @@ __device__ __forceinline__ float4 tex_sample(const DevTex &t, float u, float v, 
                        lerp2(t00.z, t10.z, t01.z, t11.z), lerp2(t00.w, t10.w, t01.w, t11.w));
 }
 
-// ---- Moller-Trumbore (common.wgsl:78-100) ------------------------------------------------------
-__device__ __forceinline__ float intersect_triangle(f3 ro, f3 rd, f3 v0, f3 v1, f3 v2) {
-    f3 e1 = v1 - v0;
-    f3 e2 = v2 - v0;
-    f3 h = cross(rd, e2);
-    float a = dot(e1, h);
-    if (fabsf(a) < 1e-7f) return kInf;
-    float f = 1.0f / a;
-    f3 s = ro - v0;
-    float u = f * dot(s, h);
-    if (u < 0.0f || u > 1.0f) return kInf;
-    f3 q = cross(s, e1);
-    float v = f * dot(rd, q);
-    if (v < 0.0f || u + v > 1.0f) return kInf;
-    float t = f * dot(e2, q);
-    if (t > kEps) return t;
-    return kInf;
-}
-
 struct Bary {
     float uvx, uvy, u, v;
 };
