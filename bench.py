@@ -433,18 +433,38 @@ def job_objects(spec: dict, pool):
     return scene, cfg, cam
 
 
-def frame_launches(cfgs) -> int:
-    """Kernel launches of one batch frame over jobs with these configs: one generate and one finalize
-    launch over all jobs, per iteration one trace launch (closest-hit rays of the iteration with the
+def wide_records(scene) -> int:
+    """Four-wide records of the scene's tree."""
+    import ctypes as C
+
+    from rustracer_gb300 import _abi as A
+
+    d = scene.describe()
+    records, stack = C.c_uint64(), C.c_uint32()
+    A.check("rt_bvh_wide_layout", A.load().rt_bvh_wide_layout(d.bvh_nodes, d.bvh_node_count, None, 0, C.byref(records),
+                                                              C.byref(stack)))
+    return records.value
+
+
+def frame_launches(jobs, sms: int) -> int:
+    """Kernel launches of one frame over these (scene, config) jobs on a GPU of `sms` SMs.  Up to 512 pixels
+    per SM, 8/5 of that where every tree has at most 64 records: one launch.  Else one generate and one
+    finalize launch over all jobs, per iteration one trace launch (closest-hit rays of the iteration with the
     occlusion rays of the one before), one shade and, when a job has a photon map, one photon-lookup
     launch; before every third shade (every second with a photon map) the launch that runs the last
-    paths once few are left; the closing trace launch, the counter kernel, then per job the denoise
+    paths once few are left; the closing trace launch and the counter kernel.  Then per job the denoise
     passes and the resolve."""
+    cfgs = [c for _, c in jobs]
+    post = sum((c.denoise_passes or 2) * int(c.enable_denoise) + 1 for c in cfgs)
+    limit = 512 * sms
+    if all(wide_records(s) <= 64 for s in {id(s): s for s, _ in jobs}.values()):
+        limit += limit // 5 * 3
+    if sum(c.width * c.height for c in cfgs) <= limit:
+        return 1 + post
     iters = max(max(c.spp, 1) * (c.max_bounces or 6) for c in cfgs)
     photons = any(c.enable_photon_map for c in cfgs)
     per_iter, tries = (3, len(range(1, iters - 1, 2))) if photons else (2, len(range(3, iters - 2, 3)))
-    return (2 + per_iter * iters + tries + 2 +
-            sum((c.denoise_passes or 2) * int(c.enable_denoise) + 1 for c in cfgs))
+    return 2 + per_iter * iters + tries + 2 + post
 
 
 def batched_leg(n_jobs: int, steps: int, warmup: int, pool, seed: int = 4) -> dict:
@@ -534,7 +554,8 @@ def batched_leg(n_jobs: int, steps: int, warmup: int, pool, seed: int = 4) -> di
         "autotune": {"default": default_shape, "chosen": tuned_shape, "ms_per_frame": tuned_ms,
                      "seconds": tune_s},
         "graph_captures": int(s1.graph_captures),
-        "gpu_launches_per_frame": frame_launches([job_objects(s, pool)[1] for s in specs]),
+        "gpu_launches_per_frame": frame_launches([job_objects(s, pool)[:2] for s in specs],
+                                                 torch.cuda.get_device_properties(0).multi_processor_count),
         "resident_scenes": len(resident),
     }
 
@@ -742,7 +763,8 @@ def run_ours(args, w):
             "config": {"workload": args.workload, **{k: v for k, v in w.items()}, "l2": "inputs larger than L2",
                        "parallelism": f"replicas{world}"},
             "shadow_rays_per_s": shd_all / (ms_max / 1000.0),
-            "gpu_launches": int(frame_launches([cfg]) * args.steps),
+            "gpu_launches": args.steps * frame_launches(
+                [(scene, cfg)], torch.cuda.get_device_properties(local).multi_processor_count),
             "kernel_ms": {"gather": gather_ms, "resolve": resolve_ms},
             "roofline": roofline,
             "oracle_work_per_ray": work,
