@@ -347,8 +347,10 @@ int rt_get_grid_params(const rt_renderer *r, rt_grid_params *out);
  * megakernel dispatch).  With RT_PROFILE_EVENTS set, every later rt_render_frame records CUDA events
  * around each launch of the traversal, shade and photon-lookup kernels and waits for its frame; with
  * RT_PROFILE_COUNT it runs the counting variants of the traversal kernels (same rays and results),
- * which add the records each kind of ray visits and its leaf triangle tests.  Images are unchanged
- * either way.  rt_read_profile returns the sums over the profiled frames since the previous read and
+ * which add the records each kind of ray visits and its leaf triangle tests.  A profiled frame has a
+ * launch per stage throughout: the one-launch forms that other frames take for few pixels, or for the
+ * last paths of many, are not profiled, so the times of a small frame's launches are not the ones it
+ * has unprofiled.  Images are unchanged either way.  rt_read_profile returns the sums over the profiled frames since the previous read and
  * resets them; rt_set_profiling(r, 0) stops profiling. */
 #define RT_PROFILE_EVENTS 1u
 #define RT_PROFILE_COUNT 2u
@@ -398,8 +400,8 @@ typedef struct rt_batch rt_batch;
  * 256, blocks_per_sm up to 2048 / block_threads, chunk (queue items a warp takes per atomic, its
  * segment of the shared queue) 32 .. 1024 in steps of 32, steps (traversal records between lane
  * refills) 1 .. 64, stack_entries 32 / 48 / 64, raised to what the jobs' trees need (kept for callers
- * that set it: the newest entries of a lane's stack are in shared memory and the rest in local
- * memory, whatever its value).
+ * that set it: the oldest entries of a lane's stack are in shared memory and the ones above them in
+ * local memory, whatever its value).
  * Default: 128 threads, 7 blocks per SM, chunk 32, 3 steps, 32 entries, no treelet, shade_blocks 6,
  * refill_idle 0. */
 typedef struct rt_wavefront_tuning {

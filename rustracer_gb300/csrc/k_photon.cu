@@ -208,8 +208,8 @@ __device__ bool photon_bounce(const PhotonTraceParams &p, uint32_t photon_index,
 }
 
 // ------------------------------------------------------------------------------------------------
-// Photon wavefront: generate (emission), then per bounce the shared closest-hit kernel (wf_extend,
-// persistent traversal warps) and ph_shade (one bounce body per queued photon, survivors re-queued).
+// Photon wavefront: generate (emission), then per bounce the shared closest-hit kernel
+// (wf_trace_kernel, persistent traversal warps) and ph_shade (one bounce body per queued photon, survivors re-queued).
 // Lanes stay busy when photons end at different bounces, and each kernel is small; the per-photon
 // operations and their order are those of the loop, so every photon's path is unchanged.
 // ------------------------------------------------------------------------------------------------
@@ -526,13 +526,11 @@ __device__ __forceinline__ void store_photon_wide(float4 *dst, const Photon8 &p)
 }
 
 // sorted[i] = photons[order[i]] for i < total, two photons per thread with both records loaded
-// before the stores; 32-byte accesses when both buffers are 32-byte aligned (`wide`).  sorted_pos,
-// when given, gets each photon's first float4.
+// before the stores; 32-byte accesses when both buffers are 32-byte aligned (`wide`).
 __global__ void __launch_bounds__(256) photon_gather_kernel(const float4 *__restrict__ photons,
                                                             const uint32_t *__restrict__ order,
                                                             const uint32_t *__restrict__ total, uint64_t cap,
-                                                            float4 *__restrict__ sorted,
-                                                            float4 *__restrict__ sorted_pos, bool wide) {
+                                                            float4 *__restrict__ sorted, bool wide) {
     grid_dependency_wait();
     const uint64_t n = min((uint64_t)*total, cap);
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
@@ -546,11 +544,7 @@ __global__ void __launch_bounds__(256) photon_gather_kernel(const float4 *__rest
             load_photon_wide(s0, a);
             load_photon_wide(s1, b);
             store_photon_wide(sorted + 4ull * i, a);
-            if (sorted_pos) sorted_pos[i] = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
-            if (two) {
-                store_photon_wide(sorted + 4ull * i2, b);
-                if (sorted_pos) sorted_pos[i2] = make_float4(b.v[0], b.v[1], b.v[2], b.v[3]);
-            }
+            if (two) store_photon_wide(sorted + 4ull * i2, b);
         } else {
             const float4 a = __ldg(s0), b = __ldg(s0 + 1), c = __ldg(s0 + 2), d = __ldg(s0 + 3);
             const float4 e = __ldg(s1), f = __ldg(s1 + 1), g = __ldg(s1 + 2), h = __ldg(s1 + 3);
@@ -559,14 +553,12 @@ __global__ void __launch_bounds__(256) photon_gather_kernel(const float4 *__rest
             d0[1] = b;
             d0[2] = c;
             d0[3] = d;
-            if (sorted_pos) sorted_pos[i] = a;
             if (two) {
                 float4 *d1 = sorted + 4ull * i2;
                 d1[0] = e;
                 d1[1] = f;
                 d1[2] = g;
                 d1[3] = h;
-                if (sorted_pos) sorted_pos[i2] = e;
             }
         }
     }
@@ -1204,7 +1196,7 @@ cudaError_t launch_small_grid(const SmallGrid &g, const rt_grid_params &gp, cuda
                               g.total + 1, g.counts, g.order, words_log2)) != cudaSuccess)
         return e;
     return launch_dependent(photon_gather_kernel, std::min(blocks(blocks(n, 2u), 256u), sm * 8u), 256u, 0, st, g.photons,
-                            g.order, g.total, (uint64_t)n, g.sorted, (float4 *)nullptr, wide);
+                            g.order, g.total, (uint64_t)n, g.sorted, wide);
 }
 
 }  // namespace rtd

@@ -243,11 +243,10 @@ __global__ void __launch_bounds__(128) wf_photon_kernel(const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------------------------------------
-// shadow: the deferred NEE occlusion test (gather.wgsl:91-103); a visible light marks its slot's NEE term.
-// ------------------------------------------------------------------------------------------------
-// trace: the occlusion rays of iteration `shd_iter` and the closest-hit rays of iteration `ext_iter` in
-// one persistent launch (either may be kNoIter).  Both depend only on the shade pass before them and
-// touch disjoint state (shadow records and accumulators / path rays and hits), so one launch carries
+// trace: the deferred NEE occlusion rays of iteration `shd_iter` (gather.wgsl:91-103; a visible light marks its
+// slot's NEE term) and the closest-hit rays of iteration `ext_iter` in one persistent launch (either may be
+// kNoIter).  Both depend only on the shade pass before them and touch disjoint state (shadow records and NEE
+// words / path rays and hits), so one launch carries
 // them with one tail instead of two.  Closest-hit rays come first in the work list: the longer rays
 // start early and the shorter occlusion rays fill the end.
 constexpr uint32_t kNoIter = 0xFFFFFFFFu;

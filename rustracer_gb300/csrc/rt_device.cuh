@@ -167,9 +167,9 @@ struct DevScene {
     const float4 *cnodes;
     const float4 *tri_ord;
     uint32_t cnode_count, stack_cap;
-    // The same tree with up to four children per 128-byte record (per child (min, ref), (max, count);
-    // count 0xFFFFFFFF marks an empty place), when a near-first walk of it needs at most 64 stack
-    // entries (wide_stack); otherwise wnodes is null and only the two-wide records are used.
+    // The same tree with up to four children per 128-byte record (per child (min.x, max.x, min.y, max.y),
+    // (min.z, max.z, ref, count); an empty place has a NaN box), when a near-first walk of it needs at most
+    // 64 stack entries (wide_stack); otherwise wnodes is null and only the two-wide records are used.
     const float4 *wnodes;
     uint32_t wnode_count, wide_stack;
     uint32_t any_hit_shadows;  // 1: no alpha-cutout material, shadow rays may stop at the first hit

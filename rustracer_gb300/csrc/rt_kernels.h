@@ -211,7 +211,9 @@ cudaError_t launch_resolve(const float4 *frame, float4 *accum, const float4 *gbu
 
 // Launches `kernel` as a programmatic dependent of the previous kernel in the stream: its blocks may be
 // scheduled as that kernel's blocks leave and wait for its end in grid_dependency_wait(), which every such
-// kernel calls before it touches memory.
+// kernel calls before it touches memory that an earlier launch writes or reads.  (small_count_kernel reads the
+// caller's photons before it: the launch in front of it, small_clear_kernel, has to stay an ordinary one, which
+// begins when everything before it has ended.)
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent_if(bool early, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
                                 cudaStream_t st, Args... args) {
