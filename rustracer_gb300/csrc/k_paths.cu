@@ -50,10 +50,10 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
     static_assert(sizeof(WarpTrav) >= 32 * (kRunsA * sizeof(uint2) + kHitList * sizeof(uint32_t)), "lookup state");
     // A step is some 3,000 instructions without a loop, which the warps of a scheduler would each fetch at another
     // place (40% of their cycles), so a block's warps start each shade step together: 16 Cornell frames of
-    // 256 x 256 2.07 -> 1.71 ms (blocks of four warps 1.79, of sixteen 1.73).  Not with photon maps and several
-    // samples in every pixel, where lookups that cannot wait keep the others waiting (relight at 4 spp 4.28 against
-    // 4.25 ms; one sample, 640 x 360, four frames: 1.88 against 1.95).
-    const bool lockstep = !kPhotons || p.lockstep != 0u;
+    // 256 x 256 2.07 -> 1.71 ms (blocks of four warps 1.79, of sixteen 1.73).  With photon maps too: gather of a whole
+    // Cornell frame at 300 x 240, 1 / 4 spp, 0.067 / 0.217 ms against 0.082 / 0.333 with each warp on its own, a
+    // 20k-triangle room 0.250 / 0.967 against 0.279 / 1.137; the last paths of 640 x 360 0.494 / 1.899 against
+    // 0.515 / 1.989 in the room, 0.197 / 0.650 against 0.195 / 0.643 in the Cornell box.
     const Treelet tree{nullptr, nullptr, 0u};
     LaneWalk r;
     r.busy = r.visiting = r.any_hit = false;
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
                 if (lit) p.nee[slot].w = __uint_as_float(__float_as_uint(p.nee[slot].w) | kNeeLit);
                 out.shadow = false;
             }
-            if (lockstep ? !__syncthreads_or(alive) : !__any_sync(0xFFFFFFFFu, alive)) break;
+            if (!__syncthreads_or(alive)) break;
             if (alive) {
                 uint32_t prim = 0u, word = 0u;
                 if (hit_dist < kInf) {
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) wf_paths_kerne
             }
             left -= 1u;
             // A lookup's term comes before the next one added to its slot: the lookups wait until a lane that
-            // has one goes on, or the block's paths have all ended (without lockstep the warp's), and run together
+            // has one goes on, or the block's paths have all ended, and run together
             // (640 x 360 with a photon map, four frames: 2.15 ms with each lookup right after its shade step).
             if (kPhotons && __any_sync(0xFFFFFFFFu, lookup && alive)) look_up();
         }

@@ -614,7 +614,6 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         wide_need = jobs[j].wide_stack > wide_need ? jobs[j].wide_stack : wide_need;
         wide = wide && jobs[j].wide != 0u;
         cut = cut || jobs[j].scene->any_hit_shadows == 0u;
-        if (jobs[j].spp <= 1u) p.lockstep = 1u;
         few_records = few_records && jobs[j].scene->wnode_count <= 64u;
     }
     if (n_jobs == 1u) set_scene0(p, *jobs[0].scene, wide);
@@ -629,7 +628,8 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     // 8/5 as many (Cornell box at 400 x 300, 1 and 4 spp: 189 and 653 us against 222 and 699, 20 leaf cards 204 / 265;
     // a 20k-triangle room 491 / 462; 512 x 300 at 3 spp 576 / 547).  Few paths left: the rest of them in one launch, tried at
     // every third iteration, with photon maps (which end most paths at once) at every second (an idle try
-    // costs 2.5 us).  Gather with and without the tries: config 2 18.7 / 19.1 ms, 640 x 480 at 4 spp in a
+    // costs 2.5 us, and a frame of one sample without a photon map up to 0.8% where its paths are never few: 800 x 600
+    // and up; with more samples the tries gain there too, 1% to 3% at 4 spp, with a photon map up to 33%).  Gather with and without the tries: config 2 18.7 / 19.1 ms, 640 x 480 at 4 spp in a
     // 328k-triangle room 4.39 / 4.71, cut-out foliage 1.51 / 1.57, 640 x 480 with a photon map 0.81 / 1.13;
     // a limit of half as many paths measures 18.9, 4.44, 1.50 and 0.81, later 1080p room frames 17.99 against 17.83, with
     // twice as many 17.98.  Both need the four-wide records, no
@@ -668,10 +668,12 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
     else
         shade = photons ? (debug ? wf_shade_kernel<true, true, true, 4> : wf_shade_kernel<true, false, true, 4>)
                         : (debug ? wf_shade_kernel<false, true, true, 4> : wf_shade_kernel<false, false, true, 4>);
-    // In a small pass each launch's blocks are scheduled while the one before drains (gather 1.05 against 1.10 ms
-    // at 480 x 270, 0.56 against 0.59 at 640 x 360 with a photon map).  In a large one that keeps traversal and
-    // shade on the same SMs and with them the traversal's split of L1 for both (19.2 against 18.3 ms on config 2,
-    // 0.98 against 0.96 at 800 x 600).
+    // In a small pass each launch's blocks are scheduled while the one before drains.  In a large one that keeps
+    // traversal and shade on the same SMs and with them the traversal's split of L1 for both.  Gather without it
+    // over gather with it, rooms of 20k and 328k triangles and the Cornell box at 1 and 3 spp, then with a photon
+    // map: 480 x 270 1.02 .. 1.17, 1.06 .. 1.24; 640 x 360, just below the line, 0.99 .. 1.11, 1.04 .. 1.19;
+    // 800 x 600 1.00 .. 1.03, 1.03 .. 1.12; 1280 x 720 0.96 .. 0.99, 1.00 .. 1.06; config 2 0.95.  So the line is on
+    // the safe side: the two are even near twice as many slots, and later with a photon map.
     const bool early = slots <= (uint64_t)num_sms * 1536u;
     uint32_t n_trc = 0, n_shd = 0, n_pho = 0;
     // Events of the profiled pass around one launch (never inside a captured graph: prof is null there).

@@ -53,7 +53,6 @@ struct WaveParams {
     // any hit and whether it has no triangles; filled by the launchers.
     const float4 *records0, *tris0;
     uint32_t any_hit0, empty0;
-    uint32_t lockstep;  // the few-path kernel's blocks with photon lookups shade together too (set by launch_wavefront)
 };
 // The parameters of the kernels that read a job's tables.  A launch over one job whose values are known when it
 // is enqueued (not captured) carries the job itself: its words are constant operands then instead of loads, each
@@ -69,7 +68,7 @@ __device__ __forceinline__ const DevJob &job_at(const WaveJob &p, uint32_t jid) 
 }
 // Host-side shape of a job for the per-job launches.
 struct JobShape {
-    uint32_t width, height, npix, base, stack_cap, spp;
+    uint32_t width, height, npix, base, stack_cap;
     uint32_t photons;  // the job gathers from a photon map (rt_image_params.use_photons)
     uint32_t debug;    // the job renders a debug view (rt_image_params._pad[0] != 0)
     uint32_t wide;     // the job's scene has four-wide records (DevScene.wnodes)

@@ -675,7 +675,6 @@ extern "C" int rt_render_frame(rt_renderer *r) {
                                   (uint32_t)npix,
                                   0u,
                                   r->scene.stack_cap,
-                                  c.spp,
                                   c.enable_photon_map ? 1u : 0u,
                                   c.debug_view != 0u ? 1u : 0u,
                                   r->scene.wnodes ? 1u : 0u,
