@@ -544,7 +544,7 @@ __device__ __forceinline__ void photon_lookup(const WaveParams &p, const DevJob 
                                               f3 shn, f3 td, uint32_t lanes, const Runs &runs, uint32_t *hit_list) {
     const rt_image_params &ip = job.ip;
     const rt_grid_params &gp = job.gp;
-    const float radius = ip.photon_radius, r2max = radius * radius, cell = gp.cell_size;
+    const float radius = fabsf(ip.photon_radius), r2max = radius * radius, cell = gp.cell_size;  // (only its square counts)
     const int32_t bx = f2i_sat((hp.x - gp.room_min_x) / cell);
     const int32_t by = f2i_sat((hp.y - gp.room_min_y) / cell);
     const int32_t bz = f2i_sat((hp.z - gp.room_min_z) / cell);
