@@ -11,10 +11,10 @@
 // What bounds few paths in the wavefront is its chain of launches, each of them one dependent load after the
 // other for a fraction of a warp per scheduler: the Cornell box at 256 x 256, 5 segments deep, took 15
 // launches and 188 us.  Here a warp waits for its own loads only.  It is bound by the fetch and the latency of one
-// path's instructions (16 warps per SM, issue 35% of cycles): 118 us for that frame, 40% of it waits for instructions,
-// before the warps of a block shaded together, 95 since.  With more paths
-// than the SMs hold at once the compacted queues win: lanes whose path has ended idle here until the warp's
-// last one ends.
+// path's instructions (16 warps per SM, issue 45% of cycles): 118 us for that frame, 40% of it waits for instructions,
+// before the warps of a block shaded together, 95 with that, 84 since idle lanes look for work after every
+// record.  With more paths than the SMs hold at once the compacted queues win: lanes whose path has ended idle
+// here until the warp's last one ends.
 #include "rt_paths.cuh"
 
 namespace rtd {
@@ -249,9 +249,11 @@ void prepare_paths_kernels() {
     }
 }
 
-// As many paths as the SMs hold threads of the kernel.  Measured against the wavefront (gather, ms): 320 x 240
-// 1 spp in a 20k-triangle room 0.39 against 0.43, 2 spp in a 328k-triangle room 0.90 against 1.25, cut-out
-// foliage 0.71 against 0.91; at 400 x 300 0.43 against 0.45; at 480 x 270 1.32 against 1.14.
+// As many paths as the SMs hold threads of the kernel.  Measured against the wavefront (gather, ms, 1 and 4 spp):
+// 304 x 250 in a 20k-triangle room 0.28 / 0.99 against 0.38 / 1.17, in a 328k-triangle room 0.46 / 1.59 against
+// 0.60 / 1.70, cut-out foliage 0.19 / 0.64 against 0.28 / 0.85; above the limit, 352 x 280, 0.40 / 1.45 against
+// 0.39 / 1.31 and 0.63 / 2.20 against 0.64 / 1.97 in the rooms.  (With photon maps it still gains there: 0.29 / 1.16
+// against 0.37 / 1.33, up to 480 x 270.)
 uint32_t paths_limit(int num_sms) { return (uint32_t)num_sms * kPathsBlocksPerSm * kPathsBlock; }
 
 cudaError_t launch_paths_frame(const WaveJob &p, uint32_t tiles, uint32_t steps, bool multi, bool photons, int num_sms,

@@ -257,9 +257,9 @@ constexpr uint32_t kOcclusion = 0x80000000u;  // ray id: path slot, and whether 
 // fetches together, so the step is kept short and the registers few: 7 blocks of 128 threads per SM
 // (72 registers; 64 registers for 8 blocks spill in the step and measure 4% slower, 80 for 6 blocks 4%),
 // the ray feed in shared memory, no branch in the triangle test.  Config-2 frame (28.5 M closest-hit and
-// 24.9 M occlusion rays): 13.5 ms against 16.3 ms for the kernel this one replaced, which tested every
-// step's leaves at once in a list laid out over the warp and read rays when a lane ran out; 22% fewer
-// instructions, 11% fewer records visited (pending records entered beyond the hit are dropped unread).
+// 24.8 M occlusion rays): 12.8 ms against 16.1 ms for the kernel this one replaced, which laid a step's
+// triangles out over the warp with a scan and read rays when a lane ran out; 11% fewer records visited
+// (pending records entered beyond the hit are dropped unread).
 //
 // kCount: the profiling variant, which also counts the records each kind of ray visits and its leaf
 // triangle tests into p.work (one atomic per warp at exit); the same rays and results otherwise.
@@ -624,16 +624,16 @@ cudaError_t launch_wavefront(const WaveParams &params, const JobShape *jobs, uin
         photons = photons || jobs[j].photons != 0u;
         debug = debug || jobs[j].debug != 0u;
     }
-    // Few pixels: the whole pass in one launch, with trees of a few dozen records, whose walks hardly differ, up to
-    // 8/5 as many (Cornell box at 400 x 300, 1 and 4 spp: 189 and 653 us against 222 and 699, 20 leaf cards 204 / 265;
-    // a 20k-triangle room 491 / 462; 512 x 300 at 3 spp 576 / 547).  Few paths left: the rest of them in one launch, tried at
-    // every third iteration, with photon maps (which end most paths at once) at every second (an idle try
-    // costs 2.5 us, and a frame of one sample without a photon map up to 0.8% where its paths are never few: 800 x 600
-    // and up; with more samples the tries gain there too, 1% to 3% at 4 spp, with a photon map up to 33%).  Gather with and without the tries: config 2 18.7 / 19.1 ms, 640 x 480 at 4 spp in a
-    // 328k-triangle room 4.39 / 4.71, cut-out foliage 1.51 / 1.57, 640 x 480 with a photon map 0.81 / 1.13;
-    // a limit of half as many paths measures 18.9, 4.44, 1.50 and 0.81, later 1080p room frames 17.99 against 17.83, with
-    // twice as many 17.98.  Both need the four-wide records, no
-    // debug view and no per-launch profile.
+    // Few pixels: the whole pass in one launch (paths_limit), with trees of a few dozen records, whose walks hardly
+    // differ, up to 8/5 as many: Cornell box at 400 x 311, 1 and 4 spp, 155 and 526 us against 178 and 578, 20 leaf
+    // cards 91 and 237 against 138 and 389; above that, at 512 x 300, the Cornell box 181 and 612 against 184 and 590.
+    // Few paths left: the rest of them in one launch, tried at every third iteration, with photon maps (which end
+    // most paths at once) at every second.  Gather without the tries over gather with them, rooms of 20k and 328k
+    // triangles and the Cornell box, 1 to 4 spp, then with a photon map: 420 x 300 1.06 .. 1.20, 1.07 .. 1.67;
+    // 640 x 360 1.00 .. 1.13, 1.05 .. 1.55; 800 x 600 0.99 .. 1.03, 1.00 .. 1.33; 1080p 0.99 .. 1.01, 1.00 .. 1.10.
+    // (An idle try costs 2.5 us; the 0.99s are frames of one sample, whose paths are never few.)  With a limit of
+    // half as many paths 1080p room frames measure 17.99 against 17.83 ms, with twice as many 17.98.
+    // Both need the four-wide records, no debug view and no per-launch profile.
     const uint32_t most = wide && !debug && !prof && !p.work ? paths_limit(num_sms) : 0u;
     const uint32_t whole = few_records ? most + most / 5u * 3u : most;
     if (iters && slots <= whole) return launch_paths_frame(p, (uint32_t)tiles, iters, !one, photons, num_sms, st);
